@@ -232,6 +232,10 @@ void drop_extra(hfmm_plan* P) {
 void upload_level(hfmm_plan* P, int fam, int l, const double* const* h) {
     LevelTables& T = P->tables[fam][l];
     const int n_s = P->n_s, ld = P->ld;
+    T.m2l_hi.release();   // halves of the tables being replaced
+    T.m2l_lo.release();
+    P->conv.tables = false;
+    T.host_m2l = h[8] != nullptr;
     std::vector<int32_t> none;
     relayout(h[0], 1, none, n_s, ld, false, T.up_U);   // A = U^T  -> A^T = U
     upload_vec(h[1], n_s, ld, T.up_d);
@@ -691,9 +695,16 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
         for (int k = 0; k < hfmm_plan::CX_STREAMS; ++k)   // every side stream rejoins
             HFMM_CUDA(cudaEventRecord(P->cx_join[k], P->cx_side[k]));
     }
-    // ---- downward pass (M2L + L2L in one GEMM, then X-list P2L, then decode)
+    // The FP64 M2L of every level, by convolution: it reads only the upward densities. The
+    // dense tables serve host-given M2L tables and surfaces that are no lattice's.
+    const bool use_conv = P->conv.on && !use_mx && P->rot_P == 0;
+    if (use_conv) {
+        PhaseTimer pt(X, s, 4);
+        conv_m2l(P, R, fs, s);
+    }
+    // ---- downward pass (M2L, L2L, then X-list P2L, then decode)
     for (int l = 2; l <= P->md; ++l) {
-        if (P->streamed && !use_cx) {
+        if (P->streamed && !use_cx && !use_conv) {
             PhaseTimer pt(X, s, 12);
             generate_m2l_stream(P, l, use_mx, P->ws, s);
         }
@@ -732,6 +743,10 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
                 m2l_tf32x3(static_cast<MixedMaps*>(P->mx_maps)[l], mc, s);
             }
             if (l >= 3)   // L2L (phases.py:273-278) in FP64, added to the check potential
+                gemm(K_L2L, l, P->dn_tiles[l][R - 1], P->m2l_src.p + N_DISP, M2L_ENTRIES, P->loc.p,
+                     nullptr, P->check.p);
+        } else if (use_conv) {   // the check potentials hold the M2L's: add the parent's
+            if (l >= 3)
                 gemm(K_L2L, l, P->dn_tiles[l][R - 1], P->m2l_src.p + N_DISP, M2L_ENTRIES, P->loc.p,
                      nullptr, P->check.p);
         } else if (P->rot_P > 0) {   // rotation-based M2L (m2l_rotation.cu), then the L2L GEMM
@@ -982,6 +997,7 @@ int hfmm_plan_set_kernel(hfmm_plan* P, double k, int32_t p, int32_t n_families,
         d.alloc(soa.size());
         HFMM_CUDA(cudaMemcpy(d.p, soa.data(), soa.size() * 8, cudaMemcpyHostToDevice));
     }
+    conv_surface(P, equiv_pts);
     P->finalized = false;
     return HFMM_OK;
     API_END
@@ -1082,6 +1098,23 @@ int hfmm_plan_finalize(hfmm_plan* P) {
     // A pointer table that points at them
     P->mixed_ready = false;
     compressed_prepare(P);
+    // the FP64 M2L: by convolution, unless the host gave M2L tables (they are used as given)
+    // or the surface is no lattice's; then from dense tables
+    bool host_m2l = false;
+    for (int f = 0; f < P->n_fam; ++f)
+        for (int l = 2; l <= P->md; ++l) host_m2l = host_m2l || P->tables[f][l].host_m2l;
+    P->conv.on = false;
+    if (P->conv.ok && !host_m2l) {
+        conv_schedule(P);
+        if (conv_fits(P)) {
+            if (!P->conv.tables) conv_tables(P);
+            P->conv.on = true;
+        }
+    }
+    if (!P->conv.on && !P->streamed)
+        for (int f = 0; f < P->n_fam; ++f)
+            for (int l = 2; l <= P->md; ++l)
+                if (!P->tables[f][l].m2l.p) generate_m2l(P, f, l, P->tables[f][l].m2l);
     PlanExtra* X = extra(P, true);
     build_a_ptrs(P, X->ix);   // streamed plans without a workspace yet: see evaluate
     if (!P->crit) {
@@ -1123,13 +1156,17 @@ int hfmm_plan_finalize(hfmm_plan* P) {
         } else if (P->streamed) {
             if (P->ws) stream_maps(P);
         } else {
+            DevBuf<double> dense;   // one level's matrices, for their halves only
             for (int f = 0; f < P->n_fam; ++f)
                 for (int l = 2; l <= P->md; ++l) {
                     LevelTables& T = P->tables[f][l];
                     const int nm = (int)madj.size();
-                    T.m2l_hi.alloc(nm * mat);
-                    T.m2l_lo.alloc(nm * mat);
-                    split_transpose_tables(T.m2l.p, T.m2l_hi.p, T.m2l_lo.p, P->ld, nm);
+                    if (!T.m2l_hi.p) {
+                        if (!T.m2l.p) generate_m2l(P, f, l, dense);
+                        T.m2l_hi.alloc(nm * mat);
+                        T.m2l_lo.alloc(nm * mat);
+                        split_transpose_tables(T.m2l.p ? T.m2l.p : dense.p, T.m2l_hi.p, T.m2l_lo.p, P->ld, nm);
+                    }
                     make_table_map(&maps[l].a_hi[f], T.m2l_hi.p, P->ld, nm);
                     make_table_map(&maps[l].a_lo[f], T.m2l_lo.p, P->ld, nm);
                 }

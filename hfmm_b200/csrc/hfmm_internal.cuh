@@ -83,7 +83,9 @@ struct LevelTables {
     DevBuf<double> dn_U, dn_d, dn_Vt;
     DevBuf<double> m2m;                 // 8 x (A^T) for this level as PARENT
     DevBuf<double> l2l;                 // 8 x (A^T) for this level as CHILD
-    DevBuf<double> m2l;                 // 316 x (A^T), non-adjacent displacements
+    DevBuf<double> m2l;                 // 316 x (A^T), non-adjacent displacements (host-given,
+                                        // or where the convolution does not apply)
+    bool host_m2l = false;
     // rotation-based M2L (m2l_rotation.cu): multipole-from-equivalent Q, check-from-local
     // E (complex, interleaved) and the coaxial shift matrices of every distance
     DevBuf<double> rot_Q, rot_E, rot_C;
@@ -120,11 +122,26 @@ struct LevelTables {
         grid = 0;
         xg_hi.release(); xg_lo.release();
         m2m_f.release(); l2l_f.release(); cmp_f.release(); exp_f.release();
-        set = false;
+        set = host_m2l = false;
     }
 };
 
 struct hfmm_plan_impl;
+
+// The FP64 M2L by convolution (m2l_conv.cu): the surface's lattice, the displacements'
+// spectra, the tree's slots (one per parent: its eight children) and the workspace.
+struct ConvPlan {
+    bool ok = false;       // the equivalent surface is a lattice cube's
+    bool on = false;       // the FP64 evaluate's M2L (else the dense tables)
+    bool tables = false;   // K holds the current kernel's and levels' spectra
+    int n = 0, n_slots = 0, n_groups = 0;
+    double spacing = 0.0;
+    DevBuf<int32_t> pos, line_off, line_k;   // surface points in lattice line order
+    DevBuf<double> tw, K;
+    DevBuf<int32_t> child, nbr;              // [slot][8] boxes, [slot][26] neighbour slots
+    DevBuf<int4> groups;                     // (level, first slot, slots)
+    DevBuf<double> ws;                       // X and Y of one chunk (streamed plans: P->ws)
+};
 
 }  // namespace hfmm
 
@@ -223,6 +240,7 @@ struct hfmm_plan {
     hfmm::DevBuf<const double*> a_ptrs;     // device arrays of A pointers per GEMM call
     std::vector<const double*> h_a_ptrs;
     size_t a_ptr_cursor = 0;
+    hfmm::ConvPlan conv;
 
     // evaluate scratch (allocated at finalize for R = 2)
     hfmm::DevBuf<double> q_s;        // R x n sorted charges
@@ -248,6 +266,14 @@ void lists_build(hfmm_plan* P);
 void schedules_build(hfmm_plan* P);
 void upload_level(hfmm_plan* P, int fam, int level, const double* const* h);
 void generate_tables(hfmm_plan* P, int fam, int level);
+void generate_m2l(hfmm_plan* P, int fam, int level, DevBuf<double>& out);
+// M2L by convolution (m2l_conv.cu): the lattice of the surface given to set_kernel; the
+// spectra; the current tree's slots and workspace; one evaluate's M2L into P->check
+bool conv_surface(hfmm_plan* P, const double* equiv);
+void conv_tables(hfmm_plan* P);
+void conv_schedule(hfmm_plan* P);
+bool conv_fits(const hfmm_plan* P);
+void conv_m2l(hfmm_plan* P, int R, int64_t fam_stride, cudaStream_t s);
 size_t stream_ws_bytes(const hfmm_plan* P);
 bool plan_profiling(hfmm_plan* P);
 void batch_forget_plan(struct hfmm_batch* B, hfmm_plan* P);

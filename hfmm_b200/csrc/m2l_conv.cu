@@ -1,0 +1,685 @@
+// FP64 M2L as a convolution. Both M2L surfaces are the same regular grid (surface points
+// of a p x p x p lattice, kifmm/surfaces.py:40-85 at radius 1.05), so the matrix of one
+// displacement d, G(x_m + 2 d - y_k), depends on the lattice lag m - k alone: a translation
+// (phases.py:211-236) is a 3-D convolution of p^3 values with (2p-1)^3 lags. A cyclic
+// transform of n = 2p - 1 points per axis makes it exact, and every displacement a
+// multiplication by a number per frequency, summed over the V list before one inverse
+// transform per target:
+//     X = F(x) of every box;   Y_t = sum_d K_d .* X_{s(t, d)};   check_t = F^-1(Y_t).
+// Complex charges travel as one complex sequence (the kernel is real), real charges as the
+// half spectrum. Against the dense tables (2 n_s^2 a pair and column) that is 8 n^3 a pair
+// and column pair: 27 against 350 kFLOP at p = 8, 97 against 2,120 at p = 12. One
+// evaluate, complex charges, field (B200): 1e6 points, p = 8, depth 5: 210.2 -> 42.8 ms;
+// 20,000 points, depth 3: p = 8 6.69 -> 1.55 ms, p = 12 32.7 -> 3.68 ms.
+//
+// Work is laid out by PARENT: the children of one parent ("slot") sit side by side, absent
+// ones as zeros, X as [frequency][slot][child]. The products of one frequency and one of
+// the 26 parent offsets D are then an 8 x 8 complex block (target child x source child), the
+// same for every slot: a small matrix times the columns of all slots, which the FP64 tensor
+// instruction m16n8k4 takes as it is (16 rows = re and im of 8 target children). 1,512 of
+// its 1,664 products are V pairs; the adjacent ones multiply a stored zero.
+#include "hfmm_internal.cuh"
+#include "m2l_conv.cuh"
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+namespace hfmm {
+
+namespace {
+
+// K of one frequency in shared memory, [dx + 3][dy + 3][dz + 3] with strides 66, 9, 1: a
+// phase of eight lanes reads (two target children) x (four source children), offsets
+// {-66, 0, 66} - {0, 9}, which are distinct 16-byte banks mod 8.
+constexpr int KSX = 66, KSY = 9, KTAB = 6 * KSX + 6 * KSY + 7;
+
+__device__ __forceinline__ void dmma(double (&c)[4], double a0, double a1, double b0) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+        "{%0,%1,%2,%3};\n"
+        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+        : "d"(a0), "d"(a1), "d"(b0));
+}
+
+// ---------------------------------------------------------------- tables
+// G at lag (ax, ay, az) of displacement slot d, layout [cell][343] (d fastest, as in every
+// pass below); fam as in tables.cu: 0 cos(kr)/r, 1 sin(kr)/r, 2 exp(-kr)/(4 pi r).
+__global__ void k_conv_gen(int p, int n, double spacing, double s, double kw, int fam, double* out) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= (int64_t)n * n * n * N_DISP) return;
+    const int d = (int)(i % N_DISP);
+    const int cell = (int)(i / N_DISP);
+    const int dx = d / 49 - 3, dy = (d / 7) % 7 - 3, dz = d % 7 - 3;
+    const int near = max(abs(dx), max(abs(dy), abs(dz)));
+    double v = 0.0;
+    if (near > 1) {
+        const int a[3] = {cell % n, (cell / n) % n, cell / (n * n)};
+        const int dd[3] = {dx, dy, dz};
+        double x[3];
+        for (int c = 0; c < 3; ++c) x[c] = (2.0 * dd[c] + spacing * (a[c] < p ? a[c] : a[c] - n)) * s;
+        const double r = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
+        if (fam == 2) {
+            v = exp(-kw * r) / (4.0 * M_PI * r);
+        } else {
+            double sn, cs;
+            sincos(kw * r, &sn, &cs);
+            v = (fam == 1 ? sn : cs) / r;
+        }
+    }
+    out[i] = v;
+}
+
+// One axis of the tables' transform: out[hi][k][lo][d] = scale sum_a in[hi][a][lo][d] w^(a k)
+// for k < nk, w = e^{-2 pi i / n}; `lo` cells vary faster than the axis. REAL: in is real.
+template <bool REAL>
+__global__ void k_conv_axis(const double* __restrict__ in, int n, int nk, int64_t n_lo, int64_t total,
+                            const double2* __restrict__ tw, double scale, double2* out) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= total) return;
+    const int64_t lo = i % n_lo;
+    const int k = (int)((i / n_lo) % nk);
+    const int64_t hi = i / (n_lo * nk);
+    double re = 0.0, im = 0.0;
+    int m = 0;
+    for (int a = 0; a < n; ++a) {
+        const double2 w = tw[m];
+        const int64_t src = (hi * n + a) * n_lo + lo;
+        if (REAL) {
+            const double x = in[src];
+            re = fma(x, w.x, re);
+            im = fma(-x, w.y, im);
+        } else {
+            const double2 x = reinterpret_cast<const double2*>(in)[src];
+            re = fma(x.x, w.x, fma(x.y, w.y, re));
+            im = fma(x.y, w.x, fma(-x.x, w.y, im));
+        }
+        m += k;
+        if (m >= n) m -= n;
+    }
+    out[i] = make_double2(re * scale, im * scale);
+}
+
+// ---------------------------------------------------------------- schedule
+// nbr[slot][D]: the slot of the parent at offset D when it holds a V source of this slot's
+// children (read off the M2L source table), else the zero slot.
+__global__ void k_conv_nbr(const int32_t* __restrict__ child, const int32_t* __restrict__ m2l_src,
+                           const int32_t* __restrict__ p_id, const int32_t* __restrict__ slot_of,
+                           int n_slots, int32_t* nbr) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_slots * 26) return;
+    const int slot = i / 26, D = i % 26;
+    int ox, oy, oz;
+    neigh_offset(D, ox, oy, oz);
+    int found = n_slots;
+    for (int t = 0; t < 8 && found == n_slots; ++t) {
+        const int b = child[slot * 8 + t];
+        if (b < 0) continue;
+        for (int s = 0; s < 8; ++s) {
+            const int dx = -2 * ox + (t & 1) - (s & 1);
+            const int dy = -2 * oy + ((t >> 1) & 1) - ((s >> 1) & 1);
+            const int dz = -2 * oz + ((t >> 2) & 1) - ((s >> 2) & 1);
+            if (max(abs(dx), max(abs(dy), abs(dz))) <= 1) continue;
+            const int src = m2l_src[(int64_t)b * M2L_ENTRIES + (dx + 3) * 49 + (dy + 3) * 7 + dz + 3];
+            if (src >= 0) {
+                found = slot_of[p_id[src]];
+                break;
+            }
+        }
+    }
+    nbr[i] = found;
+}
+
+// ---------------------------------------------------------------- transforms
+// Sums over one axis folded by the pair (k, n - k): with v_j real or complex,
+//   C = sum_j v_j cos(2 pi j k / n), S = sum_j v_j sin(2 pi j k / n),
+//   X_k = C - i S, X_(n-k) = C + i S,
+// four FMAs per term and pair instead of eight. PK pairs per thread share each v_j load.
+constexpr int PK = 4;
+
+__device__ __forceinline__ void axis_pairs(const double2* v, int stride, int p, int n, int k0,
+                                           const double2* tw, double2 (&C)[PK], double2 (&S)[PK]) {
+    int m[PK], kk[PK];
+#pragma unroll
+    for (int u = 0; u < PK; ++u) {
+        C[u] = S[u] = make_double2(0.0, 0.0);
+        m[u] = 0;
+        kk[u] = min(k0 + u, n - 1);
+    }
+    for (int j = 0; j < p; ++j) {
+        const double2 x = v[j * stride];
+#pragma unroll
+        for (int u = 0; u < PK; ++u) {
+            const double2 w = tw[m[u]];
+            C[u].x = fma(x.x, w.x, C[u].x);
+            C[u].y = fma(x.y, w.x, C[u].y);
+            S[u].x = fma(x.x, w.y, S[u].x);
+            S[u].y = fma(x.y, w.y, S[u].y);
+            m[u] += kk[u];
+            if (m[u] >= n) m[u] -= n;
+        }
+    }
+}
+
+// Forward transform of a slot's children (c.CH of them per CTA): the frequencies of rows
+// kz in [kz0, kz1) x ky in [ky0, ky1), all kx. Per kz: z sums of the surface lines (interior
+// lines hold two points), then y, then x; the x stage writes 16 bytes x 8 children a
+// frequency. Bound by its stores (16 n^3 bytes a box) once the folded sums are this cheap.
+template <int R>
+__global__ void __launch_bounds__(256) k_conv_fwd(ConvCall c) {
+    extern __shared__ double2 sh[];
+    const int p = c.p, n = c.n, nh = (n + 1) / 2, CH = c.CH, nky = c.ky1 - c.ky0;
+    const int slot = blockIdx.x, c0 = blockIdx.y * CH, fam = blockIdx.z;
+    double2* tw = sh;                       // n
+    double2* A1 = tw + n;                   // [p * p][CH]
+    double2* A2 = A1 + p * p * CH;          // [p][nky][CH]
+    double* xs = reinterpret_cast<double*>(A2 + p * nky * CH);   // [n_s][CH][R]
+    const int nkx = R == 2 ? n : nh;
+    const int64_t fstride = (int64_t)(c.n_slots + 1) * 8;   // values of one frequency
+    double2* X = c.X + (int64_t)fam * c.rows * nkx * fstride + (int64_t)slot * 8 + c0;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    if (slot == c.n_slots) {   // the zero slot
+        for (int64_t i = tid; i < (int64_t)c.rows * nkx * CH; i += nt)
+            X[(i / CH) * fstride + i % CH] = make_double2(0.0, 0.0);
+        return;
+    }
+    for (int i = tid; i < n; i += nt) tw[i] = c.tw[i];
+    for (int ch = 0; ch < CH; ++ch) {
+        const int b = c.child[slot * 8 + c0 + ch];
+        const double* src = c.dens + (int64_t)fam * c.fam_stride + (int64_t)b * R * c.ld;
+        for (int i = tid; i < R * c.n_s; i += nt) {
+            const int r = i / c.n_s, s = i - r * c.n_s;
+            xs[(c.pos[s] * CH + ch) * R + r] = b >= 0 ? src[r * c.ld + s] : 0.0;
+        }
+    }
+    const int groups = (nh + PK - 1) / PK;
+    for (int kz = c.kz0; kz < c.kz1; ++kz) {
+        __syncthreads();
+        for (int it = tid; it < p * p * CH; it += nt) {   // z: the lines' points
+            const int ch = it % CH, line = it / CH, i = line / p, j = line - i * p;
+            const bool edge = i == 0 || j == 0 || i == p - 1 || j == p - 1;
+            const int e0 = c.line_off[line], cnt = edge ? p : 2;
+            const int step = edge ? kz : (int)(((int64_t)(p - 1) * kz) % n);
+            double re = 0.0, im = 0.0;
+            int m = 0;
+            for (int q = 0; q < cnt; ++q) {
+                const double2 w = tw[m];
+                const double* x = xs + ((e0 + q) * CH + ch) * R;
+                re = fma(x[0], w.x, re);
+                im = fma(-x[0], w.y, im);
+                if (R == 2) {
+                    re = fma(x[1], w.y, re);
+                    im = fma(x[1], w.x, im);
+                }
+                m += step;
+                if (m >= n) m -= n;
+            }
+            A1[it] = make_double2(re, im);
+        }
+        __syncthreads();
+        for (int it = tid; it < p * CH * groups; it += nt) {   // y
+            const int ch = it % CH, i = (it / CH) % p, k0 = (it / (CH * p)) * PK;
+            double2 C[PK], S[PK];
+            axis_pairs(A1 + i * p * CH + ch, CH, p, n, k0, tw, C, S);
+#pragma unroll
+            for (int u = 0; u < PK; ++u) {
+                const int k = k0 + u, km = n - k;
+                if (k >= nh) break;
+                if (k >= c.ky0 && k < c.ky1)
+                    A2[(i * nky + k - c.ky0) * CH + ch] = make_double2(C[u].x + S[u].y, C[u].y - S[u].x);
+                if (k > 0 && km >= c.ky0 && km < c.ky1)
+                    A2[(i * nky + km - c.ky0) * CH + ch] = make_double2(C[u].x - S[u].y, C[u].y + S[u].x);
+            }
+        }
+        __syncthreads();
+        const int64_t row0 = (int64_t)(kz - c.kz0) * nky;
+        for (int it = tid; it < nky * CH * groups; it += nt) {   // x, to memory
+            const int ch = it % CH, ky = (it / CH) % nky, k0 = (it / (CH * nky)) * PK;
+            double2 C[PK], S[PK];
+            axis_pairs(A2 + ky * CH + ch, nky * CH, p, n, k0, tw, C, S);
+            double2* o = X + (row0 + ky) * nkx * fstride + ch;
+#pragma unroll
+            for (int u = 0; u < PK; ++u) {
+                const int k = k0 + u;
+                if (k >= nh) break;
+                o[k * fstride] = make_double2(C[u].x + S[u].y, C[u].y - S[u].x);
+                if (R == 2 && k > 0) o[(n - k) * fstride] = make_double2(C[u].x - S[u].y, C[u].y + S[u].x);
+            }
+        }
+    }
+}
+
+// The products of one frequency and CONV_GROUP slots: per offset D and four source children,
+// A = the 16 x 4 block of K (rows: re and im of the eight target children) against re and
+// im of the sources, 8 slots per instruction; NT slot tiles per warp share each A. FP64
+// tensor work is the bound (the CTA's X rows, 128 bytes a slot, hit L1 after the first
+// offsets); K and the neighbour lists come from shared memory.
+constexpr int NT = 2, CONV_WARPS = 4, CONV_GROUP = 8 * NT * CONV_WARPS;
+
+__global__ void __launch_bounds__(32 * CONV_WARPS) k_conv_mul(ConvCall c, int nkx) {
+    __shared__ double2 Kt[KTAB];
+    __shared__ int nb[CONV_GROUP][27];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int grp = blockIdx.x % c.n_groups;
+    const int64_t f = blockIdx.x / c.n_groups;      // frequency within the chunk
+    const int fam = blockIdx.y;
+    const int4 G = c.groups[grp];                   // level, first slot, slots
+    const int nky = c.ky1 - c.ky0;
+    {
+        const int row = (int)(f / nkx), n = c.n, nh = (n + 1) / 2;
+        int kx = (int)(f % nkx), ky = c.ky0 + row % nky, kz = c.kz0 + row / nky;
+        const bool mirror = kx >= nh;   // K is real: the other half is the conjugate
+        if (mirror) {
+            kx = n - kx;
+            ky = ky ? n - ky : 0;
+            kz = kz ? n - kz : 0;
+        }
+        const double2* K = c.K + (((int64_t)(G.x - 2) * c.n_fam + fam) * n * n * nh +
+                                  ((int64_t)kz * n + ky) * nh + kx) * N_DISP;
+        for (int d = tid; d < N_DISP; d += 32 * CONV_WARPS) {
+            double2 v = K[d];
+            if (mirror) v.y = -v.y;
+            Kt[(d / 49) * KSX + ((d / 7) % 7) * KSY + d % 7] = v;
+        }
+        for (int i = tid; i < CONV_GROUP * 26; i += 32 * CONV_WARPS) {
+            const int s = i / 26, D = i - s * 26;
+            nb[s][D] = s < G.z ? c.nbr[(int64_t)(G.y + s) * 26 + D] : c.n_slots;
+        }
+    }
+    __syncthreads();
+    const int t0 = warp * NT * 8;   // the warp's first slot in the group
+    if (t0 >= G.z) return;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int64_t fstride = (int64_t)(c.n_slots + 1) * 8;
+    const int64_t fo = ((int64_t)fam * c.rows * nkx + f) * fstride;
+    const double2* X = c.X + fo + t4;
+    const int off_t = (g & 1) * KSX + ((g >> 1) & 1) * KSY + (g >> 2);
+    const int off_s = (t4 & 1) * KSX + (t4 >> 1) * KSY;
+    const double2* Kl = Kt + 3 * (KSX + KSY + 1) + off_t - off_s;   // source children 4.. are one z further
+    double acc[NT][4];
+#pragma unroll
+    for (int a = 0; a < NT; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
+    double2 x[2][NT][2];
+    auto load = [&](int D, double2 (&v)[NT][2]) {
+#pragma unroll
+        for (int a = 0; a < NT; ++a) {
+            const double2* q = X + (int64_t)nb[t0 + a * 8 + g][D] * 8;
+            v[a][0] = __ldg(q);
+            v[a][1] = __ldg(q + 4);
+        }
+    };
+    auto mul = [&](int D, const double2 (&v)[NT][2]) {
+        int ox, oy, oz;
+        neigh_offset(D, ox, oy, oz);
+        const double2* Kd = Kl - 2 * (ox * KSX + oy * KSY + oz);
+        const double2 k0 = Kd[0], k1 = Kd[-1];
+#pragma unroll
+        for (int a = 0; a < NT; ++a) dmma(acc[a], k0.x, k0.y, v[a][0].x);
+#pragma unroll
+        for (int a = 0; a < NT; ++a) dmma(acc[a], -k0.y, k0.x, v[a][0].y);
+#pragma unroll
+        for (int a = 0; a < NT; ++a) dmma(acc[a], k1.x, k1.y, v[a][1].x);
+#pragma unroll
+        for (int a = 0; a < NT; ++a) dmma(acc[a], -k1.y, k1.x, v[a][1].y);
+    };
+    load(0, x[0]);
+#pragma unroll 1
+    for (int D = 0; D < 26; D += 2) {
+        load(D + 1, x[1]);
+        mul(D, x[0]);
+        if (D + 2 < 26) load(D + 2, x[0]);
+        mul(D + 1, x[1]);
+    }
+    double2* Y = c.Y + fo + g;
+#pragma unroll
+    for (int a = 0; a < NT; ++a) {
+        const int s = t0 + a * 8 + 2 * t4;
+        if (s < G.z) Y[(int64_t)(G.y + s) * 8] = make_double2(acc[a][0], acc[a][2]);
+        if (s + 1 < G.z) Y[(int64_t)(G.y + s + 1) * 8] = make_double2(acc[a][1], acc[a][3]);
+    }
+}
+
+// Inverse transform of a slot's children onto the surface points: per kz the x sums (folded
+// by (k, n - k)) straight from memory, the y sums, then every surface point's z term, added
+// into the points' sums in kz order. The sums start from 0 on the first chunk and from the
+// check potentials after, so whole-plane chunks of any number give the same bits. Bound by
+// the reads of Y. R = 1: the half spectrum, terms kx > 0 doubled, real part kept.
+template <int R>
+__global__ void __launch_bounds__(256) k_conv_inv(ConvCall c) {
+    extern __shared__ double2 sh[];
+    const int p = c.p, n = c.n, nh = (n + 1) / 2, CH = c.CH, nky = c.ky1 - c.ky0;
+    const int slot = blockIdx.x, c0 = blockIdx.y * CH, fam = blockIdx.z;
+    double2* tw = sh;                       // n
+    double2* U2 = tw + n;                   // [p][nky][CH]
+    double2* U1 = U2 + p * nky * CH;        // [p * p][CH]
+    double* acc = reinterpret_cast<double*>(U1 + p * p * CH);   // [n_s][CH][R]
+    const int nkx = R == 2 ? n : nh;
+    const int64_t fstride = (int64_t)(c.n_slots + 1) * 8;
+    const double2* Y = c.Y + (int64_t)fam * c.rows * nkx * fstride + (int64_t)slot * 8 + c0;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    for (int i = tid; i < n; i += nt) tw[i] = c.tw[i];
+    for (int ch = 0; ch < CH; ++ch) {
+        const int b = c.child[slot * 8 + c0 + ch];
+        const double* src = c.check + (int64_t)fam * c.fam_stride + (int64_t)b * R * c.ld;
+        for (int i = tid; i < R * c.n_s; i += nt) {
+            const int r = i / c.n_s, s = i - r * c.n_s;
+            acc[(c.pos[s] * CH + ch) * R + r] = c.first || b < 0 ? 0.0 : src[r * c.ld + s];
+        }
+    }
+    const int groups = (p + PK - 1) / PK;
+    for (int kz = c.kz0; kz < c.kz1; ++kz) {
+        __syncthreads();
+        const int64_t row0 = (int64_t)(kz - c.kz0) * nky;
+        for (int it = tid; it < nky * CH * groups; it += nt) {   // x, from memory
+            const int ch = it % CH, ky = (it / CH) % nky, i0 = (it / (CH * nky)) * PK;
+            const double2* y = Y + (row0 + ky) * nkx * fstride + ch;
+            const double2 y0 = y[0];
+            double2 u[PK];
+            int m[PK], ii[PK];
+#pragma unroll
+            for (int a = 0; a < PK; ++a) {
+                u[a] = y0;
+                ii[a] = min(i0 + a, p - 1);
+                m[a] = ii[a];
+            }
+            for (int k = 1; k < nh; ++k) {
+                const double2 a0 = y[k * fstride];
+                double2 P, M;
+                if (R == 2) {
+                    const double2 a1 = y[(n - k) * fstride];
+                    P = make_double2(a0.x + a1.x, a0.y + a1.y);
+                    M = make_double2(a0.x - a1.x, a0.y - a1.y);
+                } else {
+                    P = M = make_double2(2.0 * a0.x, 2.0 * a0.y);
+                }
+#pragma unroll
+                for (int a = 0; a < PK; ++a) {
+                    const double2 w = tw[m[a]];
+                    u[a].x = fma(P.x, w.x, fma(-M.y, w.y, u[a].x));
+                    u[a].y = fma(P.y, w.x, fma(M.x, w.y, u[a].y));
+                    m[a] += ii[a];
+                    if (m[a] >= n) m[a] -= n;
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < PK; ++a)
+                if (i0 + a < p) U2[((i0 + a) * nky + ky) * CH + ch] = u[a];
+        }
+        __syncthreads();
+        for (int it = tid; it < p * CH * groups; it += nt) {   // y
+            const int ch = it % CH, i = (it / CH) % p, j0 = (it / (CH * p)) * PK;
+            double2 u[PK];
+            int m[PK], jj[PK];
+#pragma unroll
+            for (int a = 0; a < PK; ++a) {
+                u[a] = make_double2(0.0, 0.0);
+                jj[a] = min(j0 + a, p - 1);
+                m[a] = (int)(((int64_t)c.ky0 * jj[a]) % n);
+            }
+            for (int ky = 0; ky < nky; ++ky) {
+                const double2 y = U2[(i * nky + ky) * CH + ch];
+#pragma unroll
+                for (int a = 0; a < PK; ++a) {
+                    const double2 w = tw[m[a]];
+                    u[a].x = fma(y.x, w.x, fma(-y.y, w.y, u[a].x));
+                    u[a].y = fma(y.y, w.x, fma(y.x, w.y, u[a].y));
+                    m[a] += jj[a];
+                    if (m[a] >= n) m[a] -= n;
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < PK; ++a)
+                if (j0 + a < p) U1[(i * p + j0 + a) * CH + ch] = u[a];
+        }
+        __syncthreads();
+        for (int it = tid; it < c.n_s * CH; it += nt) {   // z: each surface point's own term
+            const int ch = it % CH, e = it / CH, lk = c.line_k[e];
+            const double2 y = U1[(lk >> 8) * CH + ch], w = tw[((lk & 255) * kz) % n];
+            double* a = acc + it * R;
+            a[0] = fma(y.x, w.x, fma(-y.y, w.y, a[0]));
+            if (R == 2) a[1] = fma(y.y, w.x, fma(y.x, w.y, a[1]));
+        }
+    }
+    __syncthreads();
+    for (int ch = 0; ch < CH; ++ch) {
+        const int b = c.child[slot * 8 + c0 + ch];
+        if (b < 0) continue;
+        double* dst = c.check + (int64_t)fam * c.fam_stride + (int64_t)b * R * c.ld;
+        for (int i = tid; i < R * c.n_s; i += nt) {
+            const int r = i / c.n_s, s = i - r * c.n_s;
+            dst[r * c.ld + s] = acc[(c.pos[s] * CH + ch) * R + r];
+        }
+    }
+}
+
+// shared memory of the transform kernels for CH children and nky rows of a plane
+size_t transform_smem(int p, int n_s, int R, int CH, int nky) {
+    return ((size_t)(2 * p - 1) + (size_t)CH * (p * p + p * nky)) * sizeof(double2) +
+           (size_t)n_s * CH * R * sizeof(double);
+}
+
+constexpr size_t SMEM_MAX = 227 * 1024;
+// The transforms' working set when the plan owns it: chunks of whole planes up to this
+// size (1e6 points, p = 8: 8 GiB of spectra in all, four chunks; larger chunks measured
+// the same, smaller ones add launches)
+constexpr size_t CONV_WS = (size_t)2 << 30;
+
+int64_t chunk_values(const hfmm_plan* P, int nkx, int nf) {   // values of one (ky, kz) row
+    return (int64_t)nkx * (P->conv.n_slots + 1) * 8 * nf;
+}
+
+}  // namespace
+
+// The surface as lattice points: false when the points given are not the p x p x p
+// lattice's surface (then the dense tables serve).
+bool conv_surface(hfmm_plan* P, const double* equiv) {
+    ConvPlan& C = P->conv;
+    C.ok = false;
+    const int p = P->p, n_s = P->n_s;
+    if (p < 2 || p > 255) return false;
+    double r0 = 0.0;
+    for (int i = 0; i < 3 * n_s; ++i) r0 = std::max(r0, std::fabs(equiv[i]));
+    if (!(r0 > 0.0) || !std::isfinite(r0)) return false;
+    C.spacing = 2.0 * r0 / (p - 1);
+    std::vector<int32_t> at((size_t)p * p * p, -1);
+    for (int s = 0; s < n_s; ++s) {
+        int g[3];
+        bool face = false;
+        for (int a = 0; a < 3; ++a) {
+            const double t = (equiv[3 * s + a] + r0) / C.spacing;
+            g[a] = (int)std::lround(t);
+            if (!(std::fabs(t - g[a]) < 1e-11) || g[a] < 0 || g[a] >= p) return false;
+            face = face || g[a] == 0 || g[a] == p - 1;
+        }
+        int32_t& cell = at[((size_t)g[0] * p + g[1]) * p + g[2]];
+        if (!face || cell >= 0) return false;
+        cell = s;
+    }
+    // points in line order (x, y lattice column, then z): every surface cell must be there
+    std::vector<int32_t> pos(n_s), off((size_t)p * p), lk(n_s);
+    int e = 0;
+    for (int i = 0; i < p; ++i)
+        for (int j = 0; j < p; ++j) {
+            off[(size_t)i * p + j] = e;
+            const bool edge = i == 0 || j == 0 || i == p - 1 || j == p - 1;
+            for (int k = 0; k < p; k += (edge || p == 2) ? 1 : p - 1) {
+                const int s = at[((size_t)i * p + j) * p + k];
+                if (s < 0 || e >= n_s) return false;
+                pos[s] = e;
+                lk[e++] = ((i * p + j) << 8) | k;
+            }
+        }
+    if (e != n_s) return false;
+    // at least one child per CTA must fit
+    if (transform_smem(p, n_s, 2, 1, 2 * p - 1) > SMEM_MAX) return false;
+    C.n = 2 * p - 1;
+    std::vector<double> tw(2 * C.n);
+    for (int i = 0; i < C.n; ++i) {
+        const long double a = 2.0L * 3.141592653589793238462643383279502884L * i / C.n;
+        tw[2 * i] = (double)std::cos(a);
+        tw[2 * i + 1] = (double)std::sin(a);
+    }
+    auto up = [](auto& buf, const auto& h) {
+        buf.alloc(h.size());
+        HFMM_CUDA(cudaMemcpy(buf.p, h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice));
+    };
+    up(C.pos, pos);
+    up(C.line_off, off);
+    up(C.line_k, lk);
+    up(C.tw, tw);
+    C.tables = false;
+    C.ok = true;
+    return true;
+}
+
+// Spectra of every level's and family's 316 displacements, half of the frequencies (kx <=
+// n / 2; K is real), [level - 2][family][kz][ky][kx][343].
+void conv_tables(hfmm_plan* P) {
+    ConvPlan& C = P->conv;
+    const int n = C.n, nh = (n + 1) / 2, nl = P->md - 1;
+    const int64_t per = (int64_t)n * n * nh * N_DISP;
+    C.K.alloc((size_t)std::max(nl, 1) * P->n_fam * per * 2);
+    DevBuf<double> a, b;
+    a.alloc((size_t)n * n * n * N_DISP);
+    b.alloc((size_t)per * 2);
+    DevBuf<double> t;
+    t.alloc((size_t)per * 2);
+    const double2* tw = reinterpret_cast<const double2*>(C.tw.p);
+    auto blocks = [](int64_t m) { return (unsigned)ceil_div(m, 256); };
+    for (int l = 2; l <= P->md; ++l)
+        for (int f = 0; f < P->n_fam; ++f) {
+            const double s = P->extent * std::ldexp(1.0, -(l + 1));
+            const int64_t cells = (int64_t)n * n * n * N_DISP;
+            HFMM_LAUNCH(k_conv_gen, blocks(cells), 256, 0, 0, P->p, n, C.spacing, s, P->k,
+                        P->yukawa ? 2 : f, a.p);
+            double2* tp = reinterpret_cast<double2*>(t.p);
+            double2* bp = reinterpret_cast<double2*>(b.p);
+            double2* K = reinterpret_cast<double2*>(C.K.p) + ((int64_t)(l - 2) * P->n_fam + f) * per;
+            HFMM_LAUNCH(k_conv_axis<true>, blocks(per), 256, 0, 0, a.p, n, nh, (int64_t)N_DISP, per, tw, 1.0, tp);
+            HFMM_LAUNCH(k_conv_axis<false>, blocks(per), 256, 0, 0, t.p, n, n, (int64_t)nh * N_DISP, per, tw,
+                        1.0, bp);
+            HFMM_LAUNCH(k_conv_axis<false>, blocks(per), 256, 0, 0, b.p, n, n, (int64_t)n * nh * N_DISP, per,
+                        tw, 1.0 / ((double)n * n * n), K);
+        }
+    HFMM_CUDA(cudaDeviceSynchronize());
+    C.tables = true;
+}
+
+// Slots, neighbour lists and groups of the current tree, and the plan's own workspace.
+void conv_schedule(hfmm_plan* P) {
+    ConvPlan& C = P->conv;
+    std::vector<int32_t> slot_of(P->nb, -1), child;
+    std::vector<int4> groups;
+    int n_slots = 0;
+    for (int l = 2; l <= P->md; ++l) {
+        const int first = n_slots;
+        for (int b = P->level_lo[l]; b < P->level_hi[l]; ++b) {
+            int32_t& s = slot_of[P->h_p_id[b]];
+            if (s < 0) {
+                s = n_slots++;
+                child.insert(child.end(), 8, -1);
+            }
+            child[(size_t)s * 8 + (P->h_m_id[b] & 7ull)] = b;
+        }
+        for (int s = first; s < n_slots; s += CONV_GROUP)
+            groups.push_back(make_int4(l, s, std::min(CONV_GROUP, n_slots - s), 0));
+    }
+    C.n_slots = n_slots;
+    C.n_groups = (int)groups.size();
+    if (!n_slots) return;
+    auto up = [](auto& buf, const auto& h) {
+        buf.alloc(h.size());
+        HFMM_CUDA(cudaMemcpy(buf.p, h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice));
+    };
+    DevBuf<int32_t> so;
+    up(so, slot_of);
+    up(C.child, child);
+    up(C.groups, groups);
+    C.nbr.alloc((size_t)n_slots * 26);
+    HFMM_LAUNCH(k_conv_nbr, (unsigned)ceil_div((int64_t)n_slots * 26, 256), 256, 0, 0, C.child.p,
+                P->m2l_src.p, P->p_id.p, so.p, n_slots, C.nbr.p);
+    HFMM_CUDA(cudaDeviceSynchronize());
+    if (!P->streamed) {
+        // X and Y of as many whole planes as the limit holds; where not one fits, the limit
+        // (one family or some rows of a plane at a time), one row of one family at least
+        const size_t row = 2 * (size_t)chunk_values(P, C.n, 1) * sizeof(double2);
+        const size_t plane = row * C.n * P->n_fam;
+        const size_t planes = std::min<size_t>(C.n, CONV_WS / plane);
+        const size_t want = (planes ? plane * planes : std::max(row, CONV_WS)) / sizeof(double);
+        if (C.ws.n < want) C.ws.alloc(want);
+    } else {
+        C.ws.release();
+    }
+}
+
+bool conv_fits(const hfmm_plan* P) {   // a streamed plan's workspace must hold one row
+    if (!P->streamed) return true;
+    return 2 * (size_t)chunk_values(P, P->conv.n, 1) * sizeof(double2) <= stream_ws_bytes(P);
+}
+
+void conv_m2l(hfmm_plan* P, int R, int64_t fam_stride, cudaStream_t s) {
+    const ConvPlan& C = P->conv;
+    if (!C.n_slots) return;
+    ConvCall c{};
+    c.p = P->p;
+    c.n = C.n;
+    c.n_s = P->n_s;
+    c.ld = P->ld;
+    c.n_slots = C.n_slots;
+    c.n_groups = C.n_groups;
+    c.child = C.child.p;
+    c.nbr = C.nbr.p;
+    c.pos = C.pos.p;
+    c.line_off = C.line_off.p;
+    c.line_k = C.line_k.p;
+    c.groups = C.groups.p;
+    c.tw = reinterpret_cast<const double2*>(C.tw.p);
+    c.n_fam = P->n_fam;
+    c.fam_stride = fam_stride;
+    const int n = C.n, nkx = R == 2 ? n : (n + 1) / 2;
+    double* ws = P->streamed ? static_cast<double*>(P->ws) : C.ws.p;
+    const size_t ws_values = (P->streamed ? P->ws_bytes : C.ws.n * sizeof(double)) / sizeof(double2);
+    // families together when a plane of both fits, else one after the other; whole planes
+    // of frequencies, or rows of one plane where not even one fits
+    int nf = P->n_fam;
+    if (2 * (size_t)chunk_values(P, nkx, nf) * n > ws_values) nf = 1;
+    const size_t row = 2 * (size_t)chunk_values(P, nkx, nf);
+    const int planes = (int)std::min<size_t>(n, ws_values / (row * n));
+    const int rows = planes ? n : (int)std::min<size_t>(n, ws_values / row);
+    if (rows < 1) throw Error{HFMM_ERR_STATE, "convolution M2L: workspace too small"};
+    const int dz = std::max(planes, 1);
+    const int PT = 256;
+    int CH = 8;   // children per CTA of the transforms: all eight where they fit
+    while (CH > 1 && transform_smem(c.p, c.n_s, R, CH, rows) > SMEM_MAX) CH /= 2;
+    c.CH = CH;
+    const size_t smem = transform_smem(c.p, c.n_s, R, CH, rows);
+    auto fwd = R == 2 ? k_conv_fwd<2> : k_conv_fwd<1>;
+    auto inv = R == 2 ? k_conv_inv<2> : k_conv_inv<1>;
+    HFMM_CUDA(cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HFMM_CUDA(cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    for (int f = 0; f < P->n_fam; f += nf) {
+        c.dens = P->equiv.p + f * fam_stride;
+        c.check = P->check.p + f * fam_stride;
+        c.K = reinterpret_cast<const double2*>(C.K.p) + (int64_t)f * n * n * ((n + 1) / 2) * N_DISP;
+        c.first = 1;
+        for (int kz = 0; kz < n; kz += dz)
+            for (int ky = 0; ky < n; ky += rows) {
+                c.kz0 = kz;
+                c.kz1 = std::min(n, kz + dz);
+                c.ky0 = ky;
+                c.ky1 = std::min(n, ky + rows);
+                c.rows = (c.kz1 - c.kz0) * (c.ky1 - c.ky0);
+                c.X = reinterpret_cast<double2*>(ws);
+                c.Y = c.X + (int64_t)c.rows * chunk_values(P, nkx, nf);
+                HFMM_LAUNCH(fwd, dim3((unsigned)(c.n_slots + 1), (unsigned)(8 / CH), (unsigned)nf), PT, smem, s, c);
+                HFMM_LAUNCH(k_conv_mul, dim3((unsigned)((int64_t)c.rows * nkx * c.n_groups), (unsigned)nf),
+                            32 * CONV_WARPS, 0, s, c, nkx);
+                HFMM_LAUNCH(inv, dim3((unsigned)c.n_slots, (unsigned)(8 / CH), (unsigned)nf), PT, smem, s, c);
+                c.first = 0;
+            }
+    }
+}
+
+}  // namespace hfmm

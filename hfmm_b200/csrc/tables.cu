@@ -161,6 +161,14 @@ void generate_m2l_stream(hfmm_plan* P, int level, bool mixed, void* ws, cudaStre
                 P->n_fam, P->yukawa ? 1 : 0, mixed ? 1 : 0, ws);
 }
 
+void generate_m2l(hfmm_plan* P, int fam, int level, DevBuf<double>& out) {
+    const int ld = P->ld;
+    if (out.n != 316 * (size_t)ld * ld) out.alloc(316 * (size_t)ld * ld);
+    HFMM_LAUNCH(k_gen, dim3((unsigned)ceil_div(ld, 32), (unsigned)ceil_div(ld, 8), 316u), dim3(32, 8), 0, 0,
+                0, P->equiv_pts.p, P->check_pts.p, P->n_s, ld, P->extent * std::ldexp(1.0, -(level + 1)), P->k,
+                P->yukawa ? 2 : (fam == 1 ? 1 : 0), out.p);
+}
+
 void generate_tables(hfmm_plan* P, int fam, int level) {
     LevelTables& T = P->tables[fam][level];
     const int n_s = P->n_s, ld = P->ld;
@@ -173,13 +181,7 @@ void generate_tables(hfmm_plan* P, int fam, int level) {
     auto grid = [&](int count) {
         return dim3((unsigned)ceil_div(ld, 32), (unsigned)ceil_div(ld, 8), (unsigned)count);
     };
-    if (P->streamed) {
-        T.m2l.release();   // regenerated per evaluate (generate_m2l_stream)
-    } else {
-        T.m2l.alloc(316 * mat);
-        HFMM_LAUNCH(k_gen, grid(316), blk, 0, 0, 0, P->equiv_pts.p, P->check_pts.p, n_s, ld, s, P->k,
-                    imag, T.m2l.p);
-    }
+    T.m2l.release();   // dense M2L tables are made at finalize, where something reads them
     if (level < P->md) {
         T.m2m.alloc(8 * mat);
         HFMM_LAUNCH(k_gen, grid(8), blk, 0, 0, 1, P->equiv_pts.p, P->check_pts.p, n_s, ld, s_child,
