@@ -166,6 +166,8 @@ EvalView view(hfmm_plan* P) {
     v.ld = P->ld;
     v.k = P->k;
     v.yukawa = P->yukawa ? 1 : 0;
+    v.fast = !P->yukawa && P->n_fam == 2 && std::fabs(P->k) * P->extent < 2.5e4 && P->extent > 1e-100 &&
+             P->extent < 1e100;   // every distance met is under 4 extents
     v.pos_s = P->pos_s.p;
     v.pos_f = P->pos_f.p;
     v.q_s = P->q_s.p;
@@ -455,6 +457,7 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
     base.fam_stride = fs;
     base.pot = P->pot.p;
     base.fld = P->fld.p;
+    base.maxleaf = P->maxleaf;
 
     // The near field needs only the gathered charges: it runs on the plan's side
     // stream beside the whole far field and joins before L2P, which adds into the
@@ -702,6 +705,31 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
         PhaseTimer pt(X, s, 4);
         conv_m2l(P, R, fs, s);
     }
+    // The X list's P2L reads only charges: where no level's M2L overwrites the check
+    // potentials after this point, every level's targets go in one launch.
+    auto p2l = [&](int level) {
+        ParticlePass p = base;
+        p.op = ParticleOp::P2L;
+        p.rows = P->x_tgt.p;
+        p.nrows = P->n_x_tgt;
+        p.off = P->x_off.p;
+        p.srcs = P->x_src.p;
+        p.surf = P->equiv_pts.p;
+        p.out = P->check.p;
+        p.level = level;
+        return p;
+    };
+    const bool x_first = P->nX && (use_conv || use_cx);
+    if (x_first) {
+        PhaseTimer pt(X, s, 5);
+        if (use_cx)   // the X list's check potentials alone, decoded into y_dn below
+            for (int f = 0; f < NF; ++f)
+                for (int l = 2; l <= P->md; ++l)
+                    HFMM_CUDA(cudaMemsetAsync(P->check.p + f * fs + (int64_t)P->level_lo[l] * R * P->ld, 0,
+                                              (size_t)(P->level_hi[l] - P->level_lo[l]) * R * P->ld * sizeof(double),
+                                              s));
+        particles(p2l(-1), s);
+    }
     // ---- downward pass (M2L, L2L, then X-list P2L, then decode)
     for (int l = 2; l <= P->md; ++l) {
         if (P->streamed && !use_cx && !use_conv) {
@@ -762,23 +790,9 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
                  P->check.p);
         }
         if (P->nX) {
-            if (use_cx)   // the X list's check potentials alone, decoded into y_dn below
-                for (int f = 0; f < NF; ++f)
-                    HFMM_CUDA(cudaMemsetAsync(
-                        P->check.p + f * fs + (int64_t)P->level_lo[l] * R * P->ld, 0,
-                        (size_t)(P->level_hi[l] - P->level_lo[l]) * R * P->ld * sizeof(double), s));
-            ParticlePass p = base;
-            p.op = ParticleOp::P2L;
-            p.rows = P->x_tgt.p;
-            p.nrows = P->n_x_tgt;
-            p.off = P->x_off.p;
-            p.srcs = P->x_src.p;
-            p.surf = P->equiv_pts.p;
-            p.out = P->check.p;
-            p.level = l;
-            {
+            if (!x_first) {
                 PhaseTimer pt(X, s, 5);
-                particles(p, s);
+                particles(p2l(l), s);
             }
             if (use_cx)
                 gemm(K_DNU, l, P->dec_tiles[l][R - 1], nullptr, 0, P->check.p, nullptr, P->loc.p,
@@ -1179,8 +1193,8 @@ int hfmm_plan_finalize(hfmm_plan* P) {
     }
     plan_queue_build(P);
     P->q_s.alloc(2 * P->n);
-    P->pot.alloc((size_t)P->n_fam * 2 * P->n);
-    P->fld.alloc((size_t)P->n_fam * 2 * 3 * P->n);
+    P->pot.alloc((size_t)2 * P->n);       // real and imaginary part per particle
+    P->fld.alloc((size_t)2 * 3 * P->n);
     HFMM_CUDA(cudaDeviceSynchronize());
     P->finalized = true;
     return HFMM_OK;

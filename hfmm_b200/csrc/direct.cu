@@ -7,64 +7,32 @@
 // CTA writes its partial sums to scratch, and a second kernel adds the chunks
 // in a fixed order, so the result does not depend on scheduling.
 #include "hfmm_internal.cuh"
+#include "particles.cuh"
 
 #include <algorithm>
+#include <cstring>
+#include <type_traits>
 
 namespace hfmm {
 
 namespace {
 
-// sin and cos of a phase: Cody-Waite reduction against pi/2 with a two-part constant
-// (1.5707963267948966 + 6.123233995736766e-17, the first being pi/2 rounded to FP64,
-// both from pi itself) done with FMAs, so r = x - n pi/2 is exact to about 1e-28 for
-// |x| <= 1e5; then the Taylor series of sin and cos on |r| <= pi/4 (through r^15 and
-// r^16: the first omitted terms stay under 4.7e-17 and 2.1e-18) and the quadrant
-// n mod 4. Larger phases take sincos.
-__device__ __forceinline__ void sincos_reduced(double x, double* s, double* c) {
-    if (!(fabs(x) <= 1.0e5)) {
-        sincos(x, s, c);
-        return;
-    }
-    const double n = rint(x * 0.6366197723675814);   // x / (pi / 2), rounded
-    double r = fma(-n, 1.5707963267948966, x);
-    r = fma(-n, 6.123233995736766e-17, r);
-    const double r2 = r * r;
-    double ps = 1.0 / 1307674368000.0;               // 1/15!
-    ps = fma(ps, r2, -1.0 / 6227020800.0);           // -1/13!
-    ps = fma(ps, r2, 1.0 / 39916800.0);              // 1/11!
-    ps = fma(ps, r2, -1.0 / 362880.0);               // -1/9!
-    ps = fma(ps, r2, 1.0 / 5040.0);                  // 1/7!
-    ps = fma(ps, r2, -1.0 / 120.0);                  // -1/5!
-    ps = fma(ps, r2, 1.0 / 6.0);                     // 1/3!
-    double pc = -1.0 / 20922789888000.0;             // -1/16!
-    pc = fma(pc, r2, 1.0 / 87178291200.0);           // 1/14!
-    pc = fma(pc, r2, -1.0 / 479001600.0);            // -1/12!
-    pc = fma(pc, r2, 1.0 / 3628800.0);               // 1/10!
-    pc = fma(pc, r2, -1.0 / 40320.0);                // -1/8!
-    pc = fma(pc, r2, 1.0 / 720.0);                   // 1/6!
-    pc = fma(pc, r2, -1.0 / 24.0);                   // -1/4!
-    pc = fma(pc, r2, 0.5);                           // 1/2!
-    const double sr = fma(-r * r2, ps, r);           // sin r = r - r^3 (1/3! - ...)
-    const double cr = fma(-r2, pc, 1.0);             // cos r = 1 - r^2 (1/2! - ...)
-    switch ((int)((long long)n & 3)) {
-        case 0: *s = sr; *c = cr; break;
-        case 1: *s = cr; *c = -sr; break;
-        case 2: *s = -sr; *c = -cr; break;
-        default: *s = -cr; *c = sr; break;
-    }
-}
-
 constexpr int DT = 128;        // targets per CTA
 constexpr int DSTAGE = 256;    // sources staged per pass
 constexpr int NV = 8;          // phi re/im + field 3 x re/im
 
+// One FP64 pair costs 51 operations with complex charges and the field, which bound the
+// kernel; two sources a step keep the FP64 pipe fed (their chains are independent).
+// FAST: the Helmholtz kernel in pair64's branch-free form.
+template <int NF, int R, bool FIELD, bool FAST>
 __global__ void __launch_bounds__(DT) k_direct_partial(const double* __restrict__ pos,
                                                        const double* __restrict__ q_re,
                                                        const double* __restrict__ q_im, int64_t n,
                                                        const int32_t* __restrict__ tg, int64_t n_t,
-                                                       double k, int field, int n_split,
-                                                       double* scratch, int* err, int yukawa) {
-    __shared__ double sx[DSTAGE], sy[DSTAGE], sz[DSTAGE], sqr[DSTAGE], sqi[DSTAGE];
+                                                       double k, unsigned lo_hi, unsigned range, int n_split,
+                                                       double* scratch, int* err) {
+    constexpr int NC = PairSums<NF, R, FIELD>::NC, NA = PairSums<NF, R, FIELD>::N;
+    __shared__ double sx[DSTAGE], sy[DSTAGE], sz[DSTAGE], sq[R][DSTAGE];
     const int64_t ti = blockIdx.x * (int64_t)DT + threadIdx.x;
     const int split = blockIdx.y;
     const int64_t chunk = (n + n_split - 1) / n_split;
@@ -82,7 +50,9 @@ __global__ void __launch_bounds__(DT) k_direct_partial(const double* __restrict_
             z = pos[3 * t + 2];
         }
     }
-    double acc[NV] = {0, 0, 0, 0, 0, 0, 0, 0};
+    double acc[NA];
+#pragma unroll
+    for (int v = 0; v < NA; ++v) acc[v] = 0.0;
     for (int64_t p0 = lo; p0 < hi; p0 += DSTAGE) {
         __syncthreads();
         for (int i = threadIdx.x; i < DSTAGE; i += DT) {
@@ -91,49 +61,52 @@ __global__ void __launch_bounds__(DT) k_direct_partial(const double* __restrict_
                 sx[i] = pos[3 * s];
                 sy[i] = pos[3 * s + 1];
                 sz[i] = pos[3 * s + 2];
-                sqr[i] = q_re[s];
-                sqi[i] = q_im ? q_im[s] : 0.0;
+                sq[0][i] = q_re[s];
+                if (R == 2) sq[R - 1][i] = q_im[s];
             }
         }
         __syncthreads();
         if (!act) continue;
         const int np = (int)((hi - p0 < DSTAGE) ? hi - p0 : DSTAGE);
-        for (int i = 0; i < np; ++i) {
-            double dx = x - sx[i], dy = y - sy[i], dz = z - sz[i];
-            double r2 = dx * dx + dy * dy + dz * dz;
-            if (!(r2 > 0.0)) continue;
-            double ir = rsqrt(r2), r = r2 * ir;
-            double kr = k * r, sn, cs;
-            if (yukawa) {   // real kernel: w = G, field weight (1 + kr) G / r^2
-                cs = exp(-kr) * 0.07957747154594767;
-                sn = 0.0;
-            } else {
-                sincos_reduced(kr, &sn, &cs);
+        // The staged sources into sums of their own, so that a stage with a separation outside
+        // [1e-290, 1e290] or a phase over 1e5 (judged by r2's high word) is done over in the
+        // general form; a coincident source counts as one at zero charge.
+        double part[NA];
+        bool odd = false;
+        auto sources = [&](auto fast) {
+#pragma unroll
+            for (int v = 0; v < NA; ++v) part[v] = 0.0;
+#pragma unroll 2
+            for (int i = 0; i < np; ++i) {
+                const double dx = x - sx[i], dy = y - sy[i], dz = z - sz[i];
+                const double r2 = dx * dx + dy * dy + dz * dz;
+                const bool far = r2 > 0.0;
+                double q[NF][R];
+#pragma unroll
+                for (int f = 0; f < NF; ++f)
+#pragma unroll
+                    for (int r = 0; r < R; ++r) q[f][r] = far ? sq[r][i] : 0.0;
+                const double r2s = far ? r2 : 1.0;
+                if (decltype(fast)::value) odd = odd || (unsigned)__double2hiint(r2s) - lo_hi >= range;
+                pair64<NF, R, FIELD, decltype(fast)::value>(NF == 1, k, dx, dy, dz, r2s, q, part);
             }
-            // w = e^{ikr}/r; q w
-            double wr = cs * ir, wi = sn * ir;
-            acc[0] += sqr[i] * wr - sqi[i] * wi;
-            acc[1] += sqr[i] * wi + sqi[i] * wr;
-            if (field) {
-                // e^{ikr}(1 - ikr)/r^3 = ((cs + kr sn) + i (sn - kr cs)) / r^3
-                double ir3 = ir * ir * ir;
-                double fr = (cs + kr * sn) * ir3, fi = (sn - kr * cs) * ir3;
-                if (yukawa) {
-                    fr = cs * (1.0 + kr) * ir3;
-                    fi = 0.0;
-                }
-                double gr = sqr[i] * fr - sqi[i] * fi, gi = sqr[i] * fi + sqi[i] * fr;
-                acc[2] += gr * dx;
-                acc[3] += gi * dx;
-                acc[4] += gr * dy;
-                acc[5] += gi * dy;
-                acc[6] += gr * dz;
-                acc[7] += gi * dz;
-            }
-        }
+        };
+        if (FAST) sources(std::true_type());
+        if (!FAST || odd) sources(std::false_type());
+#pragma unroll
+        for (int v = 0; v < NA; ++v) acc[v] += part[v];
     }
-    if (act)
-        for (int v = 0; v < NV; ++v) scratch[((int64_t)split * n_t + ti) * NV + v] = acc[v];
+    if (act) {   // re, im of the potential, then of the field's components
+        double* o = scratch + ((int64_t)split * n_t + ti) * NV;
+        o[0] = acc[0];
+        o[1] = NC == 2 ? acc[NC - 1] : 0.0;
+        if (FIELD)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                o[2 + 2 * a] = acc[NC + a];
+                o[3 + 2 * a] = NC == 2 ? acc[NC + 3 * (NC - 1) + a] : 0.0;
+            }
+    }
 }
 
 // The chunks' partial sums of one (target, value) pair added by one warp: lane j takes
@@ -171,8 +144,25 @@ void direct_sum(const double* pos, const double* q_re, const double* q_im, int64
                 double* scratch, int n_split, cudaStream_t s, int* err, int yukawa) {
     if (n_t == 0) return;
     dim3 grid((unsigned)ceil_div(n_t, DT), (unsigned)n_split);
-    HFMM_LAUNCH(k_direct_partial, grid, DT, 0, s, pos, q_re, q_im, n, targets, n_t, k,
-                fld ? 1 : 0, n_split, scratch, err, yukawa);
+    // r2 in [1e-290, min(1e290, (1e5 / k)^2)), by high words (rounded inwards)
+    auto high = [](double v) {
+        uint64_t u;
+        std::memcpy(&u, &v, sizeof(u));
+        return (unsigned)(u >> 32);
+    };
+    const double far = k == 0.0 ? 1e290 : std::min(1e290, 1e10 / (k * k));
+    const unsigned lo_hi = high(1e-290) + 1, hi_hi = far > 1e-289 ? high(far) : lo_hi;
+    auto launch = [&](auto kern) {
+        HFMM_LAUNCH(kern, grid, DT, 0, s, pos, q_re, q_im, n, targets, n_t, k, lo_hi, hi_hi - lo_hi, n_split,
+                    scratch, err);
+    };
+    if (yukawa) {   // one real kernel
+        if (q_im) fld ? launch(k_direct_partial<1, 2, true, false>) : launch(k_direct_partial<1, 2, false, false>);
+        else fld ? launch(k_direct_partial<1, 1, true, false>) : launch(k_direct_partial<1, 1, false, false>);
+    } else {
+        if (q_im) fld ? launch(k_direct_partial<2, 2, true, true>) : launch(k_direct_partial<2, 2, false, true>);
+        else fld ? launch(k_direct_partial<2, 1, true, true>) : launch(k_direct_partial<2, 1, false, true>);
+    }
     HFMM_LAUNCH(k_direct_reduce, (unsigned)ceil_div(n_t * NV * 32, 256), 256, 0, s, scratch, n_t, n_split,
                 fld ? 1 : 0, phi, fld);
 }

@@ -252,8 +252,8 @@ struct hfmm_plan {
     hfmm::DevBuf<double> rot_phase;  // e^{i m phi} per slot (complex)
     hfmm::DevBuf<int32_t> rot_dist;  // coaxial matrix per slot
     hfmm::DevBuf<double> rot_M;      // multipole work array of one level
-    hfmm::DevBuf<double> pot;        // per sorted particle: [fam][R] potentials
-    hfmm::DevBuf<double> fld;        // per sorted particle: [fam][R][3]
+    hfmm::DevBuf<double> pot;        // [re, im][sorted particle]
+    hfmm::DevBuf<double> fld;        // [re, im][x, y, z][sorted particle]
     hfmm::DevBuf<int> d_err;
     bool finalized = false;
 };

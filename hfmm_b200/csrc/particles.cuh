@@ -9,6 +9,8 @@ struct EvalView {
     int n_s, ld;
     double k;                  // Helmholtz wavenumber, or the screening constant kappa
     int yukawa;                // 0: Helmholtz (two families); 1: exp(-kappa r) / (4 pi r)
+    int fast;                  // Helmholtz with two families, every phase k r under 1e5 and the
+                               // domain's size in [1e-100, 1e100]: pair64's FAST form
     const double* pos_s;       // 3 x n, leaf-major sorted
     const float* pos_f;        // 6 x n: FP32 hi parts x|y|z, then lo parts (pos = hi + lo)
     const double* q_s;         // R x n, leaf-major sorted
@@ -35,46 +37,71 @@ struct ParticlePass {
     const double* dens = nullptr;    // equivalent densities [fam][box][R][ld]
     double* out = nullptr;           // check potentials [fam][box][R][ld]
     int64_t fam_stride = 0;
-    int level = -1;
-    double* pot = nullptr;           // [fam*R][n]
-    double* fld = nullptr;           // [fam*R*3][n]
+    int level = -1;                  // P2L: one level's targets, or all (-1)
+    int maxleaf = 1;                 // the widest leaf (L2P/M2P)
+    double* pot = nullptr;           // [re, im][n] (re alone: one family, real charges)
+    double* fld = nullptr;           // [re, im][x, y, z][n]
     double* phi = nullptr;           // COMBINE outputs (complex interleaved)
     double* E = nullptr;
 };
 
-// sin and cos of a phase |x| <= 1.5 by their Taylor series about 0 (Horner form in
-// x^2, through x^21 and x^22): the first omitted terms, x^23 / 23! and x^24 / 24!, stay
-// below 4.4e-19 and 2.8e-20 there, under FP64 rounding. Larger phases take sincos.
+// Coefficients in constant memory: an FP64 operation takes one operand from there, where a
+// literal costs two moves into registers at every use (117 instructions a P2M pair, 38 of
+// them FP64, with literals).
+static __constant__ double c_trig[] = {
+    0.6366197723675814, 6755399441055744.0,            // 2 / pi, 1.5 * 2^52
+    1.5707963267948966, 6.123233995736766e-17,         // pi / 2 in two parts
+    -1.591810123027412e-10, 2.5051131455427946e-08, -2.755731610068303e-06,   // P, degree 5 down
+    0.0001984126983675497, -0.008333333333330946, 0.16666666666666666,
+    1.1367978191553177e-11, -2.0875886390883725e-09, 2.755731556415141e-07,   // Q, degree 6 down
+    -2.480158729368715e-05, 0.0013888888888880767, -0.04166666666666664, 0.5};
+
+// sin and cos of a phase. Cody-Waite reduction against pi/2 in two parts, its FP64 value and
+// the remainder of pi: x - n hi is exact for |x| < 1e5 (n < 2^16), and n comes from adding
+// 1.5 * 2^52, whose low word holds the quadrant. On |r| <= pi/4, sin r = r - r^3 P(r^2) and
+// cos r = 1 - r^2 Q(r^2) with P and Q interpolated at the Chebyshev nodes of [0, (pi/4)^2]
+// (degrees 5 and 6, computed in 60 digits): 2.0e-17 and 6.1e-19 relative, under the rounding.
+// 19 FP64 operations for any phase met; larger ones (and NaN) take sincos. The Taylor series
+// through x^22 used before took 25 up to 1.5 and left larger phases to sincos.
+__device__ __forceinline__ void sincos_reduced64(double x, double* s, double* c) {   // |x| < 1e5
+    const double t = fma(x, c_trig[0], c_trig[1]);
+    const double n = t - c_trig[1];
+    const int quad = __double2loint(t);
+    double r = fma(-n, c_trig[2], x);
+    r = fma(-n, c_trig[3], r);
+    const double z = r * r;
+    double P = fma(z, c_trig[4], c_trig[5]);
+    double Q = fma(z, c_trig[10], c_trig[11]);
+    P = fma(P, z, c_trig[6]);
+    Q = fma(Q, z, c_trig[12]);
+    P = fma(P, z, c_trig[7]);
+    Q = fma(Q, z, c_trig[13]);
+    P = fma(P, z, c_trig[8]);
+    Q = fma(Q, z, c_trig[14]);
+    P = fma(P, z, c_trig[9]);
+    Q = fma(Q, z, c_trig[15]);
+    Q = fma(Q, z, c_trig[16]);
+    const double sr = fma(-(r * z), P, r);
+    const double cr = fma(-z, Q, 1.0);
+    const double a = quad & 1 ? cr : sr, b = quad & 1 ? sr : cr;
+    *s = __hiloint2double(__double2hiint(a) ^ (int)((unsigned)(quad & 2) << 30), __double2loint(a));
+    *c = __hiloint2double(__double2hiint(b) ^ (int)((unsigned)((quad + 1) & 2) << 30), __double2loint(b));
+}
+
 __device__ __forceinline__ void sincos_phase64(double x, double* s, double* c) {
-    if (fabs(x) <= 1.5) {
-        const double x2 = x * x;
-        // sin x / x = sum (-1)^i x^(2i) / (2i+1)!,  cos x = sum (-1)^i x^(2i) / (2i)!
-        double ps = -1.0 / 51090942171709440000.0;   // -1/21!
-        ps = fma(ps, x2, 1.0 / 121645100408832000.0);   // 1/19!
-        ps = fma(ps, x2, -1.0 / 355687428096000.0);     // -1/17!
-        ps = fma(ps, x2, 1.0 / 1307674368000.0);        // 1/15!
-        ps = fma(ps, x2, -1.0 / 6227020800.0);          // -1/13!
-        ps = fma(ps, x2, 1.0 / 39916800.0);             // 1/11!
-        ps = fma(ps, x2, -1.0 / 362880.0);              // -1/9!
-        ps = fma(ps, x2, 1.0 / 5040.0);                 // 1/7! (sign applied below)
-        ps = fma(ps, x2, -1.0 / 120.0);
-        ps = fma(ps, x2, 1.0 / 6.0);
-        double pc = 1.0 / 1124000727777607680000.0;     // 1/22!
-        pc = fma(pc, x2, -1.0 / 2432902008176640000.0); // -1/20!
-        pc = fma(pc, x2, 1.0 / 6402373705728000.0);     // 1/18!
-        pc = fma(pc, x2, -1.0 / 20922789888000.0);      // -1/16!
-        pc = fma(pc, x2, 1.0 / 87178291200.0);          // 1/14!
-        pc = fma(pc, x2, -1.0 / 479001600.0);           // -1/12!
-        pc = fma(pc, x2, 1.0 / 3628800.0);              // 1/10!
-        pc = fma(pc, x2, -1.0 / 40320.0);               // -1/8!
-        pc = fma(pc, x2, 1.0 / 720.0);                  // 1/6!
-        pc = fma(pc, x2, -1.0 / 24.0);                  // -1/4!
-        pc = fma(pc, x2, 0.5);                          // 1/2!
-        *s = fma(-x * x2, ps, x);                       // x - x^3 (1/3! - x^2/5! + ...)
-        *c = fma(-x2, pc, 1.0);                         // 1 - x^2 (1/2! - x^2/4! + ...)
-    } else {
-        sincos(x, s, c);
-    }
+    if ((__double2hiint(x) & 0x7fffffff) >= 0x40f86a00) sincos(x, s, c);   // 1e5
+    else sincos_reduced64(x, s, c);
+}
+
+// 1 / sqrt(x) for x in [1e-290, 1e290]: the hardware's approximation, then one step of
+// Householder's third-order iteration, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2 (an error
+// d of the seed leaves 2.5 d^3). Five FP64 operations and no branch, so that a loop can run
+// two pairs' chains side by side.
+__device__ __forceinline__ double rsqrt_normal(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 
 // The kernel seam of the particle kernels. Helmholtz: (sn, cs) = sin, cos of the phase
@@ -92,6 +119,78 @@ __device__ __forceinline__ void kernel_pair64(int yukawa, double kr, double* sn,
         *cs = e;
     } else {
         sincos_phase64(kr, sn, cs);
+    }
+}
+
+// Sums at a particle. The result of complex charges is phi = E_cos(q_re) - E_sin(q_im) +
+// i (E_sin(q_re) + E_cos(q_im)), so a particle needs its real and imaginary part only (the
+// real one alone with one family and real charges), not one sum per family and column:
+// 10 operations a pair for the field instead of 16, and half the sums to store.
+template <int NF, int R, bool FIELD>
+struct PairSums {
+    static constexpr int NC = NF == 1 && R == 1 ? 1 : 2;
+    static constexpr int N = NC * (FIELD ? 4 : 1);   // potential, then the field's x, y, z
+};
+
+// a[0] + i a[1] += the families' weights w on the columns of family f, column r: d[f][r]
+template <int NF, int R, typename T>
+__device__ __forceinline__ void pair_columns(const T (&w)[2], const T (&d)[NF][R], T (&g)[2]) {
+    g[0] = d[0][0] * w[0];
+    if (NF == 2 && R == 2) g[0] -= d[NF - 1][R - 1] * w[1];
+    g[1] = T(0);
+    if (NF == 2) g[1] = d[NF - 1][0] * w[1];
+    if (R == 2) g[1] += d[0][R - 1] * w[0];
+}
+
+// Lanes per target of a near-field warp on a leaf of cnt particles (a power of two): the
+// count that costs the fewest source steps, ceil(cnt / (32 / G)) passes of 32 / G steps per
+// 32 sources and one step's worth of staging each. 30 particles: 1 lane (one pass, 94 % of
+// the lanes busy); 33: 4 lanes (five passes of eight targets, 82 %, where two passes of 32
+// would leave half the lanes idle); 4: 8 lanes.
+__device__ __forceinline__ int p2p_lanes(int cnt) {
+    int best = 1, cost = 1 << 30;
+#pragma unroll
+    for (int G = 1; G <= 32; G *= 2) {
+        const int TG = 32 / G, c = ((cnt + TG - 1) / TG) * (TG + 1);
+        if (c < cost) {
+            cost = c;
+            best = G;
+        }
+    }
+    return best;
+}
+
+// One FP64 pair at separation (dx, dy, dz), r2 > 0, into the sums. FAST: a Helmholtz phase
+// under 1e5 and r2 in [1e-290, 1e290], without a branch; else any kernel and any values.
+template <int NF, int R, bool FIELD, bool FAST>
+__device__ __forceinline__ void pair64(int yukawa, double k, double dx, double dy, double dz, double r2,
+                                       const double (&d)[NF][R],
+                                       double (&acc)[PairSums<NF, R, FIELD>::N]) {
+    constexpr int NC = PairSums<NF, R, FIELD>::NC;
+    const double ir = FAST ? rsqrt_normal(r2) : rsqrt(r2), kr = k * (r2 * ir);
+    double sn, cs;
+    if (FAST) sincos_reduced64(kr, &sn, &cs);
+    else kernel_pair64(yukawa, kr, &sn, &cs);
+    const double w[2] = {cs * ir, sn * ir};
+    if (NF == 2 && R == 2) {
+        acc[0] = fma(d[0][0], w[0], fma(-d[NF - 1][R - 1], w[1], acc[0]));
+        acc[NC - 1] = fma(d[NF - 1][0], w[1], fma(d[0][R - 1], w[0], acc[NC - 1]));
+    } else {
+        acc[0] = fma(d[0][0], w[0], acc[0]);
+        if (NF == 2) acc[NC - 1] = fma(d[NF - 1][0], w[1], acc[NC - 1]);
+        if (R == 2) acc[NC - 1] = fma(d[0][R - 1], w[0], acc[NC - 1]);
+    }
+    if (FIELD) {
+        const double ir2 = ir * ir;
+        const double wf[2] = {fma(kr, w[1], w[0]) * ir2, fma(-kr, w[0], w[1]) * ir2};
+        double g[2];
+        pair_columns<NF, R, double>(wf, d, g);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            acc[NC + 3 * c + 0] = fma(g[c], dx, acc[NC + 3 * c + 0]);
+            acc[NC + 3 * c + 1] = fma(g[c], dy, acc[NC + 3 * c + 1]);
+            acc[NC + 3 * c + 2] = fma(g[c], dz, acc[NC + 3 * c + 2]);
+        }
     }
 }
 

@@ -1,0 +1,37 @@
+"""The FP64 pair arithmetic of the particle kernels and the referee (own reciprocal square
+root, phase reduction and sine / cosine series) against extended precision: one unit source,
+targets at separations over twelve decades, wavenumbers that take the phase from 0 across the
+switch to the general form at 1e5. Tolerance: 1 / r and the weights carry a few roundings
+(8 eps), and rounding k r moves the phase by eps k r (2 eps k r)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+EPS = np.finfo(np.float64).eps
+
+
+@pytest.mark.parametrize("k", [0.0, 1e-3, 2.5, -7.0, 311.0, 9.0e4, 3.0e6])
+def test_single_source(k):
+    import torch
+    import hfmm_b200
+    rng = np.random.default_rng(5)
+    n = 4096
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    pos = d * (10.0 ** rng.uniform(-11.0, 1.0, n))[:, None]
+    pos[0] = 0.0
+    q = np.zeros(n, complex)
+    q[0] = 1.0
+    st = hfmm_b200.setup(pos, 1.0, p=3, N_max=64, max_depth=2)
+    st.k = k   # the referee takes its wavenumber from the state: only it runs here
+    phi, E = hfmm_b200.direct(st, q, np.arange(1, n), field=True)
+    x = pos[1:].astype(np.longdouble)
+    r = np.sqrt((x ** 2).sum(1))
+    kr = np.longdouble(k) * r
+    w = (np.cos(kr) + 1j * np.sin(kr)) / r
+    f = w * (1 - 1j * kr) / r ** 2
+    tol = 8 * EPS + 2 * EPS * np.abs(kr)
+    assert (np.abs(phi - w) * r < tol).all()
+    err = np.abs(E - f[:, None] * x).max(1) * r ** 2 / (1 + np.abs(kr))
+    assert (err < 2 * tol).all()
+    st.close()
