@@ -131,55 +131,120 @@ __global__ void k_conv_nbr(const int32_t* __restrict__ child, const int32_t* __r
 }
 
 // ---------------------------------------------------------------- transforms
-// Sums over one axis folded by the pair (k, n - k): with v_j real or complex,
-//   C = sum_j v_j cos(2 pi j k / n), S = sum_j v_j sin(2 pi j k / n),
-//   X_k = C - i S, X_(n-k) = C + i S,
-// four FMAs per term and pair instead of eight. PK pairs per thread share each v_j load.
-constexpr int PK = 4;
+// One axis is a small real matrix times many columns, and runs on the FP64 tensor
+// instruction too. The pairs (k, n - k) share their sums: with v_j complex,
+//   forward, j < p values in:   C_k = sum_j v_j cos(2 pi j k / n), S_k = sum_j v_j sin(..),
+//                               X_k = C_k - i S_k, X_(n-k) = C_k + i S_k;
+//   inverse, j < p values out:  P_k = Y_k + Y_(n-k), M_k = Y_k - Y_(n-k),
+//                               u_j = Y_0 + sum_k P_k cos(2 pi j k / n) + i M_k sin(..).
+// k and j both run over p = (n + 1) / 2 values, so one table serves: T[u][s][lane] = cos and
+// sin of 2 pi (4 s + lane % 4) (8 u + lane / 4) / n, zero where the first factor is >= p.
+// (One thread per column with scalar sums before spent its issue slots on twiddle indexes:
+// FP64 pipe 17 and 12 % busy; forward 4.0 and inverse 6.0 ms at 1e6 points, p = 8.)
+struct AxisShape {
+    int p, n, CH, lch, SR, KS, MT;   // lch = log2 CH; SR: row length in smem (CH + 2: no bank
+                                     // conflicts); KS, MT: steps of 4 and tiles of 8 over p
+};
 
-__device__ __forceinline__ void axis_pairs(const double2* v, int stride, int p, int n, int k0,
-                                           const double2* tw, double2 (&C)[PK], double2 (&S)[PK]) {
-    int m[PK], kk[PK];
-#pragma unroll
-    for (int u = 0; u < PK; ++u) {
-        C[u] = S[u] = make_double2(0.0, 0.0);
-        m[u] = 0;
-        kk[u] = min(k0 + u, n - 1);
+__device__ __forceinline__ AxisShape axis_shape(const ConvCall& c) {
+    AxisShape a;
+    a.p = c.p;
+    a.n = c.n;
+    a.CH = c.CH;
+    a.lch = 31 - __clz(c.CH);
+    a.SR = c.CH + 2;
+    a.KS = (c.p + 3) / 4;
+    a.MT = (c.p + 7) / 8;
+    return a;
+}
+
+__device__ __forceinline__ void axis_table(const AxisShape& a, const double2* tw, double2* T) {
+    for (int i = threadIdx.x; i < a.MT * a.KS * 32; i += blockDim.x) {
+        const int lane = i & 31, s = (i >> 5) % a.KS, u = (i >> 5) / a.KS;
+        const int f = 4 * s + (lane & 3);
+        T[i] = f < a.p ? tw[f * (8 * u + (lane >> 2)) % a.n] : make_double2(0.0, 0.0);
     }
-    for (int j = 0; j < p; ++j) {
-        const double2 x = v[j * stride];
-#pragma unroll
-        for (int u = 0; u < PK; ++u) {
-            const double2 w = tw[m[u]];
-            C[u].x = fma(x.x, w.x, C[u].x);
-            C[u].y = fma(x.y, w.x, C[u].y);
-            S[u].x = fma(x.x, w.y, S[u].x);
-            S[u].y = fma(x.y, w.y, S[u].y);
-            m[u] += kk[u];
-            if (m[u] >= n) m[u] -= n;
+}
+
+// Forward axis over n_grp groups of p rows of CH columns (rows[(grp * p + j) * SR + ch]):
+// a 16 x 8 tile is (C and S of eight k) x (re and im of four columns), so a lane ends with
+// C_k and S_k of one column. store(grp, ch, k, X_k, X_(n-k)) for k < p.
+template <class Store>
+__device__ __forceinline__ void axis_forward(const AxisShape& a, const double2* rows, int n_grp, const double2* T,
+                                             Store store) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int ncol = n_grp * a.CH, ntile = (ncol + 3) / 4;
+    for (int it = warp; it < ntile * a.MT; it += nw) {
+        const int u = it / ntile, tile = it - u * ntile;
+        const int col = tile * 4 + (g >> 1);
+        const bool ok = col < ncol;
+        const double* b = reinterpret_cast<const double*>(rows + ((ok ? col >> a.lch : 0) * a.p) * a.SR +
+                                                          (col & (a.CH - 1))) + (g & 1);
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int s = 0; s < a.KS; ++s) {
+            const double2 w = T[(u * a.KS + s) * 32 + lane];
+            const int j = 4 * s + t4;
+            dmma(acc, w.x, w.y, ok && j < a.p ? b[j * a.SR * 2] : 0.0);
+        }
+        const int oc = tile * 4 + t4, k = 8 * u + g;
+        if (oc < ncol && k < a.p)
+            store(oc >> a.lch, oc & (a.CH - 1), k, make_double2(acc[0] + acc[3], acc[1] - acc[2]),
+                  make_double2(acc[0] - acc[3], acc[1] + acc[2]));
+    }
+}
+
+// Inverse axis over n_grp groups: load(grp, ch, k, P, M) gives P_k and M_k; a 16 x 8 tile is
+// (re and im of eight columns) x (eight j). store(grp, ch, j, u_j) for j < p.
+template <class Load, class Store>
+__device__ __forceinline__ void axis_inverse(const AxisShape& a, int n_grp, const double2* T, Load load,
+                                             Store store) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int ncol = n_grp * a.CH, ntile = (ncol + 7) / 8;
+    for (int it = warp; it < ntile * a.MT; it += nw) {
+        const int u = it / ntile, tile = it - u * ntile;
+        const int col = tile * 8 + g, grp = col >> a.lch, ch = col & (a.CH - 1);
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int s = 0; s < a.KS; ++s) {
+            const int k = 4 * s + t4;
+            double2 P = make_double2(0.0, 0.0), M = P;
+            if (col < ncol && k < a.p) load(grp, ch, k, P, M);
+            const double2 w = T[(u * a.KS + s) * 32 + lane];
+            dmma(acc, P.x, P.y, w.x);
+            dmma(acc, -M.y, M.x, w.y);
+        }
+        const int j = 8 * u + 2 * t4;
+        if (col < ncol) {
+            if (j < a.p) store(grp, ch, j, make_double2(acc[0], acc[2]));
+            if (j + 1 < a.p) store(grp, ch, j + 1, make_double2(acc[1], acc[3]));
         }
     }
 }
 
 // Forward transform of a slot's children (c.CH of them per CTA): the frequencies of rows
 // kz in [kz0, kz1) x ky in [ky0, ky1), all kx. Per kz: z sums of the surface lines (interior
-// lines hold two points), then y, then x; the x stage writes 16 bytes x 8 children a
-// frequency. Bound by its stores (16 n^3 bytes a box) once the folded sums are this cheap.
+// lines hold two points), then the y and x axes; the x axis stores 16 bytes x 4 children a
+// frequency. 16 n^3 bytes a box leave the CTA: bound by those stores at large sizes.
 template <int R>
 __global__ void __launch_bounds__(256) k_conv_fwd(ConvCall c) {
     extern __shared__ double2 sh[];
-    const int p = c.p, n = c.n, nh = (n + 1) / 2, CH = c.CH, nky = c.ky1 - c.ky0;
-    const int slot = blockIdx.x, c0 = blockIdx.y * CH, fam = blockIdx.z;
-    double2* tw = sh;                       // n
-    double2* A1 = tw + n;                   // [p * p][CH]
-    double2* A2 = A1 + p * p * CH;          // [p][nky][CH]
-    double* xs = reinterpret_cast<double*>(A2 + p * nky * CH);   // [n_s][CH][R]
+    const AxisShape a = axis_shape(c);
+    const int p = c.p, n = c.n, nh = p, CH = c.CH, nky = c.ky1 - c.ky0;
+    const int slot = blockIdx.x, c0 = blockIdx.y * CH, fam = blockIdx.z / c.n_seg, seg = blockIdx.z % c.n_seg;
+    const int nz = c.kz1 - c.kz0, kz0 = c.kz0 + seg * nz / c.n_seg, kz1 = c.kz0 + (seg + 1) * nz / c.n_seg;
+    double2* tw = sh;                          // n
+    double2* tz = tw + n;                      // p: e^{2 pi i k kz / n}
+    double2* T = tz + p;
+    double2* A1 = T + a.MT * a.KS * 32;        // [i][j][SR]
+    double2* A2 = A1 + p * p * a.SR;           // [ky][i][SR]
+    double* xs = reinterpret_cast<double*>(A2 + p * nky * a.SR);   // [point][CH][R]
     const int nkx = R == 2 ? n : nh;
     const int64_t fstride = (int64_t)(c.n_slots + 1) * 8;   // values of one frequency
     double2* X = c.X + (int64_t)fam * c.rows * nkx * fstride + (int64_t)slot * 8 + c0;
     const int tid = threadIdx.x, nt = blockDim.x;
     if (slot == c.n_slots) {   // the zero slot
-        for (int64_t i = tid; i < (int64_t)c.rows * nkx * CH; i += nt)
+        for (int64_t i = tid; seg == 0 && i < (int64_t)c.rows * nkx * CH; i += nt)
             X[(i / CH) * fstride + i % CH] = make_double2(0.0, 0.0);
         return;
     }
@@ -187,65 +252,46 @@ __global__ void __launch_bounds__(256) k_conv_fwd(ConvCall c) {
     for (int ch = 0; ch < CH; ++ch) {
         const int b = c.child[slot * 8 + c0 + ch];
         const double* src = c.dens + (int64_t)fam * c.fam_stride + (int64_t)b * R * c.ld;
-        for (int i = tid; i < R * c.n_s; i += nt) {
-            const int r = i / c.n_s, s = i - r * c.n_s;
-            xs[(c.pos[s] * CH + ch) * R + r] = b >= 0 ? src[r * c.ld + s] : 0.0;
-        }
+        for (int r = 0; r < R; ++r)
+            for (int s = tid; s < c.n_s; s += nt) xs[(c.pos[s] * CH + ch) * R + r] = b >= 0 ? src[r * c.ld + s] : 0.0;
     }
-    const int groups = (nh + PK - 1) / PK;
-    for (int kz = c.kz0; kz < c.kz1; ++kz) {
+    __syncthreads();
+    axis_table(a, tw, T);
+    for (int kz = kz0; kz < kz1; ++kz) {
+        if (tid < p) tz[tid] = tw[tid * kz % n];
         __syncthreads();
         for (int it = tid; it < p * p * CH; it += nt) {   // z: the lines' points
-            const int ch = it % CH, line = it / CH, i = line / p, j = line - i * p;
+            const int ch = it & (CH - 1), line = it >> a.lch, i = line / p, j = line - i * p;
             const bool edge = i == 0 || j == 0 || i == p - 1 || j == p - 1;
-            const int e0 = c.line_off[line], cnt = edge ? p : 2;
-            const int step = edge ? kz : (int)(((int64_t)(p - 1) * kz) % n);
+            const double* x = xs + (c.line_off[line] * CH + ch) * R;
+            const int cnt = edge ? p : 2, step = edge ? 1 : p - 1;
             double re = 0.0, im = 0.0;
-            int m = 0;
-            for (int q = 0; q < cnt; ++q) {
-                const double2 w = tw[m];
-                const double* x = xs + ((e0 + q) * CH + ch) * R;
-                re = fma(x[0], w.x, re);
-                im = fma(-x[0], w.y, im);
+            for (int q = 0; q < cnt; ++q, x += CH * R) {
+                const double2 w = tz[q * step];
                 if (R == 2) {
-                    re = fma(x[1], w.y, re);
-                    im = fma(x[1], w.x, im);
+                    const double2 v = *reinterpret_cast<const double2*>(x);
+                    re = fma(v.x, w.x, fma(v.y, w.y, re));
+                    im = fma(v.y, w.x, fma(-v.x, w.y, im));
+                } else {
+                    re = fma(x[0], w.x, re);
+                    im = fma(-x[0], w.y, im);
                 }
-                m += step;
-                if (m >= n) m -= n;
             }
-            A1[it] = make_double2(re, im);
+            A1[line * a.SR + ch] = make_double2(re, im);
         }
         __syncthreads();
-        for (int it = tid; it < p * CH * groups; it += nt) {   // y
-            const int ch = it % CH, i = (it / CH) % p, k0 = (it / (CH * p)) * PK;
-            double2 C[PK], S[PK];
-            axis_pairs(A1 + i * p * CH + ch, CH, p, n, k0, tw, C, S);
-#pragma unroll
-            for (int u = 0; u < PK; ++u) {
-                const int k = k0 + u, km = n - k;
-                if (k >= nh) break;
-                if (k >= c.ky0 && k < c.ky1)
-                    A2[(i * nky + k - c.ky0) * CH + ch] = make_double2(C[u].x + S[u].y, C[u].y - S[u].x);
-                if (k > 0 && km >= c.ky0 && km < c.ky1)
-                    A2[(i * nky + km - c.ky0) * CH + ch] = make_double2(C[u].x - S[u].y, C[u].y + S[u].x);
-            }
-        }
+        axis_forward(a, A1, p, T, [&](int i, int ch, int k, double2 Xk, double2 Xn) {   // y
+            if (k >= c.ky0 && k < c.ky1) A2[((k - c.ky0) * p + i) * a.SR + ch] = Xk;
+            const int m = n - k;
+            if (k > 0 && m >= c.ky0 && m < c.ky1) A2[((m - c.ky0) * p + i) * a.SR + ch] = Xn;
+        });
         __syncthreads();
-        const int64_t row0 = (int64_t)(kz - c.kz0) * nky;
-        for (int it = tid; it < nky * CH * groups; it += nt) {   // x, to memory
-            const int ch = it % CH, ky = (it / CH) % nky, k0 = (it / (CH * nky)) * PK;
-            double2 C[PK], S[PK];
-            axis_pairs(A2 + ky * CH + ch, nky * CH, p, n, k0, tw, C, S);
-            double2* o = X + (row0 + ky) * nkx * fstride + ch;
-#pragma unroll
-            for (int u = 0; u < PK; ++u) {
-                const int k = k0 + u;
-                if (k >= nh) break;
-                o[k * fstride] = make_double2(C[u].x + S[u].y, C[u].y - S[u].x);
-                if (R == 2 && k > 0) o[(n - k) * fstride] = make_double2(C[u].x - S[u].y, C[u].y + S[u].x);
-            }
-        }
+        double2* o = X + (int64_t)(kz - c.kz0) * nky * nkx * fstride;
+        axis_forward(a, A2, nky, T, [&](int ky, int ch, int k, double2 Xk, double2 Xn) {   // x, to memory
+            double2* q = o + (int64_t)ky * nkx * fstride + ch;
+            q[k * fstride] = Xk;
+            if (R == 2 && k > 0) q[(n - k) * fstride] = Xn;
+        });
     }
 }
 
@@ -341,20 +387,23 @@ __global__ void __launch_bounds__(32 * CONV_WARPS) k_conv_mul(ConvCall c, int nk
     }
 }
 
-// Inverse transform of a slot's children onto the surface points: per kz the x sums (folded
-// by (k, n - k)) straight from memory, the y sums, then every surface point's z term, added
-// into the points' sums in kz order. The sums start from 0 on the first chunk and from the
-// check potentials after, so whole-plane chunks of any number give the same bits. Bound by
-// the reads of Y. R = 1: the half spectrum, terms kx > 0 doubled, real part kept.
+// Inverse transform of a slot's children onto the surface points: per kz the x axis straight
+// from memory, the y axis, then every surface point's z term, added into the points' sums in
+// kz order. The sums start from 0 on the first chunk and from the check potentials after, so
+// whole-plane chunks of any number give the same bits. Bound by the reads of Y at large
+// sizes. R = 1: the half spectrum, terms kx > 0 doubled, real part kept.
 template <int R>
 __global__ void __launch_bounds__(256) k_conv_inv(ConvCall c) {
     extern __shared__ double2 sh[];
-    const int p = c.p, n = c.n, nh = (n + 1) / 2, CH = c.CH, nky = c.ky1 - c.ky0;
+    const AxisShape a = axis_shape(c);
+    const int p = c.p, n = c.n, nh = p, CH = c.CH, nky = c.ky1 - c.ky0;
     const int slot = blockIdx.x, c0 = blockIdx.y * CH, fam = blockIdx.z;
-    double2* tw = sh;                       // n
-    double2* U2 = tw + n;                   // [p][nky][CH]
-    double2* U1 = U2 + p * nky * CH;        // [p * p][CH]
-    double* acc = reinterpret_cast<double*>(U1 + p * p * CH);   // [n_s][CH][R]
+    double2* tw = sh;                          // n
+    double2* tz = tw + n;                      // p
+    double2* T = tz + p;
+    double2* U1 = T + a.MT * a.KS * 32;        // [i][j][SR]
+    double2* U2 = U1 + p * p * a.SR;           // [i][ky][SR]
+    double* acc = reinterpret_cast<double*>(U2 + p * nky * a.SR);   // [point][CH][R]
     const int nkx = R == 2 ? n : nh;
     const int64_t fstride = (int64_t)(c.n_slots + 1) * 8;
     const double2* Y = c.Y + (int64_t)fam * c.rows * nkx * fstride + (int64_t)slot * 8 + c0;
@@ -363,83 +412,67 @@ __global__ void __launch_bounds__(256) k_conv_inv(ConvCall c) {
     for (int ch = 0; ch < CH; ++ch) {
         const int b = c.child[slot * 8 + c0 + ch];
         const double* src = c.check + (int64_t)fam * c.fam_stride + (int64_t)b * R * c.ld;
-        for (int i = tid; i < R * c.n_s; i += nt) {
-            const int r = i / c.n_s, s = i - r * c.n_s;
-            acc[(c.pos[s] * CH + ch) * R + r] = c.first || b < 0 ? 0.0 : src[r * c.ld + s];
-        }
+        for (int r = 0; r < R; ++r)
+            for (int s = tid; s < c.n_s; s += nt)
+                acc[(c.pos[s] * CH + ch) * R + r] = c.first || b < 0 ? 0.0 : src[r * c.ld + s];
     }
-    const int groups = (p + PK - 1) / PK;
+    __syncthreads();
+    axis_table(a, tw, T);
     for (int kz = c.kz0; kz < c.kz1; ++kz) {
-        __syncthreads();
-        const int64_t row0 = (int64_t)(kz - c.kz0) * nky;
-        for (int it = tid; it < nky * CH * groups; it += nt) {   // x, from memory
-            const int ch = it % CH, ky = (it / CH) % nky, i0 = (it / (CH * nky)) * PK;
-            const double2* y = Y + (row0 + ky) * nkx * fstride + ch;
-            const double2 y0 = y[0];
-            double2 u[PK];
-            int m[PK], ii[PK];
-#pragma unroll
-            for (int a = 0; a < PK; ++a) {
-                u[a] = y0;
-                ii[a] = min(i0 + a, p - 1);
-                m[a] = ii[a];
+        __syncthreads();   // T is there; the previous plane's points have read tz and U1
+        if (tid < p) tz[tid] = tw[tid * kz % n];
+        const double2* y = Y + (int64_t)(kz - c.kz0) * nky * nkx * fstride;
+        axis_inverse(a, nky, T, [&](int ky, int ch, int k, double2& P, double2& M) {   // x, from memory
+            const double2* q = y + (int64_t)ky * nkx * fstride + ch;
+            const double2 v = __ldg(q + k * fstride);
+            if (k == 0) {
+                P = v;
+            } else if (R == 2) {
+                const double2 m = __ldg(q + (n - k) * fstride);
+                P = make_double2(v.x + m.x, v.y + m.y);
+                M = make_double2(v.x - m.x, v.y - m.y);
+            } else {
+                P = M = make_double2(2.0 * v.x, 2.0 * v.y);
             }
-            for (int k = 1; k < nh; ++k) {
-                const double2 a0 = y[k * fstride];
-                double2 P, M;
-                if (R == 2) {
-                    const double2 a1 = y[(n - k) * fstride];
-                    P = make_double2(a0.x + a1.x, a0.y + a1.y);
-                    M = make_double2(a0.x - a1.x, a0.y - a1.y);
+        }, [&](int ky, int ch, int i, double2 u) { U2[(i * nky + ky) * a.SR + ch] = u; });
+        __syncthreads();
+        if (nky == n) {   // y
+            axis_inverse(a, p, T, [&](int i, int ch, int k, double2& P, double2& M) {
+                const double2* q = U2 + i * n * a.SR + ch;
+                const double2 v = q[k * a.SR];
+                if (k == 0) {
+                    P = v;
                 } else {
-                    P = M = make_double2(2.0 * a0.x, 2.0 * a0.y);
+                    const double2 m = q[(n - k) * a.SR];
+                    P = make_double2(v.x + m.x, v.y + m.y);
+                    M = make_double2(v.x - m.x, v.y - m.y);
                 }
-#pragma unroll
-                for (int a = 0; a < PK; ++a) {
-                    const double2 w = tw[m[a]];
-                    u[a].x = fma(P.x, w.x, fma(-M.y, w.y, u[a].x));
-                    u[a].y = fma(P.y, w.x, fma(M.x, w.y, u[a].y));
-                    m[a] += ii[a];
-                    if (m[a] >= n) m[a] -= n;
+            }, [&](int i, int ch, int j, double2 u) { U1[(i * p + j) * a.SR + ch] = u; });
+        } else {   // some rows of a plane (a workspace under one plane): their sums unfolded
+            for (int it = tid; it < p * p * CH; it += nt) {
+                const int ch = it & (CH - 1), line = it >> a.lch, i = line / p, j = line - i * p;
+                double re = 0.0, im = 0.0;
+                for (int ky = 0; ky < nky; ++ky) {
+                    const double2 v = U2[(i * nky + ky) * a.SR + ch], w = tw[(c.ky0 + ky) * j % n];
+                    re = fma(v.x, w.x, fma(-v.y, w.y, re));
+                    im = fma(v.y, w.x, fma(v.x, w.y, im));
                 }
+                U1[line * a.SR + ch] = make_double2(re, im);
             }
-#pragma unroll
-            for (int a = 0; a < PK; ++a)
-                if (i0 + a < p) U2[((i0 + a) * nky + ky) * CH + ch] = u[a];
-        }
-        __syncthreads();
-        for (int it = tid; it < p * CH * groups; it += nt) {   // y
-            const int ch = it % CH, i = (it / CH) % p, j0 = (it / (CH * p)) * PK;
-            double2 u[PK];
-            int m[PK], jj[PK];
-#pragma unroll
-            for (int a = 0; a < PK; ++a) {
-                u[a] = make_double2(0.0, 0.0);
-                jj[a] = min(j0 + a, p - 1);
-                m[a] = (int)(((int64_t)c.ky0 * jj[a]) % n);
-            }
-            for (int ky = 0; ky < nky; ++ky) {
-                const double2 y = U2[(i * nky + ky) * CH + ch];
-#pragma unroll
-                for (int a = 0; a < PK; ++a) {
-                    const double2 w = tw[m[a]];
-                    u[a].x = fma(y.x, w.x, fma(-y.y, w.y, u[a].x));
-                    u[a].y = fma(y.y, w.x, fma(y.x, w.y, u[a].y));
-                    m[a] += jj[a];
-                    if (m[a] >= n) m[a] -= n;
-                }
-            }
-#pragma unroll
-            for (int a = 0; a < PK; ++a)
-                if (j0 + a < p) U1[(i * p + j0 + a) * CH + ch] = u[a];
         }
         __syncthreads();
         for (int it = tid; it < c.n_s * CH; it += nt) {   // z: each surface point's own term
-            const int ch = it % CH, e = it / CH, lk = c.line_k[e];
-            const double2 y = U1[(lk >> 8) * CH + ch], w = tw[((lk & 255) * kz) % n];
-            double* a = acc + it * R;
-            a[0] = fma(y.x, w.x, fma(-y.y, w.y, a[0]));
-            if (R == 2) a[1] = fma(y.y, w.x, fma(y.x, w.y, a[1]));
+            const int ch = it & (CH - 1), lk = c.line_k[it >> a.lch];
+            const double2 v = U1[(lk >> 8) * a.SR + ch], w = tz[lk & 255];
+            if (R == 2) {
+                double2* q = reinterpret_cast<double2*>(acc) + it;
+                double2 t = *q;
+                t.x = fma(v.x, w.x, fma(-v.y, w.y, t.x));
+                t.y = fma(v.y, w.x, fma(v.x, w.y, t.y));
+                *q = t;
+            } else {
+                acc[it] = fma(v.x, w.x, fma(-v.y, w.y, acc[it]));
+            }
         }
     }
     __syncthreads();
@@ -447,16 +480,15 @@ __global__ void __launch_bounds__(256) k_conv_inv(ConvCall c) {
         const int b = c.child[slot * 8 + c0 + ch];
         if (b < 0) continue;
         double* dst = c.check + (int64_t)fam * c.fam_stride + (int64_t)b * R * c.ld;
-        for (int i = tid; i < R * c.n_s; i += nt) {
-            const int r = i / c.n_s, s = i - r * c.n_s;
-            dst[r * c.ld + s] = acc[(c.pos[s] * CH + ch) * R + r];
-        }
+        for (int r = 0; r < R; ++r)
+            for (int s = tid; s < c.n_s; s += nt) dst[r * c.ld + s] = acc[(c.pos[s] * CH + ch) * R + r];
     }
 }
 
 // shared memory of the transform kernels for CH children and nky rows of a plane
 size_t transform_smem(int p, int n_s, int R, int CH, int nky) {
-    return ((size_t)(2 * p - 1) + (size_t)CH * (p * p + p * nky)) * sizeof(double2) +
+    const size_t table = (size_t)((p + 7) / 8) * ((p + 3) / 4) * 32;
+    return ((size_t)(3 * p - 1) + table + (size_t)(CH + 2) * (p * p + p * nky)) * sizeof(double2) +
            (size_t)n_s * CH * R * sizeof(double);
 }
 
@@ -651,14 +683,22 @@ void conv_m2l(hfmm_plan* P, int R, int64_t fam_stride, cudaStream_t s) {
     if (rows < 1) throw Error{HFMM_ERR_STATE, "convolution M2L: workspace too small"};
     const int dz = std::max(planes, 1);
     const int PT = 256;
-    int CH = 8;   // children per CTA of the transforms: all eight where they fit
+    // children per CTA of the transforms: as many as leave two CTAs an SM, four at least (half
+    // the 128-byte lines) while those fit at all
+    int CH = 8;
+    while (CH > 4 && transform_smem(c.p, c.n_s, R, CH, rows) > SMEM_MAX / 2) CH /= 2;
     while (CH > 1 && transform_smem(c.p, c.n_s, R, CH, rows) > SMEM_MAX) CH /= 2;
-    c.CH = CH;
-    const size_t smem = transform_smem(c.p, c.n_s, R, CH, rows);
+    // few slots: fewer children a CTA on the inverse (its kz sum stays in one CTA), segments of
+    // kz on the forward, towards three CTAs an SM (72 slots, p = 8: 81 and 98 us with one)
+    const int64_t want = 3 * sm_count();
+    int CHi = CH;
+    while (CHi > 1 && (int64_t)c.n_slots * (8 / CHi) * nf < want) CHi /= 2;
+    const int segs = (int)std::max<int64_t>(1, want / ((int64_t)(c.n_slots + 1) * (8 / CH) * nf));
+    const size_t smem = transform_smem(c.p, c.n_s, R, CH, rows), smem_i = transform_smem(c.p, c.n_s, R, CHi, rows);
     auto fwd = R == 2 ? k_conv_fwd<2> : k_conv_fwd<1>;
     auto inv = R == 2 ? k_conv_inv<2> : k_conv_inv<1>;
     HFMM_CUDA(cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    HFMM_CUDA(cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HFMM_CUDA(cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_i));
     for (int f = 0; f < P->n_fam; f += nf) {
         c.dens = P->equiv.p + f * fam_stride;
         c.check = P->check.p + f * fam_stride;
@@ -673,10 +713,14 @@ void conv_m2l(hfmm_plan* P, int R, int64_t fam_stride, cudaStream_t s) {
                 c.rows = (c.kz1 - c.kz0) * (c.ky1 - c.ky0);
                 c.X = reinterpret_cast<double2*>(ws);
                 c.Y = c.X + (int64_t)c.rows * chunk_values(P, nkx, nf);
-                HFMM_LAUNCH(fwd, dim3((unsigned)(c.n_slots + 1), (unsigned)(8 / CH), (unsigned)nf), PT, smem, s, c);
+                c.CH = CH;
+                c.n_seg = std::min(segs, c.kz1 - c.kz0);
+                HFMM_LAUNCH(fwd, dim3((unsigned)(c.n_slots + 1), (unsigned)(8 / CH), (unsigned)(nf * c.n_seg)), PT,
+                            smem, s, c);
                 HFMM_LAUNCH(k_conv_mul, dim3((unsigned)((int64_t)c.rows * nkx * c.n_groups), (unsigned)nf),
                             32 * CONV_WARPS, 0, s, c, nkx);
-                HFMM_LAUNCH(inv, dim3((unsigned)c.n_slots, (unsigned)(8 / CH), (unsigned)nf), PT, smem, s, c);
+                c.CH = CHi;
+                HFMM_LAUNCH(inv, dim3((unsigned)c.n_slots, (unsigned)(8 / CHi), (unsigned)nf), PT, smem_i, s, c);
                 c.first = 0;
             }
     }

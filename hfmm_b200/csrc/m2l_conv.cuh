@@ -8,6 +8,7 @@ struct ConvCall {
     int p, n, n_s, ld;                // order, transform length 2p - 1, surface points, row length
     int n_slots, n_groups, CH;        // slots (the zero slot follows), groups, children per CTA
     int kz0, kz1, ky0, ky1, rows;     // the chunk's frequencies; rows = its (kz, ky) pairs
+    int n_seg;                        // kz segments of the forward transform's CTAs
     int first;                        // the first chunk stores the check potentials, others add
     int n_fam;
     const int32_t *child, *nbr, *pos, *line_off, *line_k;
