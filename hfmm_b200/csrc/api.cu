@@ -522,34 +522,10 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
         c.part_cap = P->gemm_part.n;
         gemm_f64(c, P->d_err.p, s);
     };
-    // The decode scale vector differs per family: run the first decode step once per family.
+    // the two factors of a level's decode, each for both families in one launch
     auto decode = [&](int l, bool up, const double* in, double* out) {
         const hfmm_plan::Tiles& tiles = P->dec_tiles[l][R - 1];
-        for (int f = 0; f < NF; ++f) {
-            PhaseTimer pt(X, s, up ? 3 : 6);
-            GemmCall c{};
-            c.tile_tgt = tiles.tgt.p;
-            c.ntiles = tiles.ntiles;
-            c.src_tab = nullptr;
-            c.src_ld = 0;
-            c.n_entries = 1;
-            c.b_split = 1;
-            c.A = P->a_ptrs.p + X->ix.off[up ? K_UPU : K_DNU][l] + f;
-            c.B0 = in + f * fs;
-            c.B1 = nullptr;
-            c.out = P->tmp.p + f * fs;
-            c.scale = up ? P->tables[f][l].up_d.p : P->tables[f][l].dn_d.p;
-            c.accumulate = 0;
-            c.R = R;
-            c.ld = P->ld;
-            c.n_s = P->n_s;
-            c.k_valid = P->n_s;
-            c.fam_stride = 0;
-            c.a_fam_stride = 0;
-            c.n_fam = 1;
-            c.nb = P->nb;
-            gemm_f64(c, P->d_err.p, s);
-        }
+        gemm(up ? K_UPU : K_DNU, l, tiles, nullptr, 0, in, nullptr, P->tmp.p, up ? SCALE_UP : SCALE_DN);
         gemm(up ? K_UPV : K_DNV, l, tiles, nullptr, 0, P->tmp.p, nullptr, out);
     };
 

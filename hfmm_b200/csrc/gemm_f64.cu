@@ -17,7 +17,14 @@
 //
 // Tensor path: mma.sync.m16n8k4 f64 (DMMA). tcgen05 has no f64 kind, so this
 // is the FP64 tensor path on sm_100a. CTA tile 64 (m) x 64 (n = targets x R),
-// k-chunk 16, 4 warps of 32 x 32, two-stage cp.async pipeline.
+// k-chunk 16, 4 warps of 32 x 32, three-stage cp.async pipeline with one barrier a chunk.
+// An SM sub-partition takes 32 cycles per DMMA, so a chunk's 32 a warp are 1,024 cycles; what
+// kept it from them were the instructions around (640 a chunk and warp: copy addresses and
+// source lookups worked out anew every chunk, eight 8-byte fragment loads a step). Now the
+// copy addresses are pointers that advance, looked up once an entry, and fragments are
+// 16-byte loads: lane t of four takes k = 2t and 2t + 1 of eight as two steps' B values, and
+// accumulator rows g and g + 8 are matrix rows 2g and 2g + 1 (the order of k and m within a
+// tile is free), which the epilogue then stores as 16-byte pairs straight from registers.
 // Small grids (coarse levels: a few dozen output tiles, each walking all its entries)
 // are latency-bound, so there the entries are split into contiguous ranges, one CTA
 // per range and output tile; each writes its partial tile to a scratch array and
@@ -31,10 +38,11 @@ namespace hfmm {
 
 namespace {
 
-constexpr int TM = 64, TN = 64, KC = 16;
-constexpr int AP = TM + 8;   // As[k][AP]: conflict-free a-fragment loads (AP = 8 mod 16)
-constexpr int BP = KC + 4;   // Bs[n][BP]: conflict-free b-fragment loads (BP = 4 mod 16)
+constexpr int TM = 64, TN = 64, KC = 16, STAGES = 3;
+constexpr int AP = TM + 2;   // As[k][AP]: two k rows apart is 32 bytes mod 128
+constexpr int BP = KC + 8;   // Bs[n][BP]: one column apart is 64 bytes mod 128
 constexpr int MAX_ENTRIES = 352;
+constexpr int SRC_ENTRIES = 8;   // entry counts whose tile sources are kept in shared memory
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
     unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -54,23 +62,36 @@ __device__ __forceinline__ void dmma(double (&c)[4], double a0, double a1, doubl
 }
 
 struct __align__(16) Smem {
-    union {
-        struct {
-            double A[2][KC][AP];
-            double B[2][TN][BP];
-        } ld;
-        double C[TN][TM + 2];   // epilogue staging, column-major by target column
-    } u;
+    double A[STAGES][KC][AP];
+    double B[STAGES][TN][BP];
+    int src[TN][SRC_ENTRIES + 1];
     int tgt[TN];
     short act[MAX_ENTRIES];
     unsigned char used[MAX_ENTRIES];   // entry has a source for some target of the tile
     int n_act;
 };
 
+// scale, accumulation and store of one column's rows m, m + 1
+__device__ __forceinline__ void store_pair(const GemmCall& c, double* out, const double* sc, int64_t row, int m,
+                                           double v0, double v1) {
+    if (sc) {
+        v0 *= sc[m];
+        v1 *= sc[m + 1];
+    }
+    double2* o = reinterpret_cast<double2*>(out + row * c.ldm + m);
+    if (c.accumulate) {
+        const double2 old = *o;
+        v0 += old.x;
+        v1 += old.y;
+    }
+    *o = make_double2(v0, v1);
+}
+
 template <int R>
-__global__ void __launch_bounds__(128, 5) k_gemm_f64(GemmCall c, int* err) {
+__global__ void __launch_bounds__(128, 3) k_gemm_f64(GemmCall c, int* err) {
     constexpr int TT = TN / R;
-    __shared__ Smem sm;
+    extern __shared__ __align__(16) char smem_raw[];
+    Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int S = c.n_split > 1 ? c.n_split : 1;
     const int tile = blockIdx.x, m0 = blockIdx.y * TM, fam = blockIdx.z / S, split = blockIdx.z % S;
@@ -80,6 +101,7 @@ __global__ void __launch_bounds__(128, 5) k_gemm_f64(GemmCall c, int* err) {
     const double* B0 = c.B0 + (int64_t)fam * c.fam_stride;
     const double* B1 = c.B1 ? c.B1 + (int64_t)fam * c.fam_stride : nullptr;
     double* out = c.out + (int64_t)fam * c.fam_stride;
+    const bool keep = c.src_tab && c.n_entries <= SRC_ENTRIES;
 
     if (tid < TT) {
         int t = c.tile_tgt[(int64_t)tile * TT + tid];
@@ -109,8 +131,16 @@ __global__ void __launch_bounds__(128, 5) k_gemm_f64(GemmCall c, int* err) {
                 }
             }
 #pragma unroll
-            for (int u = 0; u < BATCH; ++u)
-                if (src[u] >= 0) sm.used[(i0 + u * 128) % c.n_entries] = 1;
+            for (int u = 0; u < BATCH; ++u) {
+                const int i = i0 + u * 128;
+                if (i >= pairs) break;
+                if (src[u] >= c.nb) {
+                    atomicOr(err, ERRF_BOUNDS);
+                    src[u] = -1;
+                }
+                if (src[u] >= 0) sm.used[i % c.n_entries] = 1;
+                if (keep) sm.src[i / c.n_entries][i % c.n_entries] = src[u];
+            }
         }
         __syncthreads();
     }
@@ -126,36 +156,45 @@ __global__ void __launch_bounds__(128, 5) k_gemm_f64(GemmCall c, int* err) {
         if (lane == 0) sm.n_act = base;
     }
     __syncthreads();
-    const int n_act = sm.n_act;
-    const int kch = c.k_valid > 0 ? (c.k_valid + KC - 1) / KC : c.ldk / KC;
-    const int nq = n_act * kch;
+    const int k_len = c.k_valid > 0 ? c.k_valid : c.ldk;   // rows of A^T that can be nonzero
+    const int kch = (k_len + KC - 1) / KC;
+    const int nq = sm.n_act * kch;
 
-    auto load = [&](int q, int buf) {
-        const int e = sm.act[q / kch];
-        const int k0 = (q % kch) * KC;
-        const double* Ae = A[e];
-        const double* Bsel = (e >= c.b_split && B1) ? B1 : B0;
+    // the next chunk to copy: its entry, its k, and this thread's source addresses there
+    int l_e = 0, l_k = 0;
+    const double* ap = nullptr;
+    const double* bp[4];
+    unsigned bok = 0;
+    const bool aok = m0 + (tid & 31) * 2 < c.ldm;
+    auto load = [&](int buf) {
+        if (l_k == 0) {   // a new entry
+            const int e = sm.act[l_e++];
+            ap = A[e] + (int64_t)(tid >> 5) * c.ldm + (aok ? m0 + (tid & 31) * 2 : 0);
+            const double* Bsel = (e >= c.b_split && B1) ? B1 : B0;
+            bok = 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {   // A: 16 rows x 64 doubles = 512 x 16 B
-            int ch = tid + 128 * i;
-            int row = ch >> 5, col = (ch & 31) * 2;
-            bool ok = (m0 + col) < c.ldm;
-            const double* g = ok ? Ae + (int64_t)(k0 + row) * c.ldm + m0 + col : Ae;
-            cp_async16(&sm.u.ld.A[buf][row][col], g, ok);
+            for (int i = 0; i < 4; ++i) {   // B: 64 columns x 16 doubles, 8 threads a column
+                const int col = (tid >> 3) + 16 * i, j = col / R, r = col % R;
+                const int t = sm.tgt[j];
+                int s = -1;
+                if (keep) s = sm.src[j][e];
+                else if (t >= 0) s = c.src_tab ? c.src_tab[(int64_t)t * c.src_ld + e] : t;
+                const bool ok = s >= 0 && s < c.nb;
+                if (ok) bok |= 1u << i;
+                bp[i] = ok ? Bsel + ((int64_t)s * R + r) * c.ldk + (tid & 7) * 2 : B0;
+            }
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {   // B: 64 columns x 16 doubles = 512 x 16 B
-            int ch = tid + 128 * i;
-            int col = ch >> 3, part = (ch & 7) * 2;
-            int j = col / R, r = col % R;
-            int t = sm.tgt[j];
-            int s = -1;
-            if (t >= 0) s = c.src_tab ? c.src_tab[(int64_t)t * c.src_ld + e] : t;
-            bool ok = s >= 0 && s < c.nb;
-            if (s >= c.nb) atomicOr(err, ERRF_BOUNDS);
-            const double* g = ok ? Bsel + ((int64_t)s * R + r) * c.ldk + k0 + part : B0;
-            cp_async16(&sm.u.ld.B[buf][col][part], g, ok);
-        }
+        for (int i = 0; i < 4; ++i)   // A: 16 rows x 64 doubles, a warp a row
+            cp_async16(&sm.A[buf][(tid >> 5) + 4 * i][(tid & 31) * 2], ap + (int64_t)(4 * i) * c.ldm, aok);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            cp_async16(&sm.B[buf][(tid >> 3) + 16 * i][(tid & 7) * 2], bp[i], bok >> i & 1);
+        ap += (int64_t)KC * c.ldm;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (bok >> i & 1) bp[i] += KC;
+        l_k = l_k + 1 == kch ? 0 : l_k + 1;
     };
 
     double acc[2][4][4];
@@ -168,74 +207,65 @@ __global__ void __launch_bounds__(128, 5) k_gemm_f64(GemmCall c, int* err) {
 
     const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
     const int g = lane >> 2, t4 = lane & 3;
-    if (nq > 0) {
-        load(0, 0);
+    // 16-row halves of the warp's tile with rows that can be nonzero
+    const int m_rows = min(2, max(0, ((c.ldm == c.ld ? c.n_s : c.ldm) - (m0 + wm) + 15) / 16));
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; ++i) {
+        if (i < nq) load(i);
         cp_async_commit();
     }
+    int buf = 0, kq = 0;
     for (int q = 0; q < nq; ++q) {
-        const int buf = q & 1;
-        if (q + 1 < nq) {
-            load(q + 1, buf ^ 1);
-            cp_async_commit();
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();   // chunk q is there, and every warp is done with chunk q - 1
+        if (q + STAGES - 1 < nq) load(buf == 0 ? STAGES - 1 : buf - 1);
+        cp_async_commit();
+        const int k8n = min(KC, k_len - kq * KC);   // the entry's last chunk may be partial
+        kq = kq + 1 == kch ? 0 : kq + 1;
+        if (m_rows > 0) {
+            const double* As = &sm.A[buf][2 * t4][wm + 2 * g];
+            const double* Bs = &sm.B[buf][wn + g][2 * t4];
 #pragma unroll
-        for (int kk = 0; kk < KC; kk += 4) {
-            double a[2][2], b[4];
+            for (int kk = 0; kk < KC; kk += 8) {
+                if (kk >= k8n) break;
+                double2 b[4];
 #pragma unroll
-            for (int mi = 0; mi < 2; ++mi) {
-                a[mi][0] = sm.u.ld.A[buf][kk + t4][wm + mi * 16 + g];
-                a[mi][1] = sm.u.ld.A[buf][kk + t4][wm + mi * 16 + g + 8];
+                for (int ni = 0; ni < 4; ++ni) b[ni] = *reinterpret_cast<const double2*>(Bs + ni * 8 * BP + kk);
+#pragma unroll
+                for (int mi = 0; mi < 2; ++mi) {
+                    if (mi >= m_rows) break;
+                    const double2 a0 = *reinterpret_cast<const double2*>(As + kk * AP + mi * 16);
+                    const double2 a1 = *reinterpret_cast<const double2*>(As + (kk + 1) * AP + mi * 16);
+#pragma unroll
+                    for (int ni = 0; ni < 4; ++ni) dmma(acc[mi][ni], a0.x, a0.y, b[ni].x);
+#pragma unroll
+                    for (int ni = 0; ni < 4; ++ni) dmma(acc[mi][ni], a1.x, a1.y, b[ni].y);
+                }
             }
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni) b[ni] = sm.u.ld.B[buf][wn + ni * 8 + g][kk + t4];
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni) dmma(acc[mi][ni], a[mi][0], a[mi][1], b[ni]);
         }
-        __syncthreads();
+        buf = buf + 1 == STAGES ? 0 : buf + 1;
     }
-    // epilogue: stage through shared memory, write columns coalesced along m
+    cp_async_wait<0>();
+    // epilogue from registers: rows m, m + 1 of columns n and n + 1, 128 bytes a column
+    double* part = S > 1 ? c.part + ((int64_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * TN * TM
+                         : nullptr;
+    const double* sc = (fam == 1 && c.scale_f1) ? c.scale_f1 : c.scale;
 #pragma unroll
     for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni) {
-            int m = wm + mi * 16 + g, n = wn + ni * 8 + 2 * t4;
-            sm.u.C[n][m] = acc[mi][ni][0];
-            sm.u.C[n + 1][m] = acc[mi][ni][1];
-            sm.u.C[n][m + 8] = acc[mi][ni][2];
-            sm.u.C[n + 1][m + 8] = acc[mi][ni][3];
-        }
-    __syncthreads();
-    if (S > 1) {   // a split: the partial tile goes to the scratch, k_gemm_reduce finishes it
-        double* dst = c.part + ((int64_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * TN * TM;
-        for (int idx = tid; idx < TN * TM; idx += 128) dst[idx] = sm.u.C[idx / TM][idx % TM];
-        return;
-    }
-    const double* sc = (fam == 1 && c.scale_f1) ? c.scale_f1 : c.scale;
-    for (int idx = tid; idx < TN * (TM / 2); idx += 128) {
-        int col = idx / (TM / 2), mm = (idx % (TM / 2)) * 2;
-        int j = col / R, r = col % R;
-        int t = sm.tgt[j];
-        int m = m0 + mm;
-        if (t < 0 || m >= c.ldm) continue;
-        double v0 = sm.u.C[col][mm], v1 = sm.u.C[col][mm + 1];
-        if (sc) {
-            v0 *= sc[m];
-            v1 *= sc[m + 1];
-        }
-        double2* o = reinterpret_cast<double2*>(out + ((int64_t)t * R + r) * c.ldm + m);
-        if (c.accumulate) {
-            double2 old = *o;
-            v0 += old.x;
-            v1 += old.y;
-        }
-        *o = make_double2(v0, v1);
-    }
+        for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int ml = wm + mi * 16 + 2 * g, col = wn + ni * 8 + 2 * t4 + h, m = m0 + ml;
+                const double v0 = acc[mi][ni][h], v1 = acc[mi][ni][2 + h];
+                if (S > 1) {   // a split: the partial tile goes to the scratch, k_gemm_reduce finishes it
+                    *reinterpret_cast<double2*>(part + col * TM + ml) = make_double2(v0, v1);
+                    continue;
+                }
+                const int t = sm.tgt[col / R];
+                if (t < 0 || m >= c.ldm) continue;
+                store_pair(c, out, sc, (int64_t)t * R + col % R, m, v0, v1);
+            }
 }
 
 // The split GEMM's epilogue: per output tile, the n_split partial tiles added in
@@ -270,17 +300,7 @@ __global__ void __launch_bounds__(128) k_gemm_reduce(GemmCall c, int* err) {
             v0 += src[col * TM + mm];
             v1 += src[col * TM + mm + 1];
         }
-        if (sc) {
-            v0 *= sc[m];
-            v1 *= sc[m + 1];
-        }
-        double2* o = reinterpret_cast<double2*>(out + ((int64_t)t * R + r) * c.ldm + m);
-        if (c.accumulate) {
-            double2 old = *o;
-            v0 += old.x;
-            v1 += old.y;
-        }
-        *o = make_double2(v0, v1);
+        store_pair(c, out, sc, (int64_t)t * R + r, m, v0, v1);
     }
 }
 
@@ -319,8 +339,9 @@ void gemm_f64(const GemmCall& call, int* d_err, cudaStream_t s) {
     }
     c.n_split = S;
     grid.z *= S;
-    if (c.R == 1) HFMM_LAUNCH(k_gemm_f64<1>, grid, 128, 0, s, c, d_err);
-    else HFMM_LAUNCH(k_gemm_f64<2>, grid, 128, 0, s, c, d_err);
+    auto kern = c.R == 1 ? k_gemm_f64<1> : k_gemm_f64<2>;
+    HFMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
+    HFMM_LAUNCH(kern, grid, 128, sizeof(Smem), s, c, d_err);
     if (S > 1) {
         grid.z /= S;
         if (c.R == 1) HFMM_LAUNCH(k_gemm_reduce<1>, grid, 128, 0, s, c, d_err);
