@@ -236,7 +236,7 @@ void upload_level(hfmm_plan* P, int fam, int l, const double* const* h) {
     const int n_s = P->n_s, ld = P->ld;
     T.m2l_hi.release();   // halves of the tables being replaced
     T.m2l_lo.release();
-    P->conv.tables = false;
+    P->conv.tables = P->folded = false;
     T.host_m2l = h[8] != nullptr;
     std::vector<int32_t> none;
     relayout(h[0], 1, none, n_s, ld, false, T.up_U);   // A = U^T  -> A^T = U
@@ -845,6 +845,7 @@ int hfmm_tree_build(const double* pos_dev, int64_t n, int32_t n_max, int32_t max
     if (n_max < 1) return fail(HFMM_ERR_ARG, "N_max must be a positive integer");
     if (n > (int64_t)INT32_MAX) return fail(HFMM_ERR_CAPACITY, "more than 2^31-1 points");
     hfmm_plan* P = new hfmm_plan();
+    dev_plan_count(1);
     API_BEGIN
     HFMM_CUDA(cudaGetDevice(&P->device));
     require_device_ptr(pos_dev, "positions");
@@ -860,10 +861,12 @@ int hfmm_tree_build(const double* pos_dev, int64_t n, int32_t n_max, int32_t max
     }
     catch (const hfmm::Error& e) {
         delete P;
+        dev_plan_count(-1);
         return fail(e.code, e.msg);
     }
     catch (...) {
         delete P;
+        dev_plan_count(-1);
         return fail(HFMM_ERR_STATE, "tree build failed");
     }
 }
@@ -880,6 +883,7 @@ int hfmm_tree_build_in_domain(const double* pos_dev, int64_t n, int32_t n_max, i
         return fail(HFMM_ERR_ARG, "the domain needs a finite corner and a positive extent");
     if (n > (int64_t)INT32_MAX) return fail(HFMM_ERR_CAPACITY, "more than 2^31-1 points");
     hfmm_plan* P = new hfmm_plan();
+    dev_plan_count(1);
     API_BEGIN
     HFMM_CUDA(cudaGetDevice(&P->device));
     require_device_ptr(pos_dev, "positions");
@@ -898,10 +902,12 @@ int hfmm_tree_build_in_domain(const double* pos_dev, int64_t n, int32_t n_max, i
     }
     catch (const hfmm::Error& e) {
         delete P;
+        dev_plan_count(-1);
         return fail(e.code, e.msg);
     }
     catch (...) {
         delete P;
+        dev_plan_count(-1);
         return fail(HFMM_ERR_STATE, "tree build failed");
     }
 }
@@ -1285,6 +1291,7 @@ void hfmm_plan_destroy(hfmm_plan* P) {
     if (P->nf_fork) cudaEventDestroy(P->nf_fork);
     if (P->nf_join) cudaEventDestroy(P->nf_join);
     delete P;
+    dev_plan_count(-1);
 }
 
 int hfmm_export_tree(const hfmm_plan* P, uint64_t* m_id, int32_t* p_id, int32_t* lvls,

@@ -159,12 +159,13 @@ void compressed_prepare(hfmm_plan* P) {
                 T.grid = G;
             }
         }
-    {
+    if (!P->folded) {   // a plan rebuilt for moved points keeps its tables
         DevBuf<double> tmp;
         tmp.alloc(8 * (size_t)P->ld * P->ld);
         for (int f = 0; f < P->n_fam; ++f)
             for (int l = 2; l <= P->md; ++l) fold_level(P, f, l, tmp);
         HFMM_CUDA(cudaDeviceSynchronize());   // tmp is freed on return
+        P->folded = true;
     }
     if (!P->cx_fork) {   // side streams and fork/join events of the concurrent M2L
         HFMM_CUDA(cudaEventCreateWithFlags(&P->cx_fork, cudaEventDisableTiming));
@@ -213,6 +214,7 @@ int hfmm_plan_set_m2l_compressed(hfmm_plan* P, int32_t family, int32_t level, in
         require_device_ptr(U_dev, "U");
         require_device_ptr(C_dev, "C");
         LevelTables& T = P->tables[family][level];
+        P->folded = false;
         const int ckld = std::max(32, (int)round_up(rank, 32));    // K: one 32-wide chunk at least
         const int cmld = std::max(128, (int)round_up(rank, 32));   // M: one 128-row MMA tile at least
         T.cr = rank;

@@ -49,25 +49,40 @@ enum : int {
 };
 
 // ---------------------------------------------------------------- device memory
+// Blocks of device memory for DevBuf (devmem.cu). Like cudaFree, giving a block back waits
+// for the device, so no kernel on any stream still uses it; while plans are alive, blocks
+// are then kept for the next allocation of their size (a bounded amount per process).
+void* dev_alloc(size_t bytes, size_t* cap, int* device);
+void dev_free(void* p, size_t cap, int device) noexcept;
+void dev_plan_count(int change);   // plans alive; the last one gives every kept block back
+
 template <typename T>
 struct DevBuf {
     T* p = nullptr;
     size_t n = 0;
+    size_t cap = 0;   // bytes of the block
+    int device = -1;
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
+    // contents are undefined, also where the block at hand is large enough and stays
     void alloc(size_t count) {
-        release();
         if (count == 0) count = 1;
-        HFMM_CUDA(cudaMalloc((void**)&p, count * sizeof(T)));
+        const size_t bytes = count * sizeof(T);
+        if (p && cap >= bytes && cap / 4 <= bytes) {
+            HFMM_CUDA(cudaDeviceSynchronize());   // earlier users of the block
+        } else {
+            release();
+            p = static_cast<T*>(dev_alloc(bytes, &cap, &device));
+        }
         n = count;
     }
     void zero(cudaStream_t s = 0) { HFMM_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s)); }
     void release() {
-        if (p) cudaFree(p);
+        if (p) dev_free(p, cap, device);
         p = nullptr;
-        n = 0;
+        n = cap = 0;
     }
 };
 
@@ -218,6 +233,7 @@ struct hfmm_plan {
     hfmm::DevBuf<float> e_hi, e_lo, l_hi, l_lo;   // split densities [fam][box][R][ld]
     void* mx_maps = nullptr;                // MixedMaps per level (host array)
     bool compressed = false;                // every level has a compressed M2L (mixed path)
+    bool folded = false;                    // its folded tables are those of the current tables
     void* cx_maps = nullptr;                // MixedMaps [2][MAX_LEVELS] of the C_d tables
     void* cxq[2] = {nullptr, nullptr};      // PlanQueue per charge-column count (finalize)
     bool queue_m2l = true;                  // run the low-rank M2L as the plan's queue
