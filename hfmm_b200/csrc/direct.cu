@@ -25,7 +25,7 @@ constexpr int NV = 8;          // phi re/im + field 3 x re/im
 // kernel; two sources a step keep the FP64 pipe fed (their chains are independent).
 // FAST: the Helmholtz kernel in pair64's branch-free form.
 template <int NF, int R, bool FIELD, bool FAST>
-__global__ void __launch_bounds__(DT) k_direct_partial(const double* __restrict__ pos,
+__global__ void __launch_bounds__(DT, 5) k_direct_partial(const double* __restrict__ pos,
                                                        const double* __restrict__ q_re,
                                                        const double* __restrict__ q_im, int64_t n,
                                                        const int32_t* __restrict__ tg, int64_t n_t,
@@ -134,7 +134,8 @@ __global__ void k_direct_reduce(const double* __restrict__ scratch, int64_t n_t,
 
 int direct_splits(int64_t n, int64_t n_t) {
     int64_t tblocks = ceil_div(std::max<int64_t>(n_t, 1), DT);
-    int64_t want = ceil_div(4 * 148, tblocks);                 // about 4 CTAs per SM
+    // five CTAs per SM are resident: at most so many in all, one wave
+    int64_t want = std::max<int64_t>(1, 5 * 148 / tblocks);
     int64_t by_work = ceil_div(std::max<int64_t>(n, 1), 2048);  // at least 2048 sources a split
     return (int)std::max<int64_t>(1, std::min<int64_t>(want, by_work));
 }

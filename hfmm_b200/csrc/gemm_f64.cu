@@ -269,38 +269,37 @@ __global__ void __launch_bounds__(128, 3) k_gemm_f64(GemmCall c, int* err) {
 }
 
 // The split GEMM's epilogue: per output tile, the n_split partial tiles added in
-// entry-range order, then the scale, accumulation and store of k_gemm_f64.
+// entry-range order, then the scale, accumulation and store of k_gemm_f64. RED_COLS columns
+// of a tile per CTA: a coarse level has 10 to 50 tiles, and a CTA a tile took 15 to 24 us.
+constexpr int RED_COLS = 8;
 template <int R>
 __global__ void __launch_bounds__(128) k_gemm_reduce(GemmCall c, int* err) {
-    constexpr int TT = TN / R;
-    __shared__ int tgt[TT];
+    constexpr int TT = TN / R, PARTS = TN / RED_COLS;
     const int tid = threadIdx.x;
-    const int tile = blockIdx.x, m0 = blockIdx.y * TM, fam = blockIdx.z, S = c.n_split;
+    const int tile = blockIdx.x, m0 = blockIdx.y * TM, fam = blockIdx.z / PARTS, S = c.n_split;
     double* out = c.out + (int64_t)fam * c.fam_stride;
-    if (tid < TT) {
-        int t = c.tile_tgt[(int64_t)tile * TT + tid];
+    const double* sc = (fam == 1 && c.scale_f1) ? c.scale_f1 : c.scale;
+    const int64_t tile_of = (int64_t)gridDim.y * gridDim.x * TN * TM;   // doubles between ranges
+    const double* part = c.part + (int64_t)fam * S * tile_of + ((int64_t)blockIdx.y * gridDim.x + tile) * TN * TM;
+#pragma unroll
+    for (int q = 0; q < RED_COLS * (TM / 2) / 128; ++q) {
+        const int idx = tid + q * 128;
+        const int col = blockIdx.z % PARTS * RED_COLS + idx / (TM / 2), mm = (idx % (TM / 2)) * 2;
+        const int t = c.tile_tgt[(int64_t)tile * TT + col / R], m = m0 + mm;
         if (t >= c.nb) {
             atomicOr(err, ERRF_BOUNDS);
-            t = -1;
+            continue;
         }
-        tgt[tid] = t;
-    }
-    __syncthreads();
-    const double* sc = (fam == 1 && c.scale_f1) ? c.scale_f1 : c.scale;
-    for (int idx = tid; idx < TN * (TM / 2); idx += 128) {
-        int col = idx / (TM / 2), mm = (idx % (TM / 2)) * 2;
-        int j = col / R, r = col % R;
-        int t = tgt[j];
-        int m = m0 + mm;
         if (t < 0 || m >= c.ldm) continue;
         double v0 = 0.0, v1 = 0.0;
+        const double* src = part + col * TM + mm;
+#pragma unroll 4
         for (int sp = 0; sp < S; ++sp) {
-            const double* src = c.part +
-                ((int64_t)((fam * S + sp) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * TN * TM;
-            v0 += src[col * TM + mm];
-            v1 += src[col * TM + mm + 1];
+            const double2 v = *reinterpret_cast<const double2*>(src + sp * tile_of);
+            v0 += v.x;
+            v1 += v.y;
         }
-        store_pair(c, out, sc, (int64_t)t * R + r, m, v0, v1);
+        store_pair(c, out, sc, (int64_t)t * R + col % R, m, v0, v1);
     }
 }
 
@@ -343,7 +342,7 @@ void gemm_f64(const GemmCall& call, int* d_err, cudaStream_t s) {
     HFMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
     HFMM_LAUNCH(kern, grid, 128, sizeof(Smem), s, c, d_err);
     if (S > 1) {
-        grid.z /= S;
+        grid.z = grid.z / S * (TN / RED_COLS);
         if (c.R == 1) HFMM_LAUNCH(k_gemm_reduce<1>, grid, 128, 0, s, c, d_err);
         else HFMM_LAUNCH(k_gemm_reduce<2>, grid, 128, 0, s, c, d_err);
     }

@@ -168,65 +168,80 @@ __device__ __forceinline__ void axis_table(const AxisShape& a, const double2* tw
 
 // Forward axis over n_grp groups of p rows of CH columns (rows[(grp * p + j) * SR + ch]):
 // a 16 x 8 tile is (C and S of eight k) x (re and im of four columns), so a lane ends with
-// C_k and S_k of one column. store(grp, ch, k, X_k, X_(n-k)) for k < p.
-template <class Store>
+// C_k and S_k of one column. store(grp, ch, k, X_k, X_(n-k)) for k < p. KS > 0: the steps
+// over p at compile time, their table values in registers for all tiles (0: any count).
+template <int KS, class Store>
 __device__ __forceinline__ void axis_forward(const AxisShape& a, const double2* rows, int n_grp, const double2* T,
                                              Store store) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int g = lane >> 2, t4 = lane & 3;
-    const int ncol = n_grp * a.CH, ntile = (ncol + 3) / 4;
-    for (int it = warp; it < ntile * a.MT; it += nw) {
-        const int u = it / ntile, tile = it - u * ntile;
-        const int col = tile * 4 + (g >> 1);
-        const bool ok = col < ncol;
-        const double* b = reinterpret_cast<const double*>(rows + ((ok ? col >> a.lch : 0) * a.p) * a.SR +
-                                                          (col & (a.CH - 1))) + (g & 1);
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int s = 0; s < a.KS; ++s) {
-            const double2 w = T[(u * a.KS + s) * 32 + lane];
-            const int j = 4 * s + t4;
-            dmma(acc, w.x, w.y, ok && j < a.p ? b[j * a.SR * 2] : 0.0);
+    const int g = lane >> 2, t4 = lane & 3, ks = KS ? KS : a.KS;
+    const int ncol = n_grp * a.CH, step = 8 * a.SR;   // doubles between rows j and j + 4
+    for (int u = 0; u < a.MT; ++u) {
+        const double2* Tu = T + u * ks * 32 + lane;
+        double2 w[KS ? KS : 1];
+#pragma unroll
+        for (int s = 0; s < KS; ++s) w[s] = Tu[s * 32];
+        const int k = 8 * u + g;
+        for (int tile = warp; tile * 4 < ncol; tile += nw) {
+            const int col = tile * 4 + (g >> 1), oc = tile * 4 + t4;
+            const bool ok = col < ncol;
+            const double* b = reinterpret_cast<const double*>(rows + ((ok ? col >> a.lch : 0) * a.p + t4) * a.SR +
+                                                              (col & (a.CH - 1))) + (g & 1);
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+            if (KS) {
+                double v[KS ? KS : 1];
+#pragma unroll
+                for (int s = 0; s < KS; ++s) v[s] = ok && 4 * s + t4 < a.p ? b[s * step] : 0.0;
+#pragma unroll
+                for (int s = 0; s < KS; ++s) dmma(acc, w[s].x, w[s].y, v[s]);
+            } else {
+                for (int s = 0; s < ks; ++s) {
+                    const double2 ws = Tu[s * 32];
+                    dmma(acc, ws.x, ws.y, ok && 4 * s + t4 < a.p ? b[s * step] : 0.0);
+                }
+            }
+            if (oc < ncol && k < a.p)
+                store(oc >> a.lch, oc & (a.CH - 1), k, make_double2(acc[0] + acc[3], acc[1] - acc[2]),
+                      make_double2(acc[0] - acc[3], acc[1] + acc[2]));
         }
-        const int oc = tile * 4 + t4, k = 8 * u + g;
-        if (oc < ncol && k < a.p)
-            store(oc >> a.lch, oc & (a.CH - 1), k, make_double2(acc[0] + acc[3], acc[1] - acc[2]),
-                  make_double2(acc[0] - acc[3], acc[1] + acc[2]));
     }
 }
 
 // Inverse axis over n_grp groups: load(grp, ch, k, P, M) gives P_k and M_k; a 16 x 8 tile is
-// (re and im of eight columns) x (eight j). store(grp, ch, j, u_j) for j < p.
+// (re and im of eight columns) x (eight j). store(grp, ch, j, u_j) for j < p. (Steps at
+// compile time, all loads ahead, took twice the registers and 35 % more time.)
 template <class Load, class Store>
 __device__ __forceinline__ void axis_inverse(const AxisShape& a, int n_grp, const double2* T, Load load,
                                              Store store) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int g = lane >> 2, t4 = lane & 3;
-    const int ncol = n_grp * a.CH, ntile = (ncol + 7) / 8;
-    for (int it = warp; it < ntile * a.MT; it += nw) {
-        const int u = it / ntile, tile = it - u * ntile;
-        const int col = tile * 8 + g, grp = col >> a.lch, ch = col & (a.CH - 1);
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int s = 0; s < a.KS; ++s) {
-            const int k = 4 * s + t4;
-            double2 P = make_double2(0.0, 0.0), M = P;
-            if (col < ncol && k < a.p) load(grp, ch, k, P, M);
-            const double2 w = T[(u * a.KS + s) * 32 + lane];
-            dmma(acc, P.x, P.y, w.x);
-            dmma(acc, -M.y, M.x, w.y);
+    const int ncol = n_grp * a.CH;
+    for (int u = 0; u < a.MT; ++u)
+        for (int tile = warp; tile * 8 < ncol; tile += nw) {
+            const int col = tile * 8 + g, grp = col >> a.lch, ch = col & (a.CH - 1);
+            const bool ok = col < ncol;
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int s = 0; s < a.KS; ++s) {
+                const int k = 4 * s + t4;
+                double2 P = make_double2(0.0, 0.0), M = P;
+                if (ok && k < a.p) load(grp, ch, k, P, M);
+                const double2 w = T[(u * a.KS + s) * 32 + lane];
+                dmma(acc, P.x, P.y, w.x);
+                dmma(acc, -M.y, M.x, w.y);
+            }
+            const int j = 8 * u + 2 * t4;
+            if (ok) {
+                if (j < a.p) store(grp, ch, j, make_double2(acc[0], acc[2]));
+                if (j + 1 < a.p) store(grp, ch, j + 1, make_double2(acc[1], acc[3]));
+            }
         }
-        const int j = 8 * u + 2 * t4;
-        if (col < ncol) {
-            if (j < a.p) store(grp, ch, j, make_double2(acc[0], acc[2]));
-            if (j + 1 < a.p) store(grp, ch, j + 1, make_double2(acc[1], acc[3]));
-        }
-    }
 }
 
 // Forward transform of a slot's children (c.CH of them per CTA): the frequencies of rows
 // kz in [kz0, kz1) x ky in [ky0, ky1), all kx. Per kz: z sums of the surface lines (interior
 // lines hold two points), then the y and x axes; the x axis stores 16 bytes x 4 children a
 // frequency. 16 n^3 bytes a box leave the CTA: bound by those stores at large sizes.
-template <int R>
+template <int R, int KS>
 __global__ void __launch_bounds__(256) k_conv_fwd(ConvCall c) {
     extern __shared__ double2 sh[];
     const AxisShape a = axis_shape(c);
@@ -257,37 +272,64 @@ __global__ void __launch_bounds__(256) k_conv_fwd(ConvCall c) {
     }
     __syncthreads();
     axis_table(a, tw, T);
+    // the z items of this thread, (line, child): first value, count and spacing of its points
+    // and its place in A1, worked out once for the first ZI of them
+    constexpr int ZI = 3;
+    int z_x[ZI], z_n[ZI], z_o[ZI];
+    auto item = [&](int it, int& x, int& cnt, int& o) {
+        const int ch = it & (CH - 1), line = it >> a.lch, i = line / p, j = line - i * p;
+        cnt = i == 0 || j == 0 || i == p - 1 || j == p - 1 ? p : 2;
+        x = (c.line_off[line] * CH + ch) * R;
+        o = line * a.SR + ch;
+    };
+#pragma unroll
+    for (int q = 0; q < ZI; ++q) {
+        z_n[q] = 0;
+        if (tid + q * nt < p * p * CH) item(tid + q * nt, z_x[q], z_n[q], z_o[q]);
+    }
+    auto line_sum = [&](int x0, int cnt, int o) {
+        const double* x = xs + x0;
+        const double2* w = tz;
+        const int step = cnt == p ? 1 : p - 1;
+        double re = 0.0, im = 0.0;
+        for (int q = 0; q < cnt; ++q, x += CH * R, w += step) {
+            if (R == 2) {
+                const double2 v = *reinterpret_cast<const double2*>(x);
+                re = fma(v.x, w->x, fma(v.y, w->y, re));
+                im = fma(v.y, w->x, fma(-v.x, w->y, im));
+            } else {
+                re = fma(x[0], w->x, re);
+                im = fma(-x[0], w->y, im);
+            }
+        }
+        A1[o] = make_double2(re, im);
+    };
+    const bool full = nky == n;
     for (int kz = kz0; kz < kz1; ++kz) {
         if (tid < p) tz[tid] = tw[tid * kz % n];
         __syncthreads();
-        for (int it = tid; it < p * p * CH; it += nt) {   // z: the lines' points
-            const int ch = it & (CH - 1), line = it >> a.lch, i = line / p, j = line - i * p;
-            const bool edge = i == 0 || j == 0 || i == p - 1 || j == p - 1;
-            const double* x = xs + (c.line_off[line] * CH + ch) * R;
-            const int cnt = edge ? p : 2, step = edge ? 1 : p - 1;
-            double re = 0.0, im = 0.0;
-            for (int q = 0; q < cnt; ++q, x += CH * R) {
-                const double2 w = tz[q * step];
-                if (R == 2) {
-                    const double2 v = *reinterpret_cast<const double2*>(x);
-                    re = fma(v.x, w.x, fma(v.y, w.y, re));
-                    im = fma(v.y, w.x, fma(-v.x, w.y, im));
-                } else {
-                    re = fma(x[0], w.x, re);
-                    im = fma(-x[0], w.y, im);
-                }
-            }
-            A1[line * a.SR + ch] = make_double2(re, im);
+#pragma unroll
+        for (int q = 0; q < ZI; ++q)
+            if (z_n[q]) line_sum(z_x[q], z_n[q], z_o[q]);
+        for (int it = tid + ZI * nt; it < p * p * CH; it += nt) {
+            int x, cnt, o;
+            item(it, x, cnt, o);
+            line_sum(x, cnt, o);
         }
         __syncthreads();
-        axis_forward(a, A1, p, T, [&](int i, int ch, int k, double2 Xk, double2 Xn) {   // y
-            if (k >= c.ky0 && k < c.ky1) A2[((k - c.ky0) * p + i) * a.SR + ch] = Xk;
+        axis_forward<KS>(a, A1, p, T, [&](int i, int ch, int k, double2 Xk, double2 Xn) {   // y
             const int m = n - k;
-            if (k > 0 && m >= c.ky0 && m < c.ky1) A2[((m - c.ky0) * p + i) * a.SR + ch] = Xn;
+            if (full) {
+                A2[(k * p + i) * a.SR + ch] = Xk;
+                if (k > 0) A2[(m * p + i) * a.SR + ch] = Xn;
+            } else {
+                if (k >= c.ky0 && k < c.ky1) A2[((k - c.ky0) * p + i) * a.SR + ch] = Xk;
+                if (k > 0 && m >= c.ky0 && m < c.ky1) A2[((m - c.ky0) * p + i) * a.SR + ch] = Xn;
+            }
         });
         __syncthreads();
         double2* o = X + (int64_t)(kz - c.kz0) * nky * nkx * fstride;
-        axis_forward(a, A2, nky, T, [&](int ky, int ch, int k, double2 Xk, double2 Xn) {   // x, to memory
+        axis_forward<KS>(a, A2, nky, T, [&](int ky, int ch, int k, double2 Xk, double2 Xn) {   // x, to memory
             double2* q = o + (int64_t)ky * nkx * fstride + ch;
             q[k * fstride] = Xk;
             if (R == 2 && k > 0) q[(n - k) * fstride] = Xn;
@@ -404,11 +446,13 @@ __global__ void __launch_bounds__(256) k_conv_inv(ConvCall c) {
     double2* U1 = T + a.MT * a.KS * 32;        // [i][j][SR]
     double2* U2 = U1 + p * p * a.SR;           // [i][ky][SR]
     double* acc = reinterpret_cast<double*>(U2 + p * nky * a.SR);   // [point][CH][R]
+    int* pts = reinterpret_cast<int*>(acc + c.n_s * CH * R);        // [point] U1 row and k
     const int nkx = R == 2 ? n : nh;
     const int64_t fstride = (int64_t)(c.n_slots + 1) * 8;
     const double2* Y = c.Y + (int64_t)fam * c.rows * nkx * fstride + (int64_t)slot * 8 + c0;
     const int tid = threadIdx.x, nt = blockDim.x;
     for (int i = tid; i < n; i += nt) tw[i] = c.tw[i];
+    for (int i = tid; i < c.n_s; i += nt) pts[i] = c.line_k[i];
     for (int ch = 0; ch < CH; ++ch) {
         const int b = c.child[slot * 8 + c0 + ch];
         const double* src = c.check + (int64_t)fam * c.fam_stride + (int64_t)b * R * c.ld;
@@ -462,7 +506,7 @@ __global__ void __launch_bounds__(256) k_conv_inv(ConvCall c) {
         }
         __syncthreads();
         for (int it = tid; it < c.n_s * CH; it += nt) {   // z: each surface point's own term
-            const int ch = it & (CH - 1), lk = c.line_k[it >> a.lch];
+            const int ch = it & (CH - 1), lk = pts[it >> a.lch];
             const double2 v = U1[(lk >> 8) * a.SR + ch], w = tz[lk & 255];
             if (R == 2) {
                 double2* q = reinterpret_cast<double2*>(acc) + it;
@@ -489,7 +533,7 @@ __global__ void __launch_bounds__(256) k_conv_inv(ConvCall c) {
 size_t transform_smem(int p, int n_s, int R, int CH, int nky) {
     const size_t table = (size_t)((p + 7) / 8) * ((p + 3) / 4) * 32;
     return ((size_t)(3 * p - 1) + table + (size_t)(CH + 2) * (p * p + p * nky)) * sizeof(double2) +
-           (size_t)n_s * CH * R * sizeof(double);
+           (size_t)n_s * CH * R * sizeof(double) + (size_t)n_s * sizeof(int);
 }
 
 constexpr size_t SMEM_MAX = 227 * 1024;
@@ -695,8 +739,15 @@ void conv_m2l(hfmm_plan* P, int R, int64_t fam_stride, cudaStream_t s) {
     while (CHi > 1 && (int64_t)c.n_slots * (8 / CHi) * nf < want) CHi /= 2;
     const int segs = (int)std::max<int64_t>(1, want / ((int64_t)(c.n_slots + 1) * (8 / CH) * nf));
     const size_t smem = transform_smem(c.p, c.n_s, R, CH, rows), smem_i = transform_smem(c.p, c.n_s, R, CHi, rows);
-    auto fwd = R == 2 ? k_conv_fwd<2> : k_conv_fwd<1>;
-    auto inv = R == 2 ? k_conv_inv<2> : k_conv_inv<1>;
+    using Kernel = void (*)(ConvCall);
+    Kernel fwd = nullptr;
+    switch ((c.p + 3) / 4) {
+        case 1: fwd = R == 2 ? k_conv_fwd<2, 1> : k_conv_fwd<1, 1>; break;
+        case 2: fwd = R == 2 ? k_conv_fwd<2, 2> : k_conv_fwd<1, 2>; break;
+        case 3: fwd = R == 2 ? k_conv_fwd<2, 3> : k_conv_fwd<1, 3>; break;
+        default: fwd = R == 2 ? k_conv_fwd<2, 0> : k_conv_fwd<1, 0>; break;
+    }
+    const Kernel inv = R == 2 ? k_conv_inv<2> : k_conv_inv<1>;
     HFMM_CUDA(cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     HFMM_CUDA(cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_i));
     for (int f = 0; f < P->n_fam; f += nf) {
