@@ -234,8 +234,7 @@ void drop_extra(hfmm_plan* P) {
 void upload_level(hfmm_plan* P, int fam, int l, const double* const* h) {
     LevelTables& T = P->tables[fam][l];
     const int n_s = P->n_s, ld = P->ld;
-    T.m2l_hi.release();   // halves of the tables being replaced
-    T.m2l_lo.release();
+    T.m2l_s.release();   // planes of the tables being replaced
     P->conv.tables = P->folded = false;
     T.host_m2l = h[8] != nullptr;
     std::vector<int32_t> none;
@@ -260,24 +259,21 @@ void upload_level(hfmm_plan* P, int fam, int l, const double* const* h) {
     T.set = true;
 }
 
-// Tensor maps of the streamed TF32 tables: every level reads the same workspace
-// (hi halves of both families, then the lo halves; [fam][316][m][k] each).
+// Tensor maps of the streamed tables' planes: every level reads the same workspace,
+// [plane][fam][316][m][k].
 void stream_maps(hfmm_plan* P) {
     if (!P->mx_maps) P->mx_maps = new MixedMaps[MAX_LEVELS];
     MixedMaps* maps = static_cast<MixedMaps*>(P->mx_maps);
     std::memset(maps, 0, sizeof(MixedMaps) * MAX_LEVELS);
     const size_t fam = (size_t)316 * P->ld * P->ld;
-    const float* hi = static_cast<const float*>(P->ws);
-    const float* lo = hi + (size_t)P->n_fam * fam;
+    const uint16_t* ws = static_cast<const uint16_t*>(P->ws);
     for (int l = 2; l <= P->md; ++l)
-        for (int f = 0; f < P->n_fam; ++f) {
-            make_table_map(&maps[l].a_hi[f], hi + f * fam, P->ld, 316);
-            make_table_map(&maps[l].a_lo[f], lo + f * fam, P->ld, 316);
-        }
+        for (int f = 0; f < P->n_fam; ++f)
+            make_table_maps(maps[l].a[f], ws + f * fam, P->n_fam * fam, P->n_s, P->ld, 316);
 }
 
 // The low-rank mixed M2L of one level and family (R charge columns): the call of
-// m2l_tf32x3 / one entry of the batch's M2L queue.
+// m2l_split / one entry of the batch's M2L queue.
 MixedCall cx_call(hfmm_plan* P, int l, int f, int R) {
     LevelTables& T = P->tables[f][l];
     auto lb = [&](auto* buf, int cld) { return buf - (int64_t)P->level_lo[l] * R * cld; };
@@ -286,10 +282,10 @@ MixedCall cx_call(hfmm_plan* P, int l, int f, int R) {
     mc.ntiles = P->mx_tiles[l][R - 1].ntiles;
     mc.src_tab = P->m2l_src.p;
     mc.disp_compact = P->disp_compact.p;
-    mc.Bhi = lb(T.xc_hi.p, T.ckld);
-    mc.Blo = lb(T.xc_lo.p, T.ckld);
-    mc.Lhi = nullptr;
-    mc.Llo = nullptr;
+    mc.B = lb(T.xc_s.p, T.ckld);
+    mc.b_plane = T.xc_s.n / 2;
+    mc.b_max[0] = P->x_max.p + f * MAX_LEVELS + l;
+    mc.a_scale[0] = T.c_scale;
     mc.out = lb(T.yc.p, T.cmld);
     mc.src_lo = P->level_lo[l];   // the level's buffers hold its own boxes only
     mc.src_hi = P->level_hi[l];
@@ -297,9 +293,11 @@ MixedCall cx_call(hfmm_plan* P, int l, int f, int R) {
     mc.ld = T.cmld;
     mc.ldk = T.ckld;
     mc.ldm = T.cmld;
-    mc.m_valid = T.cr;   // rows r..cmld of the C_d tables are zero
+    // 24 MMAs a unit: the error of the low-rank M2L is 0.7 to 0.8 of that of TF32 halves at 24
+    // (12 a unit: 0.6, and 6.65 against 5.96 ms at 5e5 points, p = 8)
+    mc.fold2 = 1;
+    mc.valid = T.cr;   // rows r..cmld and columns r..ckld of the C_d tables are zero
     mc.n_fam = 1;
-    mc.has_l2l = 0;
     mc.fam_stride = 0;
     mc.out_fam_stride = 0;
     mc.nb = P->nb;
@@ -337,10 +335,10 @@ std::string queue_items(hfmm_plan* const* plans, int n_plans, int R, std::vector
                 calls.push_back(c);
                 maps.push_back(static_cast<MixedMaps*>(P->cx_maps)[f * MAX_LEVELS + l]);
                 const int blocks = (c.ldm + 127) / 128;
-                const int valid = c.m_valid > 0 ? c.m_valid : c.ldm;
+                const int valid = c.valid;
                 for (int t = 0; t < c.ntiles; ++t)
                     for (int b = 0; b < blocks; ++b) {
-                        const double cost = (double)(c.ldk / 32) * (valid - 128 * b <= 64 ? 0.6 : 1.0);
+                        const double cost = (double)valid * (valid - 128 * b <= 64 ? 0.6 : 1.0);
                         list.push_back({cost, M2LItem{id, t, b}});
                     }
             }
@@ -573,9 +571,10 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
     };
     // one-entry GEMM over every box of level l between layouts of different widths
     auto gemm_1 = [&](int kind, int l, int f, const double* in, int ldk, double* out, int ldm,
-                      cudaStream_t st, const double* scale = nullptr) {
+                      cudaStream_t st, const double* scale = nullptr, unsigned long long* most = nullptr) {
         GemmCall c{};
         c.scale = scale;
+        c.most = most;
         c.k_valid = kind == K_EXP ? P->tables[f][l].cr : P->n_s;   // compress reads y (n_s)
         c.tile_tgt = P->dec_tiles[l][R - 1].tgt.p;
         c.ntiles = P->dec_tiles[l][R - 1].ntiles;
@@ -595,23 +594,32 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
         c.nb = P->nb;
         gemm_f64(c, P->d_err.p, st);
     };
+    if (up && use_mx)
+        HFMM_CUDA(cudaMemsetAsync(P->x_max.p, 0, P->x_max.n * sizeof(unsigned long long), s));
     if (up && use_cx) {   // compress every level's densities (x' = y Vt_up U_c), then split them
         PhaseTimer pt(X, s, 14);
         for (int l = 2; l <= P->md; ++l)
             for (int f = 0; f < NF; ++f) {
                 LevelTables& T = P->tables[f][l];
                 gemm_1(K_CMP, l, f, P->equiv.p + f * fs, P->ld, level_base(T.xc.p, l, T.ckld), T.ckld,
-                       s);
+                       s, nullptr, P->x_max.p + f * MAX_LEVELS + l);
                 const int64_t nbl = P->level_hi[l] - P->level_lo[l];
                 if (R == 2 && T.grid && g_m2l_grid.load())   // complete level: into the dense grid
-                    split_tf32_grid(T.xc.p, P->m_id.p + P->level_lo[l], nbl, T.grid, T.ckld,
-                                    T.xg_hi.p, T.xg_lo.p, s);
+                    split_planes_grid(T.xc.p, P->x_max.p + f * MAX_LEVELS + l, P->m_id.p + P->level_lo[l], nbl, T.grid, T.ckld,
+                                      T.xg_s.p, s);
                 else
-                    split_tf32(T.xc.p, T.xc_hi.p, T.xc_lo.p, nbl * R * T.ckld, s);
+                    split_planes(T.xc.p, P->x_max.p + f * MAX_LEVELS + l, T.xc_s.p, T.xc_s.n / 2, nbl * R * T.ckld,
+                                 s);
             }
-    } else if (up && use_mx) {   // TF32 hi/lo halves of every equivalent density (B operand)
+    } else if (up && use_mx) {   // the planes of every equivalent density (B operand)
         PhaseTimer pt(X, s, 11);
-        split_tf32(P->equiv.p, P->e_hi.p, P->e_lo.p, (int64_t)NF * fs, s);
+        for (int f = 0; f < NF; ++f)
+            for (int l = 2; l <= P->md; ++l) {
+                const int64_t o = f * fs + (int64_t)P->level_lo[l] * R * P->ld;
+                const int64_t m = (int64_t)(P->level_hi[l] - P->level_lo[l]) * R * P->ld;
+                absmax(P->equiv.p + o, m, P->x_max.p + f * MAX_LEVELS + l, s);
+                split_planes(P->equiv.p + o, P->x_max.p + f * MAX_LEVELS + l, P->e_s.p + o, P->e_s.n / 2, m, s);
+            }
     }
     // split evaluate (a batch's queued M2L): the upward half ends here; the downward half
     // starts with every level's expansion of the queue's check potentials
@@ -661,7 +669,7 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
         auto launch = [&](int l, int f, cudaStream_t ss) {
             LevelTables& T = P->tables[f][l];
             MixedCall mc = cx_call(P, l, f, R);
-            m2l_tf32x3(static_cast<MixedMaps*>(P->cx_maps)[f * MAX_LEVELS + l], mc, ss);
+            m2l_split(static_cast<MixedMaps*>(P->cx_maps)[f * MAX_LEVELS + l], mc, ss);
             // expand into the level's downward coordinates: y_dn = d_dn .* (y' U_c^T U_dn)
             // (overwrites; the L2L and X list add to it on the main stream)
             gemm_1(K_EXP, l, f, level_base(T.yc.p, l, T.cmld), T.cmld, P->loc.p + f * fs, P->ld,
@@ -729,24 +737,27 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
             mc.ntiles = P->mx_tiles[l][R - 1].ntiles;
             mc.src_tab = P->m2l_src.p;
             mc.disp_compact = P->disp_compact.p;
-            mc.Bhi = P->e_hi.p;
-            mc.Blo = P->e_lo.p;
-            mc.Lhi = nullptr;
-            mc.Llo = nullptr;
+            mc.B = P->e_s.p;
+            mc.b_plane = P->e_s.n / 2;
+            for (int f = 0; f < NF; ++f) {
+                mc.b_max[f] = P->x_max.p + f * MAX_LEVELS + l;
+                mc.a_scale[f] = m2l_scale(P, f, l);
+            }
+            mc.fold2 = 0;   // dense tables: 24 MMAs a unit gave 1.1 of the TF32 halves' error, 12 give 0.6
+            mc.valid = P->n_s;
             mc.out = P->check.p;
             mc.R = R;
             mc.ld = P->ld;
             mc.n_fam = NF;
-            mc.has_l2l = 0;   // L2L stays FP64 (below): the downward locals are ill-conditioned
             mc.fam_stride = fs;
             mc.out_fam_stride = fs;
             mc.nb = P->nb;
             mc.err = P->d_err.p;
             {
                 PhaseTimer pt(X, s, 4);
-                m2l_tf32x3(static_cast<MixedMaps*>(P->mx_maps)[l], mc, s);
+                m2l_split(static_cast<MixedMaps*>(P->mx_maps)[l], mc, s);
             }
-            if (l >= 3)   // L2L (phases.py:273-278) in FP64, added to the check potential
+            if (l >= 3)   // L2L (phases.py:273-278) stays FP64 (ill-conditioned locals), added
                 gemm(K_L2L, l, P->dn_tiles[l][R - 1], P->m2l_src.p + N_DISP, M2L_ENTRIES, P->loc.p,
                      nullptr, P->check.p);
         } else if (use_conv) {   // the check potentials hold the M2L's: add the parent's
@@ -1135,8 +1146,8 @@ int hfmm_plan_finalize(hfmm_plan* P) {
     P->equiv.zero();
     P->loc.zero();
     P->tmp.zero();
-    // mixed path: TF32 hi/lo tables, tensor maps, split density buffers (needs ld >= 128);
-    // with a compressed M2L on every level the dense TF32 tables are not needed
+    // mixed path: the tables' FP16 planes, tensor maps, split density buffers (needs ld >= 128);
+    // with a compressed M2L on every level the dense planes are not needed
     if (P->ld >= 128) {
         std::vector<int32_t> dc(N_DISP, -1);
         auto madj = nonadjacent_map();
@@ -1152,25 +1163,22 @@ int hfmm_plan_finalize(hfmm_plan* P) {
         } else if (P->streamed) {
             if (P->ws) stream_maps(P);
         } else {
-            DevBuf<double> dense;   // one level's matrices, for their halves only
+            DevBuf<double> dense;   // one level's matrices, for their planes only
             for (int f = 0; f < P->n_fam; ++f)
                 for (int l = 2; l <= P->md; ++l) {
                     LevelTables& T = P->tables[f][l];
                     const int nm = (int)madj.size();
-                    if (!T.m2l_hi.p) {
+                    if (!T.m2l_s.p) {
                         if (!T.m2l.p) generate_m2l(P, f, l, dense);
-                        T.m2l_hi.alloc(nm * mat);
-                        T.m2l_lo.alloc(nm * mat);
-                        split_transpose_tables(T.m2l.p ? T.m2l.p : dense.p, T.m2l_hi.p, T.m2l_lo.p, P->ld, nm);
+                        T.m2l_s.alloc(2 * nm * mat);
+                        split_transpose_tables(T.m2l.p ? T.m2l.p : dense.p, m2l_scale(P, f, l), T.m2l_s.p, P->ld, nm);
                     }
-                    make_table_map(&maps[l].a_hi[f], T.m2l_hi.p, P->ld, nm);
-                    make_table_map(&maps[l].a_lo[f], T.m2l_lo.p, P->ld, nm);
+                    make_table_maps(maps[l].a[f], T.m2l_s.p, nm * mat, P->n_s, P->ld, nm);
                 }
         }
-        P->e_hi.alloc(exp);
-        P->e_lo.alloc(exp);
-        P->e_hi.zero();
-        P->e_lo.zero();
+        P->e_s.alloc(2 * exp);
+        P->e_s.zero();
+        P->x_max.alloc(2 * MAX_LEVELS);
         P->mixed_ready = true;
     }
     plan_queue_build(P);

@@ -1,8 +1,8 @@
 // Compressed M2L of the mixed path: the 316 M2L matrices of a level share their
 // dominant subspace U (n_s x r), so K_d ~ U C_d U^T with C_d = U^T K_d U (r x r).
 // The M2L of a level then runs as: compress the densities (x' = U^T x, FP64
-// GEMM), apply the C_d per V pair on the tensor cores (3xTF32, the kernel of
-// m2l_tf32x3.cu with ld = the padded rank), expand (y = U y', FP64 GEMM) into
+// GEMM), apply the C_d per V pair on the tensor cores (two FP16 planes, the
+// kernels of m2l_split.cu and m2l_queue.cu with ld = the padded rank), expand (y = U y', FP64 GEMM) into
 // the check potential. No counterpart in the reference, which applies every
 // K_d densely (jaxfmm/kifmm/phases.py:176-237); U and C_d come from the host
 // library (hfmm_b200/compress.py: leading eigenvectors of sum_d K_d K_d^T).
@@ -36,22 +36,15 @@ __global__ void k_pack_exp(const double* __restrict__ U, int n_s, int r, int ld,
     out[(int64_t)k * ld + m] = (k < r && m < n_s) ? U[(int64_t)m * r + k] : 0.0;
 }
 
-__device__ __forceinline__ float tf32_round(float x) {
-    return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
-}
-
-// C_d as TF32 hi/lo halves in the A layout [d][m][k] of the tcgen05 kernel (cmld x ckld)
-__global__ void k_pack_c(const double* __restrict__ C, int r, int ckld, int cmld, float* hi,
-                         float* lo) {
+// C_d as FP16 planes in the A layout [plane][d][m][k] of the tcgen05 kernel (cmld x ckld)
+__global__ void k_pack_c(const double* __restrict__ C, int r, int ckld, int cmld, double scale, uint16_t* out) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int m = blockIdx.y;
     const int d = blockIdx.z;
     if (k >= ckld || m >= cmld) return;
-    const double v = (m < r && k < r) ? C[((int64_t)d * r + m) * r + k] : 0.0;
-    const float h = tf32_round((float)v);
-    const int64_t o = ((int64_t)d * cmld + m) * ckld + k;
-    hi[o] = h;
-    lo[o] = tf32_round((float)(v - (double)h));
+    uint16_t p[2];
+    split2((m < r && k < r) ? C[((int64_t)d * r + m) * r + k] * scale : 0.0, p);
+    for (int i = 0; i < 2; ++i) out[(((int64_t)i * N_M2L + d) * cmld + m) * ckld + k] = p[i];
 }
 
 // C = A B for row-major FP64 matrices, batched over blockIdx.z with element strides
@@ -135,28 +128,22 @@ void compressed_prepare(hfmm_plan* P) {
             const size_t rows = (size_t)(P->level_hi[l] - P->level_lo[l]) * 2;   // R <= 2
             T.xc.alloc(rows * T.ckld);
             T.yc.alloc(rows * T.cmld);
-            T.xc_hi.alloc(rows * T.ckld);
-            T.xc_lo.alloc(rows * T.ckld);
+            T.xc_s.alloc(2 * rows * T.ckld);
             T.xc.zero();
             T.yc.zero();
-            T.xc_hi.zero();
-            T.xc_lo.zero();
-            make_table_map(&maps[f * MAX_LEVELS + l].a_hi[0], T.c_hi.p, T.ckld, N_M2L, T.cmld);
-            make_table_map(&maps[f * MAX_LEVELS + l].a_lo[0], T.c_lo.p, T.ckld, N_M2L, T.cmld);
+            T.xc_s.zero();
+            make_table_maps(maps[f * MAX_LEVELS + l].a[0], T.c_s.p, (size_t)N_M2L * T.cmld * T.ckld, T.cr, T.ckld,
+                            N_M2L, T.cmld);
             // complete level: the complex-charge M2L reads its densities from a dense grid
             T.grid = 0;
-            T.xg_hi.release();
-            T.xg_lo.release();
             if (P->gx_tiles[l].ntiles > 0) {
                 const int G = 1 << l;
-                const size_t cells = (size_t)G * G * G * 2 * T.ckld;
-                T.xg_hi.alloc(cells);
-                T.xg_lo.alloc(cells);
-                T.xg_hi.zero();
-                T.xg_lo.zero();
-                make_grid_map(&maps[f * MAX_LEVELS + l].b_hi[0], T.xg_hi.p, T.ckld, G);
-                make_grid_map(&maps[f * MAX_LEVELS + l].b_lo[0], T.xg_lo.p, T.ckld, G);
+                T.xg_s.alloc(2 * (size_t)G * G * G * 2 * T.ckld);
+                T.xg_s.zero();
+                make_grid_maps(maps[f * MAX_LEVELS + l].b[0], T.xg_s.p, T.cr, T.ckld, G);
                 T.grid = G;
+            } else {
+                T.xg_s.release();
             }
         }
     if (!P->folded) {   // a plan rebuilt for moved points keeps its tables
@@ -222,14 +209,20 @@ int hfmm_plan_set_m2l_compressed(hfmm_plan* P, int32_t family, int32_t level, in
         T.cmld = cmld;
         T.c_cmp.alloc((size_t)P->ld * ckld);
         T.c_exp.alloc((size_t)cmld * P->ld);
-        T.c_hi.alloc((size_t)N_M2L * cmld * ckld);
-        T.c_lo.alloc((size_t)N_M2L * cmld * ckld);
+        T.c_s.alloc(2 * (size_t)N_M2L * cmld * ckld);
+        DevBuf<unsigned long long> most;
+        most.alloc(1);
+        most.zero();
+        absmax(C_dev, (int64_t)N_M2L * rank * rank, most.p, 0);
+        unsigned long long h_most = 0;
+        HFMM_CUDA(cudaMemcpy(&h_most, most.p, sizeof(h_most), cudaMemcpyDeviceToHost));
+        T.c_scale = plane_scale(h_most);
         HFMM_LAUNCH(k_pack_cmp, dim3((unsigned)ceil_div(ckld, 128), (unsigned)P->ld), 128, 0, 0,
                     U_dev, P->n_s, rank, P->ld, ckld, T.c_cmp.p);
         HFMM_LAUNCH(k_pack_exp, dim3((unsigned)ceil_div(P->ld, 128), (unsigned)cmld), 128, 0, 0,
                     U_dev, P->n_s, rank, P->ld, cmld, T.c_exp.p);
         HFMM_LAUNCH(k_pack_c, dim3((unsigned)ceil_div(ckld, 128), (unsigned)cmld, N_M2L), 128, 0, 0,
-                    C_dev, rank, ckld, cmld, T.c_hi.p, T.c_lo.p);
+                    C_dev, rank, ckld, cmld, T.c_scale, T.c_s.p);
         HFMM_CUDA(cudaDeviceSynchronize());
         P->finalized = false;
         return HFMM_OK;

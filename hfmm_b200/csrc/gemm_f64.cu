@@ -250,6 +250,23 @@ __global__ void __launch_bounds__(128, 3) k_gemm_f64(GemmCall c, int* err) {
     double* part = S > 1 ? c.part + ((int64_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * TN * TM
                          : nullptr;
     const double* sc = (fam == 1 && c.scale_f1) ? c.scale_f1 : c.scale;
+    if (c.most) {   // (one-entry calls without scale or split: what is stored is acc)
+        double top = 0.0;
+        bool odd = false;   // infinities and NaN: the largest bits there are
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            const double v = fabs((&acc[0][0][0])[i]);
+            odd = odd || !(v <= 1.7976931348623157e308);
+            top = fmax(top, v);
+        }
+        unsigned long long bits = odd ? 0x7ff0000000000000ull : (unsigned long long)__double_as_longlong(top);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long v = __shfl_xor_sync(0xffffffffu, bits, o);
+            bits = v > bits ? v : bits;
+        }
+        if (lane == 0 && bits) atomicMax(c.most, bits);
+    }
 #pragma unroll
     for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
@@ -332,6 +349,8 @@ void gemm_f64(const GemmCall& call, int* d_err, cudaStream_t s) {
     const int64_t ctas = (int64_t)grid.x * grid.y * grid.z;
     const int sms = sm_count();
     int S = 1;
+    if (c.most && (c.scale || c.accumulate || c.n_entries != 1))
+        throw Error{HFMM_ERR_STATE, "gemm_f64: largest magnitude of a plain one-entry call only"};
     if (c.part && c.n_entries > 1 && ctas < 4 * sms) {
         S = (int)std::min<int64_t>({(int64_t)c.n_entries, 16, (4 * sms + ctas - 1) / ctas});
         while (S > 1 && ctas * S * TN * TM > c.part_cap) --S;

@@ -105,19 +105,21 @@ struct LevelTables {
     // E (complex, interleaved) and the coaxial shift matrices of every distance
     DevBuf<double> rot_Q, rot_E, rot_C;
     double rot_pref = 0.0;
-    // mixed path: TF32 hi/lo halves of M2L and L2L as A[m][k] (fp32 containers)
-    DevBuf<float> m2l_hi, m2l_lo, l2l_hi, l2l_lo;
+    // mixed path: the two FP16 planes of the M2L tables as A [plane][316][m][k]
+    DevBuf<uint16_t> m2l_s;
+    double c_scale = 1.0;          // scale of the C_d planes
     // compressed M2L of the mixed path, K_d ~ U C_d U^T (rank cr): the K side padded
     // to ckld (>= 32), the M side to cmld (>= 128, the MMA tile), both multiples of 32
     int cr = 0, ckld = 0, cmld = 0;
     DevBuf<double> c_cmp, c_exp;   // A^T of U^T (ld -> ckld) and of U (cmld -> ld)
-    DevBuf<float> c_hi, c_lo;      // C_d halves as A [316][cmld][ckld]
+    DevBuf<uint16_t> c_s;          // C_d planes as A [plane][316][cmld][ckld]
     DevBuf<double> xc, yc;         // the level's compressed densities [.][R][ckld] and
-    DevBuf<float> xc_hi, xc_lo;    // check potentials [.][R][cmld] (box - level_lo first)
+                                   // check potentials [.][R][cmld] (box - level_lo first)
+    DevBuf<uint16_t> xc_s;         // the densities' planes [plane][.][R][ckld]
     // a complete level's split densities as a dense box grid [x][y][z][2][ckld] (complex
     // charges): a target tile's sources at one displacement are then one strided TMA box
     int grid = 0;                  // grid side 2^level when the grid is in use, else 0
-    DevBuf<float> xg_hi, xg_lo;
+    DevBuf<uint16_t> xg_s;
     // the low-rank plan's folded tables (row-major right multipliers, zero padded):
     // the decodes' Vt and U taken into the operators next to them, so a box keeps its
     // densities as scaled SVD coordinates (d .* (U^T x)) through both passes
@@ -129,13 +131,13 @@ struct LevelTables {
         up_U.release(); up_d.release(); up_Vt.release();
         dn_U.release(); dn_d.release(); dn_Vt.release();
         m2m.release(); l2l.release(); m2l.release();
-        m2l_hi.release(); m2l_lo.release(); l2l_hi.release(); l2l_lo.release();
+        m2l_s.release();
         cr = ckld = cmld = 0;
-        c_cmp.release(); c_exp.release(); c_hi.release(); c_lo.release();
+        c_cmp.release(); c_exp.release(); c_s.release();
         rot_Q.release(); rot_E.release(); rot_C.release();
-        xc.release(); yc.release(); xc_hi.release(); xc_lo.release();
+        xc.release(); yc.release(); xc_s.release();
         grid = 0;
-        xg_hi.release(); xg_lo.release();
+        xg_s.release();
         m2m_f.release(); l2l_f.release(); cmp_f.release(); exp_f.release();
         set = host_m2l = false;
     }
@@ -230,7 +232,8 @@ struct hfmm_plan {
     Tiles gx_tiles[hfmm::MAX_LEVELS];
     hfmm::DevBuf<int32_t> gx_org[hfmm::MAX_LEVELS];
     hfmm::DevBuf<int32_t> disp_compact;     // 343 -> M2L table index or -1
-    hfmm::DevBuf<float> e_hi, e_lo, l_hi, l_lo;   // split densities [fam][box][R][ld]
+    hfmm::DevBuf<uint16_t> e_s;             // split densities [plane][fam][box][R][ld]
+    hfmm::DevBuf<unsigned long long> x_max; // [fam][level] largest magnitude of the densities split
     void* mx_maps = nullptr;                // MixedMaps per level (host array)
     bool compressed = false;                // every level has a compressed M2L (mixed path)
     bool folded = false;                    // its folded tables are those of the current tables
@@ -283,6 +286,7 @@ void schedules_build(hfmm_plan* P);
 void upload_level(hfmm_plan* P, int fam, int level, const double* const* h);
 void generate_tables(hfmm_plan* P, int fam, int level);
 void generate_m2l(hfmm_plan* P, int fam, int level, DevBuf<double>& out);
+double m2l_scale(const hfmm_plan* P, int fam, int level);
 // M2L by convolution (m2l_conv.cu): the lattice of the surface given to set_kernel; the
 // spectra; the current tree's slots and workspace; one evaluate's M2L into P->check
 bool conv_surface(hfmm_plan* P, const double* equiv);
@@ -334,6 +338,7 @@ struct GemmCall {
     int64_t a_fam_stride;      // entries between the families' A pointer sets
     int n_fam;
     int64_t nb;                // box count (bounds checks)
+    unsigned long long* most;  // nullable: raised to the bits of the largest magnitude stored
     double* part;              // nullable: scratch for entry splits of small grids
     int64_t part_cap;          // its size in doubles
     int n_split;               // set by gemm_f64: CTAs per output tile (entry ranges)

@@ -1,4 +1,4 @@
-// Shared pieces of the tcgen05 M2L kernels (m2l_tf32x3.cu: one launch per level and
+// Shared pieces of the tcgen05 M2L kernels (m2l_split.cu: one launch per level and
 // family; m2l_queue.cu: one persistent launch over a queue of such work): tile and
 // stage geometry, warp roles and their register split, the bounded mbarrier waits,
 // the TMA / UMMA / TMEM instruction wrappers and the per-CTA control block.
@@ -13,20 +13,19 @@ namespace mxk {
 
 constexpr int BM = 128;          // UMMA M (check points per CTA)
 constexpr int BN = 128;          // UMMA N (target columns per CTA)
-// fp32 elements per k-chunk: 32 (128-byte rows, SWIZZLE_128B, three 64 KiB stages) or
-// 16 (64-byte rows, SWIZZLE_64B, six 32 KiB stages), the same 192 KiB of operands in
-// flight. Same results bit for bit; on the 1M-point p = 8 low-rank M2L 32 took 11.5 ms
-// and 16 took 14.0: each stage carries a fixed cost of about 0.3 us that the MMAs do
-// not hide, so fewer, larger stages win.
-#ifndef HFMM_MX_BK
-#define HFMM_MX_BK 32
-#endif
-constexpr int BK = HFMM_MX_BK;
-static_assert(BK == 16 || BK == 32, "k-chunk");
-constexpr int ROW_BYTES = BK * 4;           // one K-major row of a tile
+// Operands are two FP16 planes of the scaled value (mixed.cuh: split2), 11 significant bits
+// each, and a product is hi hi + hi lo + lo hi: the 22 bits of two TF32 halves in half their
+// bytes, at twice the K per MMA. What bounds the kernel is the MMAs' reading of their operands
+// from shared memory (8 KB each, about 140 cycles), so half as many MMAs take half the time:
+// 5e5 points, p = 8, all levels and both families 8.46 ms with TF32 halves, 5.96 with these.
+// (Three BF16 planes, six products and 6 bytes a value, took 9.04: as many MMAs as TF32.)
+constexpr int PLANES = 2;
+constexpr int BK = 64;                      // K values per k-chunk: 128-byte rows, SWIZZLE_128B
+constexpr int KSTEP = 16;                   // K values per MMA
+constexpr int ROW_BYTES = BK * 2;           // one K-major row of a tile
 constexpr int CPR = ROW_BYTES / 16;         // 16-byte chunks per row
-constexpr int TILE_BYTES = BM * ROW_BYTES;  // one operand half
-constexpr int STAGE_BYTES = 4 * TILE_BYTES;
+constexpr int TILE_BYTES = BM * ROW_BYTES;  // one operand plane
+constexpr int STAGE_BYTES = 2 * PLANES * TILE_BYTES;
 constexpr int STAGES = (3 * 64 * 1024) / STAGE_BYTES;
 constexpr int N_FOLD_WARPS = 16;                  // four per TMEM lane quadrant
 constexpr int FOLD_WARP0 = 8;                     // warps 0-3 gather, 4 TMA, 5 MMA, 6-7 idle
@@ -38,7 +37,6 @@ constexpr int TMEM_COLS = NACC * BN;              // 512
 constexpr int REG_GATHER = 64, REG_CTRL = 32, REG_FOLD = 96;
 static_assert(128 * REG_GATHER + 128 * REG_CTRL + 32 * N_FOLD_WARPS * REG_FOLD <= THREADS * 80,
               "register split exceeds an 80-register launch");
-constexpr int FOLD = 64 / BK;   // k-chunks per FP32 accumulation unit: 64 K values, 24 MMAs
 constexpr uint64_t WAIT_NS = 2000000000ull;   // bounded waits: 2 s
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -113,18 +111,30 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
         : "memory");
 }
 // UMMA shared-memory descriptor: K-major, swizzled rows of ROW_BYTES (layout type 2 =
-// SWIZZLE_128B, 4 = SWIZZLE_64B), 8-row groups 8 * ROW_BYTES apart.
+// SWIZZLE_128B), 8-row groups 8 * ROW_BYTES apart.
 __device__ __forceinline__ uint64_t sw_desc(uint32_t addr) {
-    constexpr uint64_t layout = BK == 32 ? 2 : 4;
+    constexpr uint64_t layout = 2;
     return (uint64_t)((addr & 0x3FFFF) >> 4) | (1ull << 16) |
            ((uint64_t)(8 * ROW_BYTES / 16) << 32) | (1ull << 46) | (layout << 61);
 }
-__device__ __forceinline__ void umma_tf32(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc,
+__device__ __forceinline__ void umma_f16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc,
                                           uint32_t acc) {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
         "l"(a), "l"(b), "r"(idesc), "r"(acc));
+}
+// One stage's MMAs: k-steps of the three plane products into the accumulator at dt, which the
+// first one overwrites when `first`. base: the stage's A planes, then its B planes.
+__device__ __forceinline__ void stage_mmas(uint32_t dt, uint32_t base, int ksteps, uint32_t idesc, bool first) {
+    const uint64_t ah = sw_desc(base), al = sw_desc(base + TILE_BYTES);
+    const uint64_t bh = sw_desc(base + 2 * TILE_BYTES), bl = sw_desc(base + 3 * TILE_BYTES);
+    for (int ks = 0; ks < ksteps; ++ks) {   // 16 values = 32 bytes per k-step
+        const uint64_t d = (uint64_t)(ks * 2);
+        umma_f16(dt, ah + d, bh + d, idesc, ks > 0 || !first ? 1u : 0u);
+        umma_f16(dt, ah + d, bl + d, idesc, 1u);
+        umma_f16(dt, al + d, bh + d, idesc, 1u);
+    }
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
@@ -140,9 +150,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* v) {
           "=r"(v[14]), "=r"(v[15])
         : "r"(taddr));
 }
-// Instruction descriptor: D = F32, A = B = TF32, both K-major, M = 128 (or 64), N = BN.
+// Instruction descriptor: D = F32, A = B = F16, both K-major, M = 128 (or 64), N = BN.
 constexpr uint32_t idesc_m(int m) {
-    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BN >> 3) << 17) |
+    return (1u << 4) | ((uint32_t)(BN >> 3) << 17) |
            ((uint32_t)(m >> 4) << 24);
 }
 constexpr uint32_t IDESC = idesc_m(BM);

@@ -3,16 +3,16 @@
 // A batch of plans (batch.cu) runs every plan's upward pass, then ONE launch of this
 // kernel for the M2L of every plan, level and kernel family, then every plan's
 // downward pass. Each work item is one target tile x one 128-row block of one
-// (plan, level, family) M2L -- the unit one CTA of k_m2l_tf32x3 computes -- and the
+// (plan, level, family) M2L -- the unit one CTA of k_m2l_split computes -- and the
 // items are queued by decreasing cost, so large levels start first and the small
 // problems' few coarse tiles fill the tail. One CTA per SM stays resident and takes
 // the next item with an atomic counter until the queue is empty: tensor memory is
 // allocated, mbarriers initialised and registers split once per CTA, and the stage
 // and accumulation-unit counters run on across items, so consecutive items keep the
-// pipeline's barrier phases. The per-item arithmetic is k_m2l_tf32x3's (3xTF32
+// pipeline's barrier phases. The per-item arithmetic is k_m2l_split's (three FP16 plane
 // products, FP32 units of 24 MMAs folded into FP64 sums held in registers), the call
 // parameters (MixedCall) and the TMA tensor maps of every (plan, level, family) come
-// from global memory. Every wait is bounded as in k_m2l_tf32x3; a timeout stops the
+// from global memory. Every wait is bounded as in k_m2l_split; a timeout stops the
 // CTA after the item, drains what it issued and frees tensor memory.
 #include "hfmm_internal.cuh"
 #include "m2l_common.cuh"
@@ -77,7 +77,7 @@ __device__ __forceinline__ bool next_item(QueueCtl& ctl, const MixedCall* __rest
         }
         for (int e = ft; e < M2L_ENTRIES; e += 32 * N_FOLD_WARPS) {
             ctl.used[e] = 0;
-            ctl.ztab[e] = (short)(e < N_DISP ? c.disp_compact[e] : (c.has_l2l ? e - N_DISP : -1));
+            ctl.ztab[e] = (short)(e < N_DISP ? c.disp_compact[e] : -1);
         }
     }
     __syncthreads();
@@ -170,10 +170,10 @@ __global__ void __launch_bounds__(THREADS, 1)
     // stages and accumulation units this CTA has issued before the current item.
     int q_total = 0, u_total = 0;
     if (warp < 4) {
-        // ---------------- B gathers (k_m2l_tf32x3's, for items that are not in grid mode)
+        // ---------------- B gathers (k_m2l_split's, for items that are not in grid mode)
         while (next_item<R, false>(ctl, calls, items, n_items, next, warp, lane, tid)) {
             const MixedCall& c = ctl.c;
-            const int kch = c.ldk / BK, nq = ctl.n_act * kch;
+            const int kch = (c.valid + BK - 1) / BK, nq = ctl.n_act * kch;
             if (!c.grid) {
                 constexpr int RSTEP = 128 / CPR;
                 const int ch = tid % CPR;
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
                 for (int i = 0; i < CPR; ++i) {
                     const int n = tid / CPR + RSTEP * i;
-                    const int sw = BK == 32 ? (n & 7) : ((n & 7) >> 1);
+                    const int sw = n & 7;
                     soff[i] = (uint32_t)((n >> 3) * 8 * ROW_BYTES + (n & 7) * ROW_BYTES + ((ch ^ sw) << 4));
                     goff[i] = -1;
                 }
@@ -204,19 +204,19 @@ __global__ void __launch_bounds__(THREADS, 1)
                                 atomicOr(c.err, ERRF_BOUNDS);
                                 s_ = -1;
                             }
-                            goff[i] = s_ >= 0 ? (s_ * R + (n % R)) * c.ldk + ch * 4 : -1;
+                            goff[i] = s_ >= 0 ? (s_ * R + (n % R)) * c.ldk + ch * 8 : -1;
                         }
                     }
                     if (!mbar_wait(smem_u32(&ctl.empty[st]), ((qg / STAGES) & 1) ^ 1, abort_flag, wait_ns)) break;
                     const int k0 = (q % kch) * BK;
-                    const uint32_t sbh = smem_u32(sm + st * STAGE_BYTES + 2 * TILE_BYTES);
-                    const uint32_t sbl = sbh + TILE_BYTES;
+                    const uint32_t sb = smem_u32(sm + st * STAGE_BYTES + PLANES * TILE_BYTES);
 #pragma unroll
                     for (int i = 0; i < CPR; ++i) {
-                        const bool ok = goff[i] >= 0;
-                        const int o = ok ? goff[i] + k0 : 0;
-                        cp_async16(sbh + soff[i], c.Bhi + o, ok);
-                        cp_async16(sbl + soff[i], c.Blo + o, ok);
+                        const bool ok = goff[i] >= 0 && k0 + ch * 8 < c.ldk;
+                        const int64_t o = ok ? goff[i] + k0 : 0;
+#pragma unroll
+                        for (int pl = 0; pl < PLANES; ++pl)
+                            cp_async16(sb + pl * TILE_BYTES + soff[i], c.B + pl * c.b_plane + o, ok);
                     }
                     if (!(starve && qg == 0))   // (test: the CTA's first stage never fills)
                         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(
@@ -236,9 +236,9 @@ __global__ void __launch_bounds__(THREADS, 1)
         while (next_item<R, true>(ctl, calls, items, n_items, next, warp, lane, tid)) {
             const MixedCall& c = ctl.c;
             const int m0 = items[ctl.item].mblock * BM;
-            const bool half = (c.m_valid > 0 ? c.m_valid : c.ldm) - m0 <= 64;
-            const int kch = c.ldk / BK, nq = ctl.n_act * kch;
-            const int n_units = (nq + FOLD - 1) / FOLD;
+            const bool half = c.valid - m0 <= 64;
+            const int kch = (c.valid + BK - 1) / BK, nq = ctl.n_act * kch;
+            const int n_units = (nq + (1 << c.fold2) - 1) >> c.fold2;
             const int m = half ? m0 + quad * 16 + lane : m0 + quad * 32 + lane;
             const bool row_ok = half ? (lane < 16 && m < c.ldm) : (m0 + quad * 32 < c.ldm);
             double sum[COLS_PER_FOLD_WARP];
@@ -269,11 +269,12 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (aborted) {
                 if (lane == 0) atomicOr(c.err, ERRF_TIMEOUT);
             } else if (row_ok) {
+                const double unscale = 1.0 / (c.a_scale[0] * plane_scale(*c.b_max[0]));
 #pragma unroll
                 for (int j = 0; j < COLS_PER_FOLD_WARP; ++j) {
                     const int n = c_lo + j;
                     const int t = ctl.tgt[n / R];
-                    if (t >= 0) c.out[((int64_t)t * R + (n % R)) * c.ldm + m] = sum[j];
+                    if (t >= 0) c.out[((int64_t)t * R + (n % R)) * c.ldm + m] = sum[j] * unscale;
                 }
             }
             u_total += n_units;
@@ -287,23 +288,23 @@ __global__ void __launch_bounds__(THREADS, 1)
         int* err = nullptr;
         while (next_item<R, false>(ctl, calls, items, n_items, next, warp, lane, tid)) {
             const MixedCall& c = ctl.c;
-            const int kch = c.ldk / BK, nq = ctl.n_act * kch;
+            const int kch = (c.valid + BK - 1) / BK, nq = ctl.n_act * kch;
             if (lane == 0) {
                 err = c.err;
                 const int tile = items[ctl.item].tile, m0 = items[ctl.item].mblock * BM;
                 const MixedMaps* mp = maps + items[ctl.item].call;
-                const CUtensorMap* mh = &mp->a_hi[0];
-                const CUtensorMap* ml = &mp->a_lo[0];
-                const CUtensorMap* bh = &mp->b_hi[0];
-                const CUtensorMap* bl = &mp->b_lo[0];
                 // the maps were written through the generic proxy (a host copy): make them
                 // visible to the tensor-map proxy before their use in this item
-                asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(mh) : "memory");
-                asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(ml) : "memory");
+#pragma unroll
+                for (int pl = 0; pl < PLANES; ++pl)
+                    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&mp->a[0][pl])
+                                 : "memory");
                 int ox = 0, oy = 0, oz = 0;
                 if (c.grid) {
-                    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(bh) : "memory");
-                    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(bl) : "memory");
+#pragma unroll
+                    for (int pl = 0; pl < PLANES; ++pl)
+                        asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&mp->b[0][pl])
+                                     : "memory");
                     ox = c.tile_org[3 * (int64_t)tile];
                     oy = c.tile_org[3 * (int64_t)tile + 1];
                     oz = c.tile_org[3 * (int64_t)tile + 2];
@@ -317,13 +318,15 @@ __global__ void __launch_bounds__(THREADS, 1)
                     const int k0 = (q % kch) * BK;
                     const uint32_t fb = smem_u32(&ctl.tfull[st]);
                     const uint32_t sa = smem_u32(sm + st * STAGE_BYTES);
-                    mbar_arrive_tx(fb, (c.grid ? 4 : 2) * TILE_BYTES);
-                    tma_load_3d(sa, mh, k0, m0, z, fb);
-                    tma_load_3d(sa + TILE_BYTES, ml, k0, m0, z, fb);
+                    mbar_arrive_tx(fb, (c.grid ? 2 : 1) * PLANES * TILE_BYTES);
+#pragma unroll
+                    for (int pl = 0; pl < PLANES; ++pl)
+                        tma_load_3d(sa + pl * TILE_BYTES, &mp->a[0][pl], k0, m0, z, fb);
                     if (c.grid) {
                         const int sx = ox - (e / 49 - 3), sy = oy - ((e / 7) % 7 - 3), sz = oz - (e % 7 - 3);
-                        tma_load_5d(sa + 2 * TILE_BYTES, bh, k0, 0, sz, sy, sx, fb);
-                        tma_load_5d(sa + 3 * TILE_BYTES, bl, k0, 0, sz, sy, sx, fb);
+#pragma unroll
+                        for (int pl = 0; pl < PLANES; ++pl)
+                            tma_load_5d(sa + (PLANES + pl) * TILE_BYTES, &mp->b[0][pl], k0, 0, sz, sy, sx, fb);
                     }
 #pragma unroll
                     for (int j = 0; j < STAGES; ++j)
@@ -350,44 +353,39 @@ __global__ void __launch_bounds__(THREADS, 1)
         uint32_t full_par = 0;
         while (next_item<R, false>(ctl, calls, items, n_items, next, warp, lane, tid)) {
             const MixedCall& c = ctl.c;
-            const int kch = c.ldk / BK, nq = ctl.n_act * kch;
-            const int n_units = (nq + FOLD - 1) / FOLD;
+            const int kch = (c.valid + BK - 1) / BK, nq = ctl.n_act * kch;
+            const int n_units = (nq + (1 << c.fold2) - 1) >> c.fold2;
             if (lane == 0) {
                 err = c.err;
                 const int m0 = items[ctl.item].mblock * BM;
-                const bool half = (c.m_valid > 0 ? c.m_valid : c.ldm) - m0 <= 64;
+                const bool half = c.valid - m0 <= 64;
                 const uint32_t idesc = half ? IDESC64 : IDESC;
+                const int fold2 = c.fold2, last = (1 << fold2) - 1, valid = c.valid;
+                const bool gridded = c.grid;
+                int kc = 0;   // k-chunk within the entry
                 for (int q = 0; q < nq; ++q) {
                     const int qg = q_total + q, st = qg % STAGES;
-                    const int u = q / FOLD, uq = q % FOLD;
+                    const int u = q >> fold2, uq = q & last;
                     const int ug = u_total + u, b = ug & (NACC - 1);
                     if (uq == 0 && ug >= NACC) {
                         if (!mbar_wait(smem_u32(&ctl.acc_empty[b]), ((ug / NACC) & 1) ^ 1, abort_flag, wait_ns))
                             break;
                         asm volatile("tcgen05.fence::after_thread_sync;");
                     }
-                    if (!c.grid) {
+                    if (!gridded) {
                         if (!mbar_wait(smem_u32(&ctl.full[st]), (full_par >> st) & 1u, abort_flag, wait_ns))
                             break;
                         full_par ^= 1u << st;
                     }
                     if (!mbar_wait(smem_u32(&ctl.tfull[st]), (qg / STAGES) & 1, abort_flag, wait_ns)) break;
-                    if (!c.grid) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    if (!gridded) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     asm volatile("tcgen05.fence::after_thread_sync;");
-                    const uint32_t base = smem_u32(sm + st * STAGE_BYTES);
-                    const uint64_t ah = sw_desc(base), al = sw_desc(base + TILE_BYTES);
-                    const uint64_t bh = sw_desc(base + 2 * TILE_BYTES), bl = sw_desc(base + 3 * TILE_BYTES);
-                    const uint32_t dt = tmem + b * BN;
-#pragma unroll
-                    for (int ks = 0; ks < BK / 8; ++ks) {
-                        const uint64_t d = (uint64_t)(ks * 2);
-                        umma_tf32(dt, ah + d, bh + d, idesc, (uq > 0 || ks > 0) ? 1u : 0u);
-                        umma_tf32(dt, ah + d, bl + d, idesc, 1u);
-                        umma_tf32(dt, al + d, bh + d, idesc, 1u);
-                    }
+                    stage_mmas(tmem + b * BN, smem_u32(sm + st * STAGE_BYTES),
+                               (min(BK, valid - kc * BK) + KSTEP - 1) / KSTEP, idesc, uq == 0);
+                    kc = kc + 1 == kch ? 0 : kc + 1;
                     issued = true;
                     umma_commit(smem_u32(&ctl.empty[st]));
-                    if (uq == FOLD - 1 || q == nq - 1) umma_commit(smem_u32(&ctl.acc_full[b]));
+                    if (uq == last || q == nq - 1) umma_commit(smem_u32(&ctl.acc_full[b]));
                 }
             }
             q_total += nq;

@@ -1,21 +1,21 @@
-// Mixed-precision M2L (+ L2L) on the 5th-generation tensor cores: split 3xTF32.
+// Mixed-precision M2L on the 5th-generation tensor cores: products of split FP16 operands.
 //
 // Same contraction as the FP64 output-stationary GEMM (gemm_f64.cu; M2L of
-// phases.py:211-236 and L2L of phases.py:273-278 summed into one check
-// potential), with every product A*B evaluated as
-//     A_hi*B_hi + A_hi*B_lo + A_lo*B_hi,   x_hi = tf32(x), x_lo = tf32(x - x_hi)
-// by tcgen05.mma kind::tf32 into one FP32 accumulator in tensor memory.
+// phases.py:211-236), with every product A*B evaluated as
+//     A_hi*B_hi + A_hi*B_lo + A_lo*B_hi,   x_hi = fp16(s x), x_lo = fp16(s x - x_hi)
+// (s a power of two, mixed.cuh) by tcgen05.mma kind::f16 into one FP32 accumulator in tensor
+// memory; the FP64 sums are scaled back when they are stored.
 //
 // CTA = one tile of target boxes (same level and octant) x one 128-row block of
 // the n_s check points x one kernel family; accumulator 128 lanes x 128 columns
-// (targets x charge columns) FP32 in TMEM. Per k-chunk of 32 (128-byte rows):
+// (targets x charge columns) FP32 in TMEM. Per k-chunk of 64 (128-byte rows):
 //   * warp 4 (one lane) loads A_hi and A_lo with TMA (3-D tensor maps over the
 //     level's tables, SWIZZLE_128B, K-major) -> mbarrier complete_tx;
 //   * warps 0-3 gather the B columns (source boxes' equivalent densities) with
 //     16-byte cp.async into the same SWIZZLE_128B K-major layout; each thread's
 //     cp.async.mbarrier.arrive counts on the stage's mbarrier once its copies land
 //     (the MMA warp fences the generic->async proxy after its wait);
-//   * warp 5 (one lane) issues 4 k-steps x 3 tcgen05.mma and commits the stage
+//   * warp 5 (one lane) issues up to 4 k-steps x 3 tcgen05.mma and commits the stage
 //     back to its "empty" mbarrier;
 // three stages in flight.
 // Grid mode (a complete level with complex charges, the uniform workloads): the
@@ -26,13 +26,13 @@
 // gather warps idle, and the stage's only barrier is the TMA transaction count.
 // Accumulation precision: the error of an FP32 accumulator grows with the
 // length of its chain of MMAs (measured: about linearly), and the damped decode
-// amplifies it. So every FOLD k-chunks (24 MMAs) accumulate into a fresh FP32
+// amplifies it. So every one or two k-chunks (c.fold2; 12 or 24 MMAs) accumulate into a fresh FP32
 // buffer in TMEM (four buffers in turn, 4 x 128 columns = all 512), and the fold
 // warps (16: four per TMEM lane quadrant, each taking 32 of the 128 columns) add each
 // finished buffer into FP64 running sums held in their own registers, 32 doubles a
 // thread, while the tensor core fills the next buffers. The FP64 sums are stored as
-// the check potentials. (Folding every 4 k-chunks instead was 22 % faster but
-// doubled the M2L error: 8.3e-7 against 4.6e-7 for the potential at p = 8.)
+// the check potentials. (With TF32 operands, folding every 48 MMAs instead of every 24 was
+// 22 % faster but doubled the M2L error: 8.3e-7 against 4.6e-7 for the potential at p = 8.)
 // Registers: the block launches with 768 threads; setmaxnreg moves registers from
 // the gather and control warpgroups (warps 0-7) to the four fold warpgroups (8-23),
 // and the host checks that the split fits the launch's register file before the
@@ -52,6 +52,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <mutex>
 
 namespace hfmm {
@@ -61,7 +62,7 @@ namespace {
 using namespace mxk;
 
 template <int R>
-__global__ void __launch_bounds__(THREADS, 1) k_m2l_tf32x3(const __grid_constant__ MixedMaps maps,
+__global__ void __launch_bounds__(THREADS, 1) k_m2l_split(const __grid_constant__ MixedMaps maps,
                                                             MixedCall c) {
     constexpr int TT = BN / R;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -71,7 +72,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_tf32x3(const __grid_constant
     const int tile = blockIdx.x, m0 = blockIdx.y * BM, fam = blockIdx.z;
     volatile int* abort_flag = &ctl.abort_flag;
     const uint64_t wait_ns = c.wait_ns ? c.wait_ns : WAIT_NS;
-    const bool half = (c.m_valid > 0 ? c.m_valid : c.ldm) - m0 <= 64;
+    const bool half = c.valid - m0 <= 64;
     const uint32_t idesc = half ? IDESC64 : IDESC;
 
     if (tid < TT) {   // targets share the sources' box range (a level's own buffers)
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_tf32x3(const __grid_constant
     }
     for (int e = tid; e < M2L_ENTRIES; e += THREADS) {
         ctl.used[e] = 0;
-        ctl.ztab[e] = (short)(e < N_DISP ? c.disp_compact[e] : (c.has_l2l ? e - N_DISP : -1));
+        ctl.ztab[e] = (short)(e < N_DISP ? c.disp_compact[e] : -1);
     }
     if (tid == 0) {
         ctl.abort_flag = 0;
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_tf32x3(const __grid_constant
     }
     __syncthreads();
     const int n_act = ctl.n_act;
-    const int kch = c.ldk / BK;
+    const int kch = (c.valid + BK - 1) / BK;
     const int nq = n_act * kch;
     const uint32_t tmem = ctl.tmem;
     const int64_t fs = (int64_t)fam * c.fam_stride;
@@ -165,12 +166,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_tf32x3(const __grid_constant
     if (warp < 4) {
         if (!c.grid) {   // (grid mode: B comes by TMA, warp 4)
             // ---------------- B gathers (cp.async, manual SWIZZLE_128B placement)
-            const float* Bh = c.Bhi + fs;
-            const float* Bl = c.Blo + fs;
+            const uint16_t* B = c.B + fs;
             // Each thread always serves chunk ch of the same CPR rows (columns) of the B
             // tile: rows n_i = tid / CPR + (128 / CPR) i. Their swizzled shared-memory
-            // offsets are fixed (the 16-byte chunk index XORs with the row's bits: all three
-            // for 128-byte rows, the upper two for 64-byte rows, as TMA and the MMA read them);
+            // offsets are fixed (the 16-byte chunk index XORs with the row's low three bits, as
+            // TMA and the MMA read them);
             // their global sources change only when the displacement entry changes.
             constexpr int RSTEP = 128 / CPR;
             const int ch = tid % CPR;
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_tf32x3(const __grid_constant
     #pragma unroll
             for (int i = 0; i < CPR; ++i) {
                 const int n = tid / CPR + RSTEP * i;
-                const int sw = BK == 32 ? (n & 7) : ((n & 7) >> 1);
+                const int sw = n & 7;
                 soff[i] = (uint32_t)((n >> 3) * 8 * ROW_BYTES + (n & 7) * ROW_BYTES + ((ch ^ sw) << 4));
                 goff[i] = -1;
             }
@@ -211,20 +211,20 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_tf32x3(const __grid_constant
                             atomicOr(c.err, ERRF_BOUNDS);
                             s_ = -1;
                         }
-                        goff[i] = s_ >= 0 ? ((int64_t)s_ * R + (n % R)) * c.ldk + ch * 4 : -1;
+                        goff[i] = s_ >= 0 ? ((int64_t)s_ * R + (n % R)) * c.ldk + ch * 8 : -1;
                     }
                     if (ai + 1 < n_act) load_sources(ai + 1);
                 }
                 if (!mbar_wait(smem_u32(&ctl.empty[st]), ((q / STAGES) & 1) ^ 1, abort_flag, wait_ns)) break;
                 const int k0 = (q % kch) * BK;
-                const uint32_t sbh = smem_u32(sm + st * STAGE_BYTES + 2 * TILE_BYTES);
-                const uint32_t sbl = sbh + TILE_BYTES;
+                const uint32_t sb = smem_u32(sm + st * STAGE_BYTES + PLANES * TILE_BYTES);
     #pragma unroll
                 for (int i = 0; i < CPR; ++i) {
-                    const bool ok = goff[i] >= 0;
+                    const bool ok = goff[i] >= 0 && k0 + ch * 8 < c.ldk;
                     const int64_t o = ok ? goff[i] + k0 : 0;
-                    cp_async16(sbh + soff[i], Bh + o, ok);
-                    cp_async16(sbl + soff[i], Bl + o, ok);
+    #pragma unroll
+                    for (int pl = 0; pl < PLANES; ++pl)
+                        cp_async16(sb + pl * TILE_BYTES + soff[i], B + pl * c.b_plane + o, ok);
                 }
                 // the stage's barrier counts this thread's arrival when its copies have
                 // landed: no thread waits for its own copies, so every stage can be in flight
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_tf32x3(const __grid_constant
 #pragma unroll
         for (int j = 0; j < COLS_PER_FOLD_WARP; ++j) sum[j] = 0.0;
         bool ok = true;
-        const int n_units = (nq + FOLD - 1) / FOLD;
+        const int n_units = (nq + (1 << c.fold2) - 1) >> c.fold2;
         for (int i = 0; i < n_units; ++i) {
             const int b = i & (NACC - 1);
             // the TMEM loads below are warp-collective: agree on the wait's outcome
@@ -279,22 +279,17 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_tf32x3(const __grid_constant
         if (aborted) {
             if (lane == 0) atomicOr(c.err, ERRF_TIMEOUT);
         } else if (row_ok) {
+            const double unscale = 1.0 / (c.a_scale[fam] * plane_scale(*c.b_max[fam]));
 #pragma unroll
             for (int j = 0; j < COLS_PER_FOLD_WARP; ++j) {
                 const int n = c_lo + j;
                 const int t = ctl.tgt[n / R];
-                if (t >= 0) out[((int64_t)t * R + (n % R)) * c.ldm + m] = sum[j];
+                if (t >= 0) out[((int64_t)t * R + (n % R)) * c.ldm + m] = sum[j] * unscale;
             }
         }
     } else if (warp == 4) {
         // ---------------- A tiles by TMA
         if (lane == 0) {
-            const CUtensorMap* mh = &maps.a_hi[fam];
-            const CUtensorMap* ml = &maps.a_lo[fam];
-            const CUtensorMap* lh = &maps.l_hi[fam];
-            const CUtensorMap* ll = &maps.l_lo[fam];
-            const CUtensorMap* bh = &maps.b_hi[fam];
-            const CUtensorMap* bl = &maps.b_lo[fam];
             int ox = 0, oy = 0, oz = 0;   // grid mode: the tile's grid origin
             if (c.grid) {
                 ox = c.tile_org[3 * (int64_t)tile];
@@ -313,18 +308,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_tf32x3(const __grid_constant
                 const int k0 = (q % kch) * BK;
                 const uint32_t fb = smem_u32(&ctl.tfull[st]);
                 const uint32_t sa = smem_u32(sm + st * STAGE_BYTES);
-                mbar_arrive_tx(fb, (c.grid ? 4 : 2) * TILE_BYTES);
-                if (e < N_DISP) {
-                    tma_load_3d(sa, mh, k0, m0, z, fb);
-                    tma_load_3d(sa + TILE_BYTES, ml, k0, m0, z, fb);
-                } else {
-                    tma_load_3d(sa, lh, k0, m0, z, fb);
-                    tma_load_3d(sa + TILE_BYTES, ll, k0, m0, z, fb);
-                }
+                mbar_arrive_tx(fb, (c.grid ? 2 : 1) * PLANES * TILE_BYTES);
+#pragma unroll
+                for (int pl = 0; pl < PLANES; ++pl)
+                    tma_load_3d(sa + pl * TILE_BYTES, &maps.a[fam][pl], k0, m0, z, fb);
                 if (c.grid) {   // sources at target - d, d = (e / 49 - 3, (e / 7) % 7 - 3, e % 7 - 3)
                     const int sx = ox - (e / 49 - 3), sy = oy - ((e / 7) % 7 - 3), sz = oz - (e % 7 - 3);
-                    tma_load_5d(sa + 2 * TILE_BYTES, bh, k0, 0, sz, sy, sx, fb);
-                    tma_load_5d(sa + 3 * TILE_BYTES, bl, k0, 0, sz, sy, sx, fb);
+#pragma unroll
+                    for (int pl = 0; pl < PLANES; ++pl)
+                        tma_load_5d(sa + (PLANES + pl) * TILE_BYTES, &maps.b[fam][pl], k0, 0, sz, sy, sx, fb);
                 }
 #pragma unroll
                 for (int j = 0; j < STAGES; ++j)
@@ -345,7 +337,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_tf32x3(const __grid_constant
             bool ok = true, issued = false;
             for (int q = 0; q < nq && ok; ++q) {
                 const int st = q % STAGES;
-                const int unit = q / FOLD, uq = q % FOLD;
+                const int unit = q >> c.fold2, uq = q & ((1 << c.fold2) - 1);
                 const int b = unit & (NACC - 1);
                 if (uq == 0 && unit >= NACC) {   // buffer b must have been folded (unit - NACC)
                     if (!mbar_wait(smem_u32(&ctl.acc_empty[b]), ((unit / NACC) & 1) ^ 1, abort_flag, wait_ns)) {
@@ -363,21 +355,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_tf32x3(const __grid_constant
                 // before the tensor core's (async proxy) reads of the stage
                 if (!c.grid) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 asm volatile("tcgen05.fence::after_thread_sync;");
-                const uint32_t base = smem_u32(sm + st * STAGE_BYTES);
-                const uint64_t ah = sw_desc(base), al = sw_desc(base + TILE_BYTES);
-                const uint64_t bh = sw_desc(base + 2 * TILE_BYTES),
-                               bl = sw_desc(base + 3 * TILE_BYTES);
-                const uint32_t dt = tmem + b * BN;
-#pragma unroll
-                for (int ks = 0; ks < BK / 8; ++ks) {   // 8 tf32 = 32 bytes per k-step
-                    const uint64_t d = (uint64_t)(ks * 2);
-                    umma_tf32(dt, ah + d, bh + d, idesc, (uq > 0 || ks > 0) ? 1u : 0u);
-                    umma_tf32(dt, ah + d, bl + d, idesc, 1u);
-                    umma_tf32(dt, al + d, bh + d, idesc, 1u);
-                }
+                const int k0 = (q % kch) * BK;
+                stage_mmas(tmem + b * BN, smem_u32(sm + st * STAGE_BYTES),
+                           (min(BK, c.valid - k0) + KSTEP - 1) / KSTEP, idesc, uq == 0);
                 issued = true;
                 umma_commit(smem_u32(&ctl.empty[st]));
-                if (uq == FOLD - 1 || q == nq - 1) umma_commit(smem_u32(&ctl.acc_full[b]));
+                if (uq == (1 << c.fold2) - 1 || q == nq - 1) umma_commit(smem_u32(&ctl.acc_full[b]));
             }
             // drain, on every exit path: the commit tracks every MMA this thread issued
             if (issued) {
@@ -395,47 +378,53 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_tf32x3(const __grid_constant
     }
 }
 
-// Round an FP32 value to TF32 (10 explicit mantissa bits, ties away from zero) and
-// clear the 13 low bits, so the container holds exactly the value the tensor core
-// multiplies, however it treats the low bits.
-__device__ __forceinline__ float tf32_exact(float x) {
-    return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
+__global__ void k_absmax(const double* __restrict__ src, int64_t n, unsigned long long* most) {
+    unsigned long long m = 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const unsigned long long v = (unsigned long long)__double_as_longlong(src[i]) & ~(1ull << 63);
+        m = v > m ? v : m;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
+        m = v > m ? v : m;
+    }
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(most, m);
 }
 
-// x -> (hi, lo) with hi = tf32(x), lo = tf32(x - hi), both exact TF32 in FP32 containers
-__device__ __forceinline__ void split2(double x, float& hi, float& lo) {
-    hi = tf32_exact((float)x);
-    lo = tf32_exact((float)(x - (double)hi));
-}
-
-__global__ void k_split_tf32(const double* __restrict__ src, float* hi, float* lo, int64_t n) {
+__global__ void k_split_planes(const double* __restrict__ src, const unsigned long long* __restrict__ most,
+                               uint16_t* out, int64_t plane, int64_t n) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    float h, l;
-    split2(src[i], h, l);
-    hi[i] = h;
-    lo[i] = l;
+    uint16_t p[2];
+    split2(src[i] * plane_scale(*most), p);
+    out[i] = p[0];
+    out[plane + i] = p[1];
 }
 
-// densities [box][2][ckld] of a complete level -> TF32 halves at the box's grid position
-__global__ void k_split_tf32_grid(const double* __restrict__ src, const uint64_t* __restrict__ m_id,
-                                  int64_t n, int G, int ckld, float* hi, float* lo) {
+// densities [box][2][ckld] of a complete level -> planes at the box's grid position; two
+// values a thread (ckld is even), so that a warp stores whole 128-byte lines
+__global__ void k_split_planes_grid(const double2* __restrict__ src, const unsigned long long* __restrict__ most,
+                                    const uint64_t* __restrict__ m_id, int64_t n, int G, int ckld, uint32_t* out) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int64_t row = 2 * (int64_t)ckld;
-    const int64_t b = i / row, within = i % row;
+    const int64_t b = i / ckld, within = i % ckld;   // pairs per box: 2 ckld / 2
     int64_t x, y, z;
     demorton3(m_id[b], x, y, z);
     if (x >= G || y >= G || z >= G) return;
-    const int64_t o = ((x * G + y) * G + z) * row + within;
-    float h, l;
-    split2(src[i], h, l);
-    hi[o] = h;
-    lo[o] = l;
+    const int64_t o = ((x * G + y) * G + z) * ckld + within, plane = (int64_t)G * G * G * ckld;
+    const double2 v = src[i];
+    const double s = plane_scale(*most);
+    uint16_t p[2], q[2];
+    split2(v.x * s, p);
+    split2(v.y * s, q);
+    out[o] = p[0] | (uint32_t)q[0] << 16;
+    out[plane + o] = p[1] | (uint32_t)q[1] << 16;
 }
 
-// FP64 A^T tables ([k][m], ld x ld) -> TF32 hi/lo A tables ([m][k]), count matrices
-__global__ void k_split_transpose(const double* __restrict__ at, float* hi, float* lo, int ld) {
+// FP64 A^T tables ([k][m], ld x ld) -> A planes ([m][k]), count matrices
+__global__ void k_split_transpose(const double* __restrict__ at, double scale, uint16_t* out, int64_t plane,
+                                  int ld) {
     __shared__ double tile[32][33];
     const int c = blockIdx.z;
     const int bk = blockIdx.x * 32, bm = blockIdx.y * 32;
@@ -448,11 +437,11 @@ __global__ void k_split_transpose(const double* __restrict__ at, float* hi, floa
     for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
         int m = bm + yy, k = bk + threadIdx.x;
         if (m < ld && k < ld) {
-            float h, l;
-            split2(tile[threadIdx.x][yy], h, l);
-            int64_t o = (int64_t)c * ld * ld + (int64_t)m * ld + k;
-            hi[o] = h;
-            lo[o] = l;
+            uint16_t p[2];
+            split2(tile[threadIdx.x][yy] * scale, p);
+            const int64_t o = (int64_t)c * ld * ld + (int64_t)m * ld + k;
+            out[o] = p[0];
+            out[plane + o] = p[1];
         }
     }
 }
@@ -474,56 +463,69 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 }  // namespace
 
-void make_table_map(CUtensorMap* map, const float* base, int ld, int count, int ldm) {
-    // [count][ldm][ld] fp32 (ldm = 0: square), boxes of BK k x 128 m
+void make_table_maps(CUtensorMap (&map)[2], const uint16_t* base, size_t plane, int valid, int ld, int count,
+                     int ldm) {
+    // [count][ldm][ld] FP16 (ldm = 0: square), boxes of BK k x 128 m; the extents stop at the
+    // rows and columns that can be nonzero, so what a box covers past them is zero fill
     if (!ldm) ldm = ld;
-    if (((uintptr_t)base & 15) || (ld * 4) % 16 || ld < BK || ldm < BM)
-        throw Error{HFMM_ERR_STATE, "tensor map: table not 16-byte aligned or smaller than a box"};
-    cuuint64_t dims[3] = {(cuuint64_t)ld, (cuuint64_t)ldm, (cuuint64_t)count};
-    cuuint64_t strides[2] = {(cuuint64_t)ld * 4, (cuuint64_t)ld * ldm * 4};
-    cuuint32_t box[3] = {BK, BM, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void*)base, dims, strides,
-                             box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             BK == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) throw Error{HFMM_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r)};
+    if (((uintptr_t)base & 15) || plane * 2 % 16 || (ld * 2) % 16 || valid < 1 || valid > ld || valid > ldm)
+        throw Error{HFMM_ERR_STATE, "tensor map: table not 16-byte aligned or smaller than its rank"};
+    for (int p = 0; p < PLANES; ++p) {
+        cuuint64_t dims[3] = {(cuuint64_t)valid, (cuuint64_t)valid, (cuuint64_t)count};
+        cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)ld * ldm * 2};
+        cuuint32_t box[3] = {BK, BM, 1};
+        cuuint32_t estr[3] = {1, 1, 1};
+        CUresult r = encode_fn()(&map[p], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (void*)(base + p * plane), dims,
+                                 strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS)
+            throw Error{HFMM_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r)};
+    }
 }
 
-void make_grid_map(CUtensorMap* map, const float* base, int ckld, int G) {
-    // dense grid [x][y][z][2][ckld] fp32: dims (k, r, z, y, x); a box is one k-chunk of both
+void make_grid_maps(CUtensorMap (&map)[2], const uint16_t* base, int valid, int ckld, int G) {
+    // dense grid [x][y][z][2][ckld] FP16: dims (k, r, z, y, x); a box is one k-chunk of both
     // charge columns of 4 x 4 x 4 boxes two grid steps apart (element strides 2: a box of
     // 8 elements loads 4 of them), 128 rows of ROW_BYTES in the tile layout of the A maps
-    if (((uintptr_t)base & 15) || (ckld * 4) % 16 || ckld < BK || G < 1)
-        throw Error{HFMM_ERR_STATE, "grid map: grid not 16-byte aligned or smaller than a box"};
-    cuuint64_t dims[5] = {(cuuint64_t)ckld, 2, (cuuint64_t)G, (cuuint64_t)G, (cuuint64_t)G};
-    cuuint64_t strides[4] = {(cuuint64_t)ckld * 4, (cuuint64_t)ckld * 8, (cuuint64_t)G * ckld * 8,
-                             (cuuint64_t)G * G * ckld * 8};
-    cuuint32_t box[5] = {BK, 2, 8, 8, 8};
-    cuuint32_t estr[5] = {1, 1, 2, 2, 2};
-    CUresult r = encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, (void*)base, dims, strides,
-                             box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             BK == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS)
-        throw Error{HFMM_ERR_CUDA, "cuTensorMapEncodeTiled (grid) failed: " + std::to_string((int)r)};
+    if (((uintptr_t)base & 15) || (ckld * 2) % 16 || valid < 1 || valid > ckld || G < 1)
+        throw Error{HFMM_ERR_STATE, "grid map: grid not 16-byte aligned or smaller than its rank"};
+    const size_t plane = (size_t)G * G * G * 2 * ckld;
+    for (int p = 0; p < PLANES; ++p) {
+        cuuint64_t dims[5] = {(cuuint64_t)valid, 2, (cuuint64_t)G, (cuuint64_t)G, (cuuint64_t)G};
+        cuuint64_t strides[4] = {(cuuint64_t)ckld * 2, (cuuint64_t)ckld * 4, (cuuint64_t)G * ckld * 4,
+                                 (cuuint64_t)G * G * ckld * 4};
+        cuuint32_t box[5] = {BK, 2, 8, 8, 8};
+        cuuint32_t estr[5] = {1, 1, 2, 2, 2};
+        CUresult r = encode_fn()(&map[p], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, (void*)(base + p * plane), dims,
+                                 strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS)
+            throw Error{HFMM_ERR_CUDA, "cuTensorMapEncodeTiled (grid) failed: " + std::to_string((int)r)};
+    }
 }
 
-void split_tf32_grid(const double* src, const uint64_t* m_id, int64_t n_boxes, int G, int ckld,
-                     float* hi, float* lo, cudaStream_t s) {
-    const int64_t n = n_boxes * 2 * ckld;
+void absmax(const double* src, int64_t n, unsigned long long* most, cudaStream_t s) {
     if (n <= 0) return;
-    HFMM_LAUNCH(k_split_tf32_grid, (unsigned)ceil_div(n, 256), 256, 0, s, src, m_id, n, G, ckld, hi, lo);
+    HFMM_LAUNCH(k_absmax, (unsigned)std::min<int64_t>(ceil_div(n, 1024), 8 * sm_count()), 256, 0, s, src, n, most);
 }
 
-void split_tf32(const double* src, float* hi, float* lo, int64_t n, cudaStream_t s) {
+void split_planes_grid(const double* src, const unsigned long long* most, const uint64_t* m_id, int64_t n_boxes,
+                       int G, int ckld, uint16_t* out, cudaStream_t s) {
+    const int64_t n = n_boxes * ckld;   // pairs
     if (n <= 0) return;
-    HFMM_LAUNCH(k_split_tf32, (unsigned)ceil_div(n, 256), 256, 0, s, src, hi, lo, n);
+    HFMM_LAUNCH(k_split_planes_grid, (unsigned)ceil_div(n, 256), 256, 0, s, reinterpret_cast<const double2*>(src),
+                most, m_id, n, G, ckld, reinterpret_cast<uint32_t*>(out));
 }
 
-void split_transpose_tables(const double* at, float* hi, float* lo, int ld, int count) {
+void split_planes(const double* src, const unsigned long long* most, uint16_t* out, int64_t plane, int64_t n,
+                  cudaStream_t s) {
+    if (n <= 0) return;
+    HFMM_LAUNCH(k_split_planes, (unsigned)ceil_div(n, 256), 256, 0, s, src, most, out, plane, n);
+}
+
+void split_transpose_tables(const double* at, double scale, uint16_t* out, int ld, int count) {
     dim3 grid((unsigned)ceil_div(ld, 32), (unsigned)ceil_div(ld, 32), (unsigned)count);
-    HFMM_LAUNCH(k_split_transpose, grid, dim3(32, 8), 0, 0, at, hi, lo, ld);
+    HFMM_LAUNCH(k_split_transpose, grid, dim3(32, 8), 0, 0, at, scale, out, (int64_t)count * ld * ld, ld);
 }
 
 // setmaxnreg.inc draws on the registers the block was launched with: the split of the
@@ -537,40 +539,40 @@ void check_register_split() {
         int fits = 1;
         for (int r = 0; r < 2; ++r) {
             cudaFuncAttributes a{};
-            HFMM_CUDA(cudaFuncGetAttributes(&a, r ? (const void*)k_m2l_tf32x3<2> : (const void*)k_m2l_tf32x3<1>));
+            HFMM_CUDA(cudaFuncGetAttributes(&a, r ? (const void*)k_m2l_split<2> : (const void*)k_m2l_split<1>));
             const long need = 128L * REG_GATHER + 128L * REG_CTRL + 32L * N_FOLD_WARPS * REG_FOLD;
             if ((long)a.numRegs * THREADS < need || a.maxThreadsPerBlock < THREADS) fits = 0;
         }
         verdict = fits ? 1 : -1;
     }
     if (verdict < 0)
-        throw Error{HFMM_ERR_STATE, "m2l_tf32x3: the warp roles' register split exceeds the launch's registers"};
+        throw Error{HFMM_ERR_STATE, "m2l_split: the warp roles' register split exceeds the launch's registers"};
 }
 
 std::atomic<uint64_t> g_m2l_wait_ns{0};
 std::atomic<int> g_m2l_grid{1};
 std::atomic<int> g_m2l_starve{0};
 
-size_t m2l_tf32x3_smem() { return (size_t)STAGES * STAGE_BYTES + sizeof(Ctl) + 1024; }
+size_t m2l_split_smem() { return (size_t)STAGES * STAGE_BYTES + sizeof(Ctl) + 1024; }
 
-void m2l_tf32x3(const MixedMaps& maps, const MixedCall& call, cudaStream_t s) {
+void m2l_split(const MixedMaps& maps, const MixedCall& call, cudaStream_t s) {
     if (call.ntiles == 0) return;
     MixedCall c = call;
     c.wait_ns = g_m2l_wait_ns.load();
     c.starve = g_m2l_starve.load();
     if (!c.ldk) c.ldk = c.ld;
     if (!c.ldm) c.ldm = c.ld;
-    if (c.ldk % BK || c.ldm % BK)
-        throw Error{HFMM_ERR_STATE, "m2l_tf32x3: ld must be a multiple of 32"};
-    const size_t smem = m2l_tf32x3_smem();
+    if (c.ldk % 32 || c.ldm % 32 || c.valid < 1 || c.valid > c.ldk || c.valid > c.ldm)
+        throw Error{HFMM_ERR_STATE, "m2l_split: ld must be a multiple of 32 that holds the rank"};
+    const size_t smem = m2l_split_smem();
     dim3 grid(c.ntiles, (c.ldm + BM - 1) / BM, c.n_fam);
     check_register_split();
     if (c.R == 1) {
-        HFMM_CUDA(cudaFuncSetAttribute(k_m2l_tf32x3<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        HFMM_LAUNCH(k_m2l_tf32x3<1>, grid, THREADS, smem, s, maps, c);
+        HFMM_CUDA(cudaFuncSetAttribute(k_m2l_split<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        HFMM_LAUNCH(k_m2l_split<1>, grid, THREADS, smem, s, maps, c);
     } else {
-        HFMM_CUDA(cudaFuncSetAttribute(k_m2l_tf32x3<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        HFMM_LAUNCH(k_m2l_tf32x3<2>, grid, THREADS, smem, s, maps, c);
+        HFMM_CUDA(cudaFuncSetAttribute(k_m2l_split<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        HFMM_LAUNCH(k_m2l_split<2>, grid, THREADS, smem, s, maps, c);
     }
 }
 

@@ -1,21 +1,22 @@
-// Mixed-precision (3xTF32 on tcgen05) M2L: shared declarations.
+// Mixed-precision (two FP16 planes on tcgen05) M2L: shared declarations.
 #pragma once
 #include "hfmm_internal.cuh"
 
 #include <cuda.h>
+#include <cuda_fp16.h>
 
 #include <atomic>
+#include <cstring>
 
 #include <string>
 #include <vector>
 
 namespace hfmm {
 
-// TMA descriptors of one level's TF32 hi/lo tables, per kernel family:
-// M2L (316 non-adjacent displacements) and L2L (8 octants), each [z][m][k] fp32.
+// TMA descriptors of the planes of one level's M2L tables (316 non-adjacent displacements,
+// [z][m][k] FP16), per kernel family, and in grid mode of its dense density grid (5-D).
 struct MixedMaps {
-    CUtensorMap a_hi[2], a_lo[2], l_hi[2], l_lo[2];
-    CUtensorMap b_hi[2], b_lo[2];   // grid mode: the level's dense density grid (5-D)
+    CUtensorMap a[2][2], b[2][2];
 };
 
 struct MixedCall {
@@ -23,20 +24,21 @@ struct MixedCall {
     int ntiles;
     const int32_t* src_tab;        // nb x 351 source boxes (-1 = none)
     const int32_t* disp_compact;   // 343: displacement -> M2L table index (-1 = adjacent)
-    const float* Bhi;              // equivalent densities, split, [fam][box][R][ld]
-    const float* Blo;
-    const float* Lhi;              // parent local densities, split (L2L entries)
-    const float* Llo;
+    const uint16_t* B;             // equivalent densities' planes, [plane][fam][box][R][ld] FP16
+    int64_t b_plane;               // elements between planes
+    const unsigned long long* b_max[2];   // per family: bits of the densities' largest magnitude
+    double a_scale[2];             // per family: the scale of A's planes
     double* out;                   // check potentials [fam][box][R][ld], FP64
-    int R, ld, n_fam, has_l2l;
+    int R, ld, n_fam;
     int ldk, ldm;                  // rectangular tables: K extent (B rows) and M extent (out
                                    // rows); 0 = ld. A tables are [count][ldm][ldk]
-    int m_valid;                   // rows of A that can be nonzero (0 = ldm): a row block
-                                   // with at most 64 of them runs the M = 64 MMA shape
+    int fold2;                     // log2 of the k-chunks per FP32 accumulation unit (0: 12 MMAs, 1: 24)
+    int valid;                     // rows and columns of A that can be nonzero: K stops there,
+                                   // and a row block with at most 64 runs the M = 64 MMA shape
     int64_t fam_stride, out_fam_stride, nb;
     int64_t src_lo, src_hi;        // valid source boxes [src_lo, src_hi) (0, nb when unset)
     int* err;
-    uint64_t wait_ns;              // limit of each bounded wait (0: 2 s); set by m2l_tf32x3
+    uint64_t wait_ns;              // limit of each bounded wait (0: 2 s); set by m2l_split
     int starve;                    // test only: leave stage 0 without its gather arrivals
     // grid mode (complete level, R = 2): B comes from the dense density grid by TMA, one
     // strided 4 x 4 x 4 box per displacement; tile_tgt then holds grid tiles and
@@ -51,17 +53,50 @@ struct MixedCall {
 extern std::atomic<uint64_t> g_m2l_wait_ns;
 extern std::atomic<int> g_m2l_starve;
 
-void make_table_map(CUtensorMap* map, const float* base, int ld, int count, int ldm = 0);
-void split_tf32(const double* src, float* hi, float* lo, int64_t n, cudaStream_t s);
-// a complete level's densities [box][2][ckld] (boxes in level order from m_id) -> TF32
-// halves in the dense grid [x][y][z][2][ckld] of side G
-void split_tf32_grid(const double* src, const uint64_t* m_id, int64_t n_boxes, int G, int ckld,
-                     float* hi, float* lo, cudaStream_t s);
-void make_grid_map(CUtensorMap* map, const float* base, int ckld, int G);
+// The two FP16 planes of a scaled value: hi its rounding, lo the rounding of the rest (exact in
+// FP64). The scale, a power of two, puts the largest magnitude of an operand in [2^13, 2^14):
+// a value down to 2^-16 of that keeps the full 22 bits, a smaller one is off by at most 2^-25
+// in scaled units, 2^-38 of the largest.
+__device__ __forceinline__ void split2(double x, uint16_t (&p)[2]) {
+    const __half h = __float2half_rn((float)x);
+    p[0] = __half_as_ushort(h);
+    p[1] = __half_as_ushort(__float2half_rn((float)(x - (double)__half2float(h))));
+}
+
+// That scale from the largest magnitude's bits; 1 where there is none (zero, infinite, NaN or
+// outside the range whose scale is a normal number).
+__host__ __device__ __forceinline__ double plane_scale(unsigned long long most) {
+    const int e = (int)(most >> 52);   // biased exponent: 2^(e - 1023) <= magnitude
+    if (e < 30 || e > 2000) return 1.0;
+    const unsigned long long bits = (unsigned long long)(2046 + 13 - e) << 52;   // 2^(13 - (e - 1023))
+    double s;
+#ifdef __CUDA_ARCH__
+    s = __longlong_as_double((long long)bits);
+#else
+    memcpy(&s, &bits, sizeof(s));
+#endif
+    return s;
+}
+
+// Maps of the two planes of tables [count][ldm][ld] (ldm 0: ld), `plane` apart, and of a grid
+// [plane][x][y][z][2][ckld]: rows and K values from `valid` on are zeros, which the loads
+// then fill in instead of reading
+void make_table_maps(CUtensorMap (&map)[2], const uint16_t* base, size_t plane, int valid, int ld, int count,
+                     int ldm = 0);
+void make_grid_maps(CUtensorMap (&map)[2], const uint16_t* base, int valid, int ckld, int G);
+// n FP64 values, the largest magnitude's bits at `most` -> their FP16 planes, `plane` elements
+// apart; absmax raises *most to the largest magnitude of src
+void split_planes(const double* src, const unsigned long long* most, uint16_t* out, int64_t plane, int64_t n,
+                  cudaStream_t s);
+void absmax(const double* src, int64_t n, unsigned long long* most, cudaStream_t s);
+// a complete level's densities [box][2][ckld] (boxes in level order from m_id) -> planes of
+// the dense grid [x][y][z][2][ckld] of side G
+void split_planes_grid(const double* src, const unsigned long long* most, const uint64_t* m_id, int64_t n_boxes,
+                       int G, int ckld, uint16_t* out, cudaStream_t s);
 // process-wide: 1 (default) lets complete levels use grid mode, 0 forces the gather
 extern std::atomic<int> g_m2l_grid;
-void split_transpose_tables(const double* at, float* hi, float* lo, int ld, int count);
-void m2l_tf32x3(const MixedMaps& maps, const MixedCall& c, cudaStream_t s);
+void split_transpose_tables(const double* at, double scale, uint16_t* out, int ld, int count);
+void m2l_split(const MixedMaps& maps, const MixedCall& c, cudaStream_t s);
 
 // the low-rank mixed M2L call of one plan, level and family for R charge columns
 MixedCall cx_call(hfmm_plan* P, int l, int f, int R);
@@ -78,7 +113,7 @@ void m2l_queue(const MixedCall* calls, const MixedMaps* maps, const M2LItem* ite
                int* next, int R, int n_ctas, cudaStream_t s, int starve = 0);
 // The work list of a queued M2L over the plans given: every (plan, level, family)
 // low-rank call with its tensor maps, one item per tile and 128-row block, largest
-// first (cost: k-chunks per entry, 0.6 for a block of at most 64 live rows). Returns
+// first (cost: K values per entry, 0.6 for a block of at most 64 live rows). Returns
 // "" when it applies, else why not (32-bit gather offsets would overflow).
 std::string queue_items(hfmm_plan* const* plans, int n_plans, int R, std::vector<MixedCall>& calls,
                         std::vector<MixedMaps>& maps, std::vector<M2LItem>& items);
@@ -93,6 +128,6 @@ struct PlanQueue {
 void plan_queue_build(hfmm_plan* P);     // both charge-column counts
 void plan_queue_release(hfmm_plan* P);
 size_t m2l_queue_smem();
-size_t m2l_tf32x3_smem();
+size_t m2l_split_smem();
 
 }  // namespace hfmm

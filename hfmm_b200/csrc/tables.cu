@@ -14,6 +14,10 @@
 // (their minimum separation is >= 1.9 s), so it is not evaluated. The result is
 // written straight into the GEMM layout (A^T, k-major, ld x ld, zero padded).
 #include "hfmm_internal.cuh"
+#include "mixed.cuh"
+
+#include <algorithm>
+#include <cmath>
 
 namespace hfmm {
 
@@ -96,16 +100,13 @@ __global__ void k_gen(int kind, const double* __restrict__ eq, const double* __r
     *o = (fam == 1 ? sn : cs) / r;
 }
 
-__device__ __forceinline__ float tf32_round(float x) {
-    return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
-}
 
 // Streamed M2L tables of one level, both kernel families from one sincos per
-// entry. layout 0: FP64 A^T [fam][c][k][m] (the FP64 GEMM); layout 1: TF32 hi/lo
-// halves as A [fam][c][m][k] (the tcgen05 path), hi at ws, lo after the hi block.
+// entry. layout 0: FP64 A^T [fam][c][k][m] (the FP64 GEMM); layout 1: FP16
+// planes of the scaled values as A [plane][fam][c][m][k] (the tcgen05 path).
 // The fastest thread index runs along the contiguous axis of the layout.
 __global__ void k_gen_m2l_stream(const double* __restrict__ eq, int n_s, int ld, double s, double kw,
-                                 int n_fam, int yukawa, int layout, void* ws) {
+                                 int n_fam, int yukawa, int layout, double scale0, double scale1, void* ws) {
     const int c = blockIdx.z;
     const int a = blockIdx.x * blockDim.x + threadIdx.x;   // contiguous axis
     const int b = blockIdx.y * blockDim.y + threadIdx.y;
@@ -137,12 +138,11 @@ __global__ void k_gen_m2l_stream(const double* __restrict__ eq, int n_s, int ld,
         double* o = static_cast<double*>(ws);
         for (int f = 0; f < n_fam; ++f) o[f * fam_stride + idx] = v[f];
     } else {
-        float* hi = static_cast<float*>(ws);
-        float* lo = hi + n_fam * fam_stride;
+        uint16_t* o = static_cast<uint16_t*>(ws);
         for (int f = 0; f < n_fam; ++f) {
-            const float h = tf32_round((float)v[f]);
-            hi[f * fam_stride + idx] = h;
-            lo[f * fam_stride + idx] = tf32_round((float)(v[f] - (double)h));
+            uint16_t p[2];
+            split2(v[f] * (f ? scale1 : scale0), p);
+            for (int i = 0; i < 2; ++i) o[(size_t)(i * n_fam + f) * fam_stride + idx] = p[i];
         }
     }
 }
@@ -153,12 +153,25 @@ size_t stream_ws_bytes(const hfmm_plan* P) {
     return (size_t)P->n_fam * 316 * (size_t)P->ld * P->ld * sizeof(double);
 }
 
+// Scale of a level's M2L planes, from the largest entry there can be: the kernel at the least
+// distance of the surfaces of two boxes of the V list, 1.9 half-sides (|sin(kr)| / r: k at most).
+double m2l_scale(const hfmm_plan* P, int fam, int level) {
+    const double r = 1.9 * P->extent * std::ldexp(1.0, -(level + 1));
+    double most = 1.0 / r;
+    if (P->yukawa) most *= std::exp(-P->k * r) / (4.0 * M_PI);
+    else if (fam == 1) most = std::min(most, std::fabs(P->k));
+    unsigned long long bits;
+    std::memcpy(&bits, &most, sizeof(bits));
+    return plane_scale(bits);
+}
+
 void generate_m2l_stream(hfmm_plan* P, int level, bool mixed, void* ws, cudaStream_t st) {
     const double s = P->extent * std::ldexp(1.0, -(level + 1));
     dim3 blk(32, 8);
     dim3 grid((unsigned)ceil_div(P->ld, 32), (unsigned)ceil_div(P->ld, 8), 316u);
     HFMM_LAUNCH(k_gen_m2l_stream, grid, blk, 0, st, P->equiv_pts.p, P->n_s, P->ld, s, P->k,
-                P->n_fam, P->yukawa ? 1 : 0, mixed ? 1 : 0, ws);
+                P->n_fam, P->yukawa ? 1 : 0, mixed ? 1 : 0, m2l_scale(P, 0, level),
+                m2l_scale(P, 1, level), ws);
 }
 
 void generate_m2l(hfmm_plan* P, int fam, int level, DevBuf<double>& out) {
