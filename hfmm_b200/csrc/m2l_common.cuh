@@ -124,18 +124,27 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem, uint64_t a, uint64_t b, 
         " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
         "l"(a), "l"(b), "r"(idesc), "r"(acc));
 }
-// One stage's MMAs: k-steps of the three plane products into the accumulator at dt, which the
-// first one overwrites when `first`. base: the stage's A planes, then its B planes.
-__device__ __forceinline__ void stage_mmas(uint32_t dt, uint32_t base, int ksteps, uint32_t idesc, bool first) {
-    const uint64_t ah = sw_desc(base), al = sw_desc(base + TILE_BYTES);
-    const uint64_t bh = sw_desc(base + 2 * TILE_BYTES), bl = sw_desc(base + 3 * TILE_BYTES);
-    for (int ks = 0; ks < ksteps; ++ks) {   // 16 values = 32 bytes per k-step
-        const uint64_t d = (uint64_t)(ks * 2);
-        umma_f16(dt, ah + d, bh + d, idesc, ks > 0 || !first ? 1u : 0u);
-        umma_f16(dt, ah + d, bl + d, idesc, 1u);
-        umma_f16(dt, al + d, bh + d, idesc, 1u);
+// One stage's MMAs: KS k-steps of the three plane products into the accumulator at dt, which
+// the first one overwrites when `first`. desc: the descriptor of the stage's first A plane (its
+// second and the B planes follow, TILE_BYTES apart).
+template <int KS>
+__device__ __forceinline__ void stage_mmas(uint32_t dt, uint64_t desc, uint32_t idesc, bool first) {
+    constexpr uint64_t T = TILE_BYTES >> 4;
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {   // 16 values = 32 bytes per k-step
+        const uint64_t d = desc + (uint64_t)(ks * 2);
+        umma_f16(dt, d, d + 2 * T, idesc, ks > 0 || !first ? 1u : 0u);
+        umma_f16(dt, d, d + 3 * T, idesc, 1u);
+        umma_f16(dt, d + T, d + 2 * T, idesc, 1u);
     }
 }
+__device__ __forceinline__ void stage_mmas(uint32_t dt, uint64_t desc, int ks, uint32_t idesc, bool first) {
+    if (ks >= 4) stage_mmas<4>(dt, desc, idesc, first);
+    else if (ks == 3) stage_mmas<3>(dt, desc, idesc, first);
+    else if (ks == 2) stage_mmas<2>(dt, desc, idesc, first);
+    else stage_mmas<1>(dt, desc, idesc, first);
+}
+static_assert(BK / KSTEP == 4, "stage_mmas");
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");

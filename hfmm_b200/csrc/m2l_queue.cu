@@ -170,60 +170,79 @@ __global__ void __launch_bounds__(THREADS, 1)
     // stages and accumulation units this CTA has issued before the current item.
     int q_total = 0, u_total = 0;
     if (warp < 4) {
-        // ---------------- B gathers (k_m2l_split's, for items that are not in grid mode)
+        // ---------------- B gathers (k_m2l_split's, for items that are not in grid mode). The
+        // next entry's sources are looked up while the current one's chunks are copied.
+        constexpr int RSTEP = 128 / CPR;
+        const int ch = tid % CPR;
+        const uint32_t soff0 = (uint32_t)((tid / CPR >> 3) * 8 * ROW_BYTES + (tid / CPR & 7) * ROW_BYTES +
+                                          ((ch ^ (tid / CPR & 7)) << 4));   // rows RSTEP apart: the same swizzle
+        static_assert(RSTEP % 8 == 0, "gather rows");
+        int st = 0;
+        uint32_t phase = 1;
         while (next_item<R, false>(ctl, calls, items, n_items, next, warp, lane, tid)) {
             const MixedCall& c = ctl.c;
-            const int kch = (c.valid + BK - 1) / BK, nq = ctl.n_act * kch;
+            const int kch = (c.valid + BK - 1) / BK, n_act = ctl.n_act, nq = n_act * kch;
             if (!c.grid) {
-                constexpr int RSTEP = 128 / CPR;
-                const int ch = tid % CPR;
-                uint32_t soff[CPR];
-                int goff[CPR];   // element offsets: the host keeps nb x R x ldk below 2^31
-#pragma unroll
-                for (int i = 0; i < CPR; ++i) {
-                    const int n = tid / CPR + RSTEP * i;
-                    const int sw = n & 7;
-                    soff[i] = (uint32_t)((n >> 3) * 8 * ROW_BYTES + (n & 7) * ROW_BYTES + ((ch ^ sw) << 4));
-                    goff[i] = -1;
-                }
-                const int64_t src_lo = c.src_hi > 0 ? c.src_lo : 0;
-                const int64_t src_hi = c.src_hi > 0 ? c.src_hi : c.nb;
-                int cur_entry = -1;
-                for (int q = 0; q < nq; ++q) {
-                    const int qg = q_total + q, st = qg % STAGES;
-                    const int ai = q / kch;
-                    if (ai != cur_entry) {
-                        cur_entry = ai;
-                        const int e = ctl.act[ai];
-#pragma unroll
-                        for (int i = 0; i < CPR; ++i) {
-                            const int n = tid / CPR + RSTEP * i;
-                            const int t = ctl.tgt[n / R];
-                            int s_ = t >= 0 ? c.src_tab[(int64_t)t * M2L_ENTRIES + e] : -1;
-                            if (s_ >= 0 && (s_ < src_lo || s_ >= src_hi)) {
-                                atomicOr(c.err, ERRF_BOUNDS);
-                                s_ = -1;
-                            }
-                            goff[i] = s_ >= 0 ? (s_ * R + (n % R)) * c.ldk + ch * 8 : -1;
-                        }
-                    }
-                    if (!mbar_wait(smem_u32(&ctl.empty[st]), ((qg / STAGES) & 1) ^ 1, abort_flag, wait_ns)) break;
-                    const int k0 = (q % kch) * BK;
-                    const uint32_t sb = smem_u32(sm + st * STAGE_BYTES + PLANES * TILE_BYTES);
+                const int src_lo = c.src_hi > 0 ? (int)c.src_lo : 0, src_hi = (int)(c.src_hi > 0 ? c.src_hi : c.nb);
+                const int ldk = c.ldk;
+                const int32_t* src_tab = c.src_tab;
+                const uint16_t* B = c.B + ch * 8;
+                const int64_t b_plane = c.b_plane;
+                int nsrc[CPR];
+                auto look_up = [&](int ai) {
+                    const int e = ctl.act[ai];
 #pragma unroll
                     for (int i = 0; i < CPR; ++i) {
-                        const bool ok = goff[i] >= 0 && k0 + ch * 8 < c.ldk;
-                        const int64_t o = ok ? goff[i] + k0 : 0;
-#pragma unroll
-                        for (int pl = 0; pl < PLANES; ++pl)
-                            cp_async16(sb + pl * TILE_BYTES + soff[i], c.B + pl * c.b_plane + o, ok);
+                        const int t = ctl.tgt[(tid / CPR + RSTEP * i) / R];
+                        nsrc[i] = t >= 0 ? __ldg(src_tab + (int64_t)t * M2L_ENTRIES + e) : -1;
                     }
-                    if (!(starve && qg == 0))   // (test: the CTA's first stage never fills)
-                        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(
-                                         smem_u32(&ctl.full[st]))
-                                     : "memory");
+                };
+                if (n_act > 0) look_up(0);
+                bool ok = true;
+                int qg = q_total;
+                for (int ai = 0; ai < n_act && ok; ++ai) {
+                    int goff[CPR];   // element offsets: the host keeps nb x R x ldk below 2^31
+#pragma unroll
+                    for (int i = 0; i < CPR; ++i) {
+                        int s_ = nsrc[i];
+                        if (s_ >= 0 && (s_ < src_lo || s_ >= src_hi)) {
+                            atomicOr(c.err, ERRF_BOUNDS);
+                            s_ = -1;
+                        }
+                        goff[i] = s_ >= 0 ? (s_ * R + (tid / CPR + RSTEP * i) % R) * ldk : -1;
+                    }
+                    if (ai + 1 < n_act) look_up(ai + 1);
+                    for (int kc = 0; kc < kch; ++kc, ++qg) {
+                        const int k0 = kc * BK;
+                        if (!mbar_wait(smem_u32(&ctl.empty[st]), phase, abort_flag, wait_ns)) {
+                            ok = false;
+                            break;
+                        }
+                        const uint32_t sb = smem_u32(sm) + st * STAGE_BYTES + PLANES * TILE_BYTES + soff0;
+                        const bool in = k0 + ch * 8 < ldk;
+#pragma unroll
+                        for (int i = 0; i < CPR; ++i) {
+                            const bool okk = goff[i] >= 0 && in;
+                            const uint16_t* g = okk ? B + goff[i] + k0 : c.B;
+#pragma unroll
+                            for (int pl = 0; pl < PLANES; ++pl)
+                                cp_async16(sb + pl * TILE_BYTES + i * (RSTEP * ROW_BYTES), g + (okk ? pl * b_plane : 0), okk);
+                        }
+                        if (!(starve && qg == 0))   // (test: the CTA's first stage never fills)
+                            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(
+                                             smem_u32(&ctl.full[st]))
+                                         : "memory");
+                        if (++st == STAGES) {
+                            st = 0;
+                            phase ^= 1;
+                        }
+                    }
                 }
                 asm volatile("cp.async.wait_all;\n" ::: "memory");
+            } else {   // the stages of a grid item pass by
+                const int at = st + nq;
+                phase ^= (uint32_t)(at / STAGES) & 1u;
+                st = at % STAGES;
             }
             q_total += nq;
             __syncthreads();
@@ -281,14 +300,18 @@ __global__ void __launch_bounds__(THREADS, 1)
             __syncthreads();
         }
     } else if (warp == 4) {
-        // ---------------- A (and, in grid mode, B) tiles by TMA
+        // ---------------- A (and, in grid mode, B) tiles by TMA. One thread issues every stage's
+        // copies, so what it computes a stage is on the pipeline's path: coordinates change
+        // with the entry only, stage and phase are carried along.
         int last_q[STAGES];   // the last stage index loaded into each stage
 #pragma unroll
         for (int st = 0; st < STAGES; ++st) last_q[st] = -1;
         int* err = nullptr;
+        int st = 0;
+        uint32_t phase = 1;   // of empty[st]: the first round finds every stage free
         while (next_item<R, false>(ctl, calls, items, n_items, next, warp, lane, tid)) {
             const MixedCall& c = ctl.c;
-            const int kch = (c.valid + BK - 1) / BK, nq = ctl.n_act * kch;
+            const int kch = (c.valid + BK - 1) / BK, n_act = ctl.n_act, nq = n_act * kch;
             if (lane == 0) {
                 err = c.err;
                 const int tile = items[ctl.item].tile, m0 = items[ctl.item].mblock * BM;
@@ -299,38 +322,49 @@ __global__ void __launch_bounds__(THREADS, 1)
                 for (int pl = 0; pl < PLANES; ++pl)
                     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&mp->a[0][pl])
                                  : "memory");
+                const bool grid = c.grid;
                 int ox = 0, oy = 0, oz = 0;
-                if (c.grid) {
+                if (grid) {
 #pragma unroll
                     for (int pl = 0; pl < PLANES; ++pl)
                         asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&mp->b[0][pl])
                                      : "memory");
-                    ox = c.tile_org[3 * (int64_t)tile];
-                    oy = c.tile_org[3 * (int64_t)tile + 1];
-                    oz = c.tile_org[3 * (int64_t)tile + 2];
+                    ox = c.tile_org[3 * (int64_t)tile] + 3;
+                    oy = c.tile_org[3 * (int64_t)tile + 1] + 3;
+                    oz = c.tile_org[3 * (int64_t)tile + 2] + 3;
                 }
-                for (int q = 0; q < nq; ++q) {
-                    const int qg = q_total + q, st = qg % STAGES;
-                    if (!mbar_wait(smem_u32(&ctl.empty[st]), ((qg / STAGES) & 1) ^ 1, abort_flag, wait_ns)) break;
-                    if (c.grid && starve && qg == 0) continue;   // (test: stage 0 never fills)
-                    const int e = ctl.act[q / kch];
-                    const int z = ctl.zidx[q / kch];
-                    const int k0 = (q % kch) * BK;
-                    const uint32_t fb = smem_u32(&ctl.tfull[st]);
-                    const uint32_t sa = smem_u32(sm + st * STAGE_BYTES);
-                    mbar_arrive_tx(fb, (c.grid ? 2 : 1) * PLANES * TILE_BYTES);
+                const uint32_t bytes = (grid ? 2 : 1) * PLANES * TILE_BYTES;
+                int qg = q_total;
+                bool ok = true;
+                for (int ai = 0; ai < n_act && ok; ++ai) {
+                    const int e = ctl.act[ai], z = ctl.zidx[ai];
+                    const int sx = ox - e / 49, sy = oy - (e / 7) % 7, sz = oz - e % 7;   // sources at target - d
+                    for (int k0 = 0; k0 < kch * BK; k0 += BK, ++qg) {
+                        const uint32_t fb = smem_u32(&ctl.tfull[st]);
+                        const uint32_t sa = smem_u32(sm) + st * STAGE_BYTES;
+                        if (!mbar_wait(smem_u32(&ctl.empty[st]), phase, abort_flag, wait_ns)) {
+                            ok = false;
+                            break;
+                        }
+                        if (!(grid && starve && qg == 0)) {   // (test: stage 0 never fills)
+                            mbar_arrive_tx(fb, bytes);
 #pragma unroll
-                    for (int pl = 0; pl < PLANES; ++pl)
-                        tma_load_3d(sa + pl * TILE_BYTES, &mp->a[0][pl], k0, m0, z, fb);
-                    if (c.grid) {
-                        const int sx = ox - (e / 49 - 3), sy = oy - ((e / 7) % 7 - 3), sz = oz - (e % 7 - 3);
+                            for (int pl = 0; pl < PLANES; ++pl)
+                                tma_load_3d(sa + pl * TILE_BYTES, &mp->a[0][pl], k0, m0, z, fb);
+                            if (grid) {
 #pragma unroll
-                        for (int pl = 0; pl < PLANES; ++pl)
-                            tma_load_5d(sa + (PLANES + pl) * TILE_BYTES, &mp->b[0][pl], k0, 0, sz, sy, sx, fb);
+                                for (int pl = 0; pl < PLANES; ++pl)
+                                    tma_load_5d(sa + (PLANES + pl) * TILE_BYTES, &mp->b[0][pl], k0, 0, sz, sy, sx, fb);
+                            }
+#pragma unroll
+                            for (int j = 0; j < STAGES; ++j)
+                                if (j == st) last_q[j] = qg;
+                        }
+                        if (++st == STAGES) {
+                            st = 0;
+                            phase ^= 1;
+                        }
                     }
-#pragma unroll
-                    for (int j = 0; j < STAGES; ++j)
-                        if (j == st) last_q[j] = qg;
                 }
             }
             q_total += nq;
@@ -344,13 +378,15 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (!drained && err) atomicOr(err, ERRF_TIMEOUT);
         }
     } else if (warp == 5) {
-        // ---------------- MMA issue
+        // ---------------- MMA issue (one thread; stage, phase and buffer are carried along)
         bool issued = false;
         int* err = nullptr;
         // The gather warps complete a stage's full barrier only for items that are not in
         // grid mode, so its phase is not the stage counter's: bit st holds the parity of
         // full[st]'s next phase.
-        uint32_t full_par = 0;
+        uint32_t full_par = 0, phase = 0;
+        int st = 0;
+        const uint64_t desc0 = sw_desc(smem_u32(sm));
         while (next_item<R, false>(ctl, calls, items, n_items, next, warp, lane, tid)) {
             const MixedCall& c = ctl.c;
             const int kch = (c.valid + BK - 1) / BK, nq = ctl.n_act * kch;
@@ -358,34 +394,44 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (lane == 0) {
                 err = c.err;
                 const int m0 = items[ctl.item].mblock * BM;
-                const bool half = c.valid - m0 <= 64;
-                const uint32_t idesc = half ? IDESC64 : IDESC;
-                const int fold2 = c.fold2, last = (1 << fold2) - 1, valid = c.valid;
-                const bool gridded = c.grid;
-                int kc = 0;   // k-chunk within the entry
+                const uint32_t idesc = c.valid - m0 <= 64 ? IDESC64 : IDESC;
+                const int last = (1 << c.fold2) - 1;
+                // k-steps of an entry's last chunk
+                const int tail = (c.valid - (kch - 1) * BK + KSTEP - 1) / KSTEP;
+                const bool grid = c.grid;
+                int ug = u_total, uq = 0, kc = 0;
                 for (int q = 0; q < nq; ++q) {
-                    const int qg = q_total + q, st = qg % STAGES;
-                    const int u = q >> fold2, uq = q & last;
-                    const int ug = u_total + u, b = ug & (NACC - 1);
+                    const int b = ug & (NACC - 1);
                     if (uq == 0 && ug >= NACC) {
                         if (!mbar_wait(smem_u32(&ctl.acc_empty[b]), ((ug / NACC) & 1) ^ 1, abort_flag, wait_ns))
                             break;
                         asm volatile("tcgen05.fence::after_thread_sync;");
                     }
-                    if (!gridded) {
+                    if (!grid) {
                         if (!mbar_wait(smem_u32(&ctl.full[st]), (full_par >> st) & 1u, abort_flag, wait_ns))
                             break;
                         full_par ^= 1u << st;
                     }
-                    if (!mbar_wait(smem_u32(&ctl.tfull[st]), (qg / STAGES) & 1, abort_flag, wait_ns)) break;
-                    if (!gridded) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    if (!mbar_wait(smem_u32(&ctl.tfull[st]), phase, abort_flag, wait_ns)) break;
+                    if (!grid) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     asm volatile("tcgen05.fence::after_thread_sync;");
-                    stage_mmas(tmem + b * BN, smem_u32(sm + st * STAGE_BYTES),
-                               (min(BK, valid - kc * BK) + KSTEP - 1) / KSTEP, idesc, uq == 0);
-                    kc = kc + 1 == kch ? 0 : kc + 1;
+                    const uint64_t d = desc0 + (uint64_t)(st * (STAGE_BYTES >> 4));
+                    ++kc;
+                    stage_mmas(tmem + b * BN, d, kc < kch ? BK / KSTEP : tail, idesc, uq == 0);
+                    if (kc == kch) kc = 0;
                     issued = true;
                     umma_commit(smem_u32(&ctl.empty[st]));
                     if (uq == last || q == nq - 1) umma_commit(smem_u32(&ctl.acc_full[b]));
+                    if (uq == last) {
+                        uq = 0;
+                        ++ug;
+                    } else {
+                        ++uq;
+                    }
+                    if (++st == STAGES) {
+                        st = 0;
+                        phase ^= 1;
+                    }
                 }
             }
             q_total += nq;

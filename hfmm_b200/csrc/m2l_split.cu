@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_split(const __grid_constant_
                 if (!c.grid) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 asm volatile("tcgen05.fence::after_thread_sync;");
                 const int k0 = (q % kch) * BK;
-                stage_mmas(tmem + b * BN, smem_u32(sm + st * STAGE_BYTES),
+                stage_mmas(tmem + b * BN, sw_desc(smem_u32(sm + st * STAGE_BYTES)),
                            (min(BK, c.valid - k0) + KSTEP - 1) / KSTEP, idesc, uq == 0);
                 issued = true;
                 umma_commit(smem_u32(&ctl.empty[st]));
