@@ -727,10 +727,12 @@ void conv_m2l(hfmm_plan* P, int R, int64_t fam_stride, cudaStream_t s) {
     if (rows < 1) throw Error{HFMM_ERR_STATE, "convolution M2L: workspace too small"};
     const int dz = std::max(planes, 1);
     const int PT = 256;
-    // children per CTA of the transforms: as many as leave two CTAs an SM, four at least (half
-    // the 128-byte lines) while those fit at all
+    // children per CTA of the transforms: eight where four CTAs an SM remain (the latency of
+    // their short stages is the rest of the time), else four (half the 128-byte lines) while
+    // those fit at all. 1e6 points, p = 8, forward / inverse: 3.45 / 4.78 ms with eight,
+    // 3.33 / 3.99 with four, 5.8 with two; p = 6 (36 KB with eight): 127 / 155 us and 142 / 173
     int CH = 8;
-    while (CH > 4 && transform_smem(c.p, c.n_s, R, CH, rows) > SMEM_MAX / 2) CH /= 2;
+    while (CH > 4 && transform_smem(c.p, c.n_s, R, CH, rows) > SMEM_MAX / 4) CH /= 2;
     while (CH > 1 && transform_smem(c.p, c.n_s, R, CH, rows) > SMEM_MAX) CH /= 2;
     // few slots: fewer children a CTA on the inverse (its kz sum stays in one CTA), segments of
     // kz on the forward, towards three CTAs an SM (72 slots, p = 8: 81 and 98 us with one)
