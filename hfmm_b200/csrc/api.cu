@@ -496,6 +496,7 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
         c.src_ld = src_ld;
         c.n_entries = k_entries[kind];
         c.b_split = kind == K_DN ? N_DISP : c.n_entries;
+        c.one_entry = kind == K_L2L || kind == K_L2LF;   // downward tiles are of one octant
         c.accumulate = accumulate >= 0 ? accumulate : (kind == K_L2L ? 1 : 0);
         c.A = P->a_ptrs.p + X->ix.off[kind][l];
         c.B0 = B0;

@@ -16,8 +16,8 @@
 // operand tiles stream into shared memory with 16-byte cp.async copies.
 //
 // Tensor path: mma.sync.m16n8k4 f64 (DMMA). tcgen05 has no f64 kind, so this
-// is the FP64 tensor path on sm_100a. CTA tile 64 (m) x 64 (n = targets x R),
-// k-chunk 16, 4 warps of 32 x 32, three-stage cp.async pipeline with one barrier a chunk.
+// is the FP64 tensor path on sm_100a. CTA tile 64 (m) x 64 (n = targets x R), or 32 x 32 on
+// small grids, k-chunk 16, 4 warps of 32 x 32 (16 x 16), three-stage cp.async pipeline with one barrier a chunk.
 // An SM sub-partition takes 32 cycles per DMMA, so a chunk's 32 a warp are 1,024 cycles; what
 // kept it from them were the instructions around (640 a chunk and warp: copy addresses and
 // source lookups worked out anew every chunk, eight 8-byte fragment loads a step). Now the
@@ -38,8 +38,8 @@ namespace hfmm {
 
 namespace {
 
-constexpr int TM = 64, TN = 64, KC = 16, STAGES = 3;
-constexpr int AP = TM + 2;   // As[k][AP]: two k rows apart is 32 bytes mod 128
+constexpr int TM = 64, TN = 64, KC = 16, STAGES = 3;   // the tile of large grids
+constexpr int TS = 32;                                  // and of small ones: 32 x 32
 constexpr int BP = KC + 8;   // Bs[n][BP]: one column apart is 64 bytes mod 128
 constexpr int MAX_ENTRIES = 352;
 constexpr int SRC_ENTRIES = 8;   // entry counts whose tile sources are kept in shared memory
@@ -61,11 +61,13 @@ __device__ __forceinline__ void dmma(double (&c)[4], double a0, double a1, doubl
         : "d"(a0), "d"(a1), "d"(b0));
 }
 
+template <int T>
 struct __align__(16) Smem {
+    static constexpr int AP = T + 2;   // A[k][AP]: two k rows apart is 32 bytes mod 128
     double A[STAGES][KC][AP];
-    double B[STAGES][TN][BP];
-    int src[TN][SRC_ENTRIES + 1];
-    int tgt[TN];
+    double B[STAGES][T][BP];
+    int src[T][SRC_ENTRIES + 1];
+    int tgt[T];
     short act[MAX_ENTRIES];
     unsigned char used[MAX_ENTRIES];   // entry has a source for some target of the tile
     int n_act;
@@ -87,14 +89,17 @@ __device__ __forceinline__ void store_pair(const GemmCall& c, double* out, const
     *o = make_double2(v0, v1);
 }
 
-template <int R>
+// T: the square tile, 64 or 32 (four warps of T / 2 squared). A tile list has 64 columns a
+// tile; with T = 32 two CTAs share one.
+template <int R, int T>
 __global__ void __launch_bounds__(128, 3) k_gemm_f64(GemmCall c, int* err) {
-    constexpr int TT = TN / R;
+    constexpr int TT = T / R, AP = Smem<T>::AP, MI = T / 32, NI = T / 16;
+    constexpr int ACH = T / 2, CPT = KC * ACH / 128;   // 16-byte copies: of an A row; of each operand a thread
     extern __shared__ __align__(16) char smem_raw[];
-    Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
+    Smem<T>& sm = *reinterpret_cast<Smem<T>*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int S = c.n_split > 1 ? c.n_split : 1;
-    const int tile = blockIdx.x, m0 = blockIdx.y * TM, fam = blockIdx.z / S, split = blockIdx.z % S;
+    const int tile = blockIdx.x, m0 = blockIdx.y * T, fam = blockIdx.z / S, split = blockIdx.z % S;
     const int e_lo = (int)((int64_t)split * c.n_entries / S);
     const int e_hi = (int)((int64_t)(split + 1) * c.n_entries / S);
     const double* const* A = c.A + (int64_t)fam * c.a_fam_stride;
@@ -163,17 +168,18 @@ __global__ void __launch_bounds__(128, 3) k_gemm_f64(GemmCall c, int* err) {
     // the next chunk to copy: its entry, its k, and this thread's source addresses there
     int l_e = 0, l_k = 0;
     const double* ap = nullptr;
-    const double* bp[4];
+    const double* bp[CPT];
     unsigned bok = 0;
-    const bool aok = m0 + (tid & 31) * 2 < c.ldm;
+    const int a_row = tid / ACH, a_col = tid % ACH * 2;   // rows 128 / ACH apart
+    const bool aok = m0 + a_col < c.ldm;
     auto load = [&](int buf) {
         if (l_k == 0) {   // a new entry
             const int e = sm.act[l_e++];
-            ap = A[e] + (int64_t)(tid >> 5) * c.ldm + (aok ? m0 + (tid & 31) * 2 : 0);
+            ap = A[e] + (int64_t)a_row * c.ldm + (aok ? m0 + a_col : 0);
             const double* Bsel = (e >= c.b_split && B1) ? B1 : B0;
             bok = 0;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {   // B: 64 columns x 16 doubles, 8 threads a column
+            for (int i = 0; i < CPT; ++i) {   // B: T columns x 16 doubles, 8 threads a column
                 const int col = (tid >> 3) + 16 * i, j = col / R, r = col % R;
                 const int t = sm.tgt[j];
                 int s = -1;
@@ -185,30 +191,30 @@ __global__ void __launch_bounds__(128, 3) k_gemm_f64(GemmCall c, int* err) {
             }
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)   // A: 16 rows x 64 doubles, a warp a row
-            cp_async16(&sm.A[buf][(tid >> 5) + 4 * i][(tid & 31) * 2], ap + (int64_t)(4 * i) * c.ldm, aok);
+        for (int i = 0; i < CPT; ++i)   // A: 16 rows x T doubles
+            cp_async16(&sm.A[buf][a_row + 128 / ACH * i][a_col], ap + (int64_t)(128 / ACH * i) * c.ldm, aok);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < CPT; ++i)
             cp_async16(&sm.B[buf][(tid >> 3) + 16 * i][(tid & 7) * 2], bp[i], bok >> i & 1);
         ap += (int64_t)KC * c.ldm;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < CPT; ++i)
             if (bok >> i & 1) bp[i] += KC;
         l_k = l_k + 1 == kch ? 0 : l_k + 1;
     };
 
-    double acc[2][4][4];
+    double acc[MI][NI][4];
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+    for (int a = 0; a < MI; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b)
+        for (int b = 0; b < NI; ++b)
 #pragma unroll
             for (int d = 0; d < 4; ++d) acc[a][b][d] = 0.0;
 
-    const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
+    const int wm = (warp & 1) * (T / 2), wn = (warp >> 1) * (T / 2);
     const int g = lane >> 2, t4 = lane & 3;
     // 16-row halves of the warp's tile with rows that can be nonzero
-    const int m_rows = min(2, max(0, ((c.ldm == c.ld ? c.n_s : c.ldm) - (m0 + wm) + 15) / 16));
+    const int m_rows = min(MI, max(0, ((c.ldm == c.ld ? c.n_s : c.ldm) - (m0 + wm) + 15) / 16));
 #pragma unroll
     for (int i = 0; i < STAGES - 1; ++i) {
         if (i < nq) load(i);
@@ -228,18 +234,18 @@ __global__ void __launch_bounds__(128, 3) k_gemm_f64(GemmCall c, int* err) {
 #pragma unroll
             for (int kk = 0; kk < KC; kk += 8) {
                 if (kk >= k8n) break;
-                double2 b[4];
+                double2 b[NI];
 #pragma unroll
-                for (int ni = 0; ni < 4; ++ni) b[ni] = *reinterpret_cast<const double2*>(Bs + ni * 8 * BP + kk);
+                for (int ni = 0; ni < NI; ++ni) b[ni] = *reinterpret_cast<const double2*>(Bs + ni * 8 * BP + kk);
 #pragma unroll
-                for (int mi = 0; mi < 2; ++mi) {
+                for (int mi = 0; mi < MI; ++mi) {
                     if (mi >= m_rows) break;
                     const double2 a0 = *reinterpret_cast<const double2*>(As + kk * AP + mi * 16);
                     const double2 a1 = *reinterpret_cast<const double2*>(As + (kk + 1) * AP + mi * 16);
 #pragma unroll
-                    for (int ni = 0; ni < 4; ++ni) dmma(acc[mi][ni], a0.x, a0.y, b[ni].x);
+                    for (int ni = 0; ni < NI; ++ni) dmma(acc[mi][ni], a0.x, a0.y, b[ni].x);
 #pragma unroll
-                    for (int ni = 0; ni < 4; ++ni) dmma(acc[mi][ni], a1.x, a1.y, b[ni].y);
+                    for (int ni = 0; ni < NI; ++ni) dmma(acc[mi][ni], a1.x, a1.y, b[ni].y);
                 }
             }
         }
@@ -254,7 +260,7 @@ __global__ void __launch_bounds__(128, 3) k_gemm_f64(GemmCall c, int* err) {
         double top = 0.0;
         bool odd = false;   // infinities and NaN: the largest bits there are
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
+        for (int i = 0; i < MI * NI * 4; ++i) {
             const double v = fabs((&acc[0][0][0])[i]);
             odd = odd || !(v <= 1.7976931348623157e308);
             top = fmax(top, v);
@@ -268,9 +274,9 @@ __global__ void __launch_bounds__(128, 3) k_gemm_f64(GemmCall c, int* err) {
         if (lane == 0 && bits) atomicMax(c.most, bits);
     }
 #pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
+    for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
+        for (int ni = 0; ni < NI; ++ni)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int ml = wm + mi * 16 + 2 * g, col = wn + ni * 8 + 2 * t4 + h, m = m0 + ml;
@@ -344,22 +350,38 @@ void gemm_f64(const GemmCall& call, int* d_err, cudaStream_t s) {
     if (c.n_entries > MAX_ENTRIES) throw Error{HFMM_ERR_STATE, "gemm_f64: too many entries"};
     if (c.R != 1 && c.R != 2) throw Error{HFMM_ERR_ARG, "gemm_f64: R must be 1 or 2"};
     dim3 grid(c.ntiles, (c.ldm + TM - 1) / TM, c.n_fam);
-    // entry splits when the grid gives the SMs fewer than four CTAs each (a CTA of 128
-    // threads hides little latency on its own): up to about four per SM
     const int64_t ctas = (int64_t)grid.x * grid.y * grid.z;
     const int sms = sm_count();
-    int S = 1;
     if (c.most && (c.scale || c.accumulate || c.n_entries != 1))
         throw Error{HFMM_ERR_STATE, "gemm_f64: largest magnitude of a plain one-entry call only"};
-    if (c.part && c.n_entries > 1 && ctas < 4 * sms) {
+    // Under six CTAs an SM, calls of one entry a tile take 32 x 32 tiles: four times the CTAs,
+    // each with a quarter of the serial chain, five an SM instead of three. All GEMMs of
+    // 20,000 points p = 8 / p = 12: 351 / 848 us with 64 x 64 tiles only, 274 / 775 with the
+    // line at one CTA an SM, 259 / 767 at two, 253 / 711 at four and above (real 1e5 p = 6:
+    // 453, 381, 382, 352). On every size, operands read twice as often cost: 1e6 points
+    // 6.83 to 7.38 ms. Calls of several entries keep 64 x 64 and the split below (p = 12:
+    // 853 with small tiles there too against 767).
+    if ((c.n_entries == 1 || c.one_entry) && ctas < 6 * sms) {
+        c.n_split = 1;
+        grid.x *= 2;
+        grid.y = (c.ldm + TS - 1) / TS;
+        auto kern = c.R == 1 ? k_gemm_f64<1, TS> : k_gemm_f64<2, TS>;
+        HFMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<TS>)));
+        HFMM_LAUNCH(kern, grid, 128, sizeof(Smem<TS>), s, c, d_err);
+        return;
+    }
+    // entry splits when the grid gives the SMs fewer than four CTAs each (a CTA of 128
+    // threads hides little latency on its own): up to about four per SM
+    int S = 1;
+    if (c.part && c.n_entries > 1 && !c.one_entry && ctas < 4 * sms) {
         S = (int)std::min<int64_t>({(int64_t)c.n_entries, 16, (4 * sms + ctas - 1) / ctas});
         while (S > 1 && ctas * S * TN * TM > c.part_cap) --S;
     }
     c.n_split = S;
     grid.z *= S;
-    auto kern = c.R == 1 ? k_gemm_f64<1> : k_gemm_f64<2>;
-    HFMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
-    HFMM_LAUNCH(kern, grid, 128, sizeof(Smem), s, c, d_err);
+    auto kern = c.R == 1 ? k_gemm_f64<1, TM> : k_gemm_f64<2, TM>;
+    HFMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<TM>)));
+    HFMM_LAUNCH(kern, grid, 128, sizeof(Smem<TM>), s, c, d_err);
     if (S > 1) {
         grid.z = grid.z / S * (TN / RED_COLS);
         if (c.R == 1) HFMM_LAUNCH(k_gemm_reduce<1>, grid, 128, 0, s, c, d_err);

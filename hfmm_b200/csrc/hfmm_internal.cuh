@@ -327,6 +327,7 @@ struct GemmCall {
     const double* scale;       // nullable, length ld
     const double* scale_f1;    // family 1's scale when it differs (nullable: scale)
     int accumulate;            // 1: out += result, 0: out = result
+    int one_entry;             // 1: a tile has sources for one of its entries only (L2L by octant)
     int R;
     int ld;                    // padded n_s (multiple of 16)
     int ldk, ldm;              // rectangular calls: K extent / B row length and M extent /
