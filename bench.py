@@ -385,30 +385,25 @@ def measured_fp64_peak(torch):
     return best
 
 
-def measured_tf32_peak(torch):
-    """cuBLAS FP32 GEMM with TF32 tensor cores on this GPU (TFLOP/s): the roofline
-    of the 3xTF32 M2L, whose work is counted as three TF32 products."""
-    prev = torch.backends.cuda.matmul.allow_tf32
-    torch.backends.cuda.matmul.allow_tf32 = True
-    try:
-        n = 8192
-        a = torch.randn(n, n, dtype=torch.float32, device="cuda")
-        b = torch.randn(n, n, dtype=torch.float32, device="cuda")
-        for _ in range(3):
-            a @ b
-        torch.cuda.synchronize()
-        best = 0.0
-        for _ in range(5):
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record()
-            a @ b
-            e1.record()
-            e1.synchronize()
-            best = max(best, 2 * n ** 3 / (e0.elapsed_time(e1) * 1e-3) / 1e12)
-        del a, b
-        return best
-    finally:
-        torch.backends.cuda.matmul.allow_tf32 = prev
+def measured_fp16_peak(torch):
+    """cuBLAS FP16 GEMM on this GPU (TFLOP/s): the roofline of the mixed M2L, whose work is
+    counted as three FP16 products."""
+    n = 8192
+    a = torch.randn(n, n, dtype=torch.float16, device="cuda")
+    b = torch.randn(n, n, dtype=torch.float16, device="cuda")
+    for _ in range(3):
+        a @ b
+    torch.cuda.synchronize()
+    best = 0.0
+    for _ in range(5):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record()
+        a @ b
+        e1.record()
+        e1.synchronize()
+        best = max(best, 2 * n ** 3 / (e0.elapsed_time(e1) * 1e-3) / 1e12)
+    del a, b
+    return best
 
 
 def m2l_flops(state, R, NF):
@@ -427,13 +422,11 @@ def m2l_flops(state, R, NF):
 
 
 def dominant_flops(state, R, NF):
-    """Algorithmic FLOPs of the M2L+L2L GEMM phase per evaluate: each V pair and each
-    L2L child is one n_s x n_s matrix times R charge columns, per kernel family."""
-    info = state.info
-    lv = state.tree()["lvls"]
-    n_l2l = int((lv >= 3).sum())
-    n_s = info["n_s"]
-    return 2.0 * n_s * n_s * R * NF * (info["n_v"] + n_l2l)
+    """Algorithmic FLOPs of the FP64 M2L per evaluate: a convolution over the surface
+    lattice, so each V pair is one complex product per frequency of the (2p-1)^3 transform
+    (real charges: of half of them) and kernel family. The transforms are not counted."""
+    n = 2 * state.p - 1
+    return 8.0 * (n ** 3 if R == 2 else n * n * state.p) * NF * state.info["n_v"]
 
 
 def run_ours(a, cfg, rank, world, local_rank):
@@ -549,15 +542,14 @@ def run_ours(a, cfg, rank, world, local_rank):
         if a.precision == "fp64":
             flops = dominant_flops(st, R, NF)
             peak = measured_fp64_peak(torch)
-            kernel = "k_gemm_f64 (M2L + L2L, all levels)"
+            kernel = "k_conv_fwd, k_conv_mul, k_conv_inv (M2L, all levels)"
             src = ("cuBLAS DGEMM 4096^3 measured in this run, FP64 (of measured; "
                    "MEASURED_PEAKS.json has no FP64 figure)")
         else:
             flops = 3.0 * m2l_flops(st, R, NF)
-            peak = measured_tf32_peak(torch)
-            kernel = "k_m2l_tf32x3 (M2L, 3xTF32 on tcgen05, all levels)"
-            src = ("cuBLAS FP32 GEMM with TF32 tensor cores, 8192^3, measured in this run "
-                   "(of measured; MEASURED_PEAKS.json has no TF32 figure)")
+            peak = measured_fp16_peak(torch)
+            kernel = "k_m2l_split (M2L, two FP16 planes on tcgen05, all levels)"
+            src = "cuBLAS FP16 GEMM, 8192^3, measured in this run (of measured)"
         achieved = flops / (dom_ms * 1e-3) / 1e12 if dom_ms > 0 else None
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": (achieved / peak) if achieved else None,
@@ -575,7 +567,7 @@ def run_ours(a, cfg, rank, world, local_rank):
             "metric": METRIC, "value": world * n / (ms * 1e-3), "unit": "points/s",
             "n_gpus": world, "steps": a.steps, "warmup": a.warmup, "ms_per_step": ms,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "f64" if a.precision == "fp64" else "f32+tf32x3+f64",
+            "dtype": "f64" if a.precision == "fp64" else "f32+f16x3+f64",
             "data": "synthetic (seeded uniform points and N(0,1) complex charges)",
             "config": {"workload": cfg["workload"], "n_points": n, "k": cfg["k"], "p": cfg["p"],
                        "n_s": st.info["n_s"], "leaf": cfg["leaf"], "max_depth": st.max_depth,
@@ -780,27 +772,26 @@ def run_auto(a, cfg, rank, world, local_rank):
     out = None
     if rank == 0:
         dom_ms = float(phase[_lib.PHASES.index("m2l_l2l_gemm")])
-        peak = measured_tf32_peak(torch)
+        peak = measured_fp16_peak(torch)
         achieved = flops / (dom_ms * 1e-3) / 1e12 if dom_ms > 0 else None
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": (achieved / peak) if achieved else None, "traffic": _traffic(a, "auto"),
                 "traffic_unit": "bytes per evaluate (all M2L launches), from profiles/traffic.json",
                 "kernel": (("k_m2l_queue (the plan's low-rank M2L: every level and family in "
-                            "one persistent launch, 3xTF32 on tcgen05, on the C_d tables)")
+                            "one persistent launch, two FP16 planes on tcgen05, on the C_d tables)")
                            if ap_cmp and not a.per_level_m2l else
-                           ("k_m2l_tf32x3 (M2L, 3xTF32 on tcgen05, one launch per level and family"
+                           ("k_m2l_split (M2L, two FP16 planes on tcgen05, one launch per level and family"
                             + (", on the low-rank C_d tables)" if ap_cmp else ")"))),
                 "algorithmic_flops_per_evaluate": flops, "kernel_ms_per_evaluate": dom_ms,
-                "flop_count": ("3 TF32 products x 2 r^2 per V pair, charge column and family, "
+                "flop_count": ("3 FP16 products x 2 r^2 per V pair, charge column and family, "
                                "r = the rank of the pair's level and family (unpadded)"
                                if ap_cmp else
-                               "3 TF32 products x 2 n_s^2 per V pair, charge column and family"),
-                "peak_source": "cuBLAS FP32 GEMM with TF32 tensor cores, 8192^3, measured in "
-                               "this run (of measured; MEASURED_PEAKS.json has no TF32 figure)"}
-        half_bf16 = _half_bf16_peak()
-        if achieved and half_bf16:
-            roof["frac_of_half_bf16_burst"] = achieved / half_bf16
-            roof["half_bf16_burst_tflops"] = half_bf16
+                               "3 FP16 products x 2 n_s^2 per V pair, charge column and family"),
+                "peak_source": "cuBLAS FP16 GEMM, 8192^3, measured in this run (of measured)"}
+        bf16 = _bf16_peak()
+        if achieved and bf16:
+            roof["frac_of_bf16_burst"] = achieved / bf16
+            roof["bf16_burst_tflops"] = bf16
         cpu = None
         if not a.no_cpu and world == 1:
             cores, blas = cpu_threads()
@@ -817,7 +808,7 @@ def run_auto(a, cfg, rank, world, local_rank):
             "metric": cfg.get("metric", METRIC), "value": world * n / (ms * 1e-3), "unit": "points/s",
             "n_gpus": world, "steps": a.steps, "warmup": a.warmup, "ms_per_step": ms,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "f32+tf32x3+f64",
+            "dtype": "f32+f16x3+f64",
             "data": "synthetic (seeded points of the workload's distribution, N(0,1) complex charges)",
             "config": {"workload": f"{workload}, tol {a.tol:g}, learned p and leaf, "
                                    "mixed precision, certified on 256 targets, potential+field",
@@ -932,7 +923,7 @@ def run_batch(a, cfg, rank, world, local_rank):
             "metric": METRIC + " (batched C4)", "value": world * n_tot / (ms * 1e-3),
             "unit": "points/s", "n_gpus": world, "steps": a.steps, "warmup": a.warmup,
             "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "f32+tf32x3+f64",
+            "dtype": "f32+f16x3+f64",
             "data": "synthetic (seeded uniform points and N(0,1) complex charges)",
             "config": {"workload": cfg["workload"], "problems": len(probs), "points_total": n_tot,
                        "n_streams": ab.batch.n_streams, "queued_m2l": bool(ab.batch.queued),
@@ -961,11 +952,11 @@ def run_batch(a, cfg, rank, world, local_rank):
     return out
 
 
-def _half_bf16_peak():
-    """Half the dense bf16 burst rate of MEASURED_PEAKS.json (TF32 runs at half the
-    bf16 rate on the tensor cores), or None when the file is absent."""
+def _bf16_peak():
+    """The dense bf16 burst rate of MEASURED_PEAKS.json (FP16 runs at the same rate on the
+    tensor cores), or None when the file is absent."""
     try:
-        return float(json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["bf16_tflops"]) / 2
+        return float(json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["bf16_tflops"])
     except Exception:
         return None
 

@@ -17,8 +17,9 @@ constexpr int BN = 128;          // UMMA N (target columns per CTA)
 // each, and a product is hi hi + hi lo + lo hi: the 22 bits of two TF32 halves in half their
 // bytes, at twice the K per MMA. What bounds the kernel is the MMAs' reading of their operands
 // from shared memory (8 KB each, about 140 cycles), so half as many MMAs take half the time:
-// 5e5 points, p = 8, all levels and both families 8.46 ms with TF32 halves, 5.96 with these.
-// (Three BF16 planes, six products and 6 bytes a value, took 9.04: as many MMAs as TF32.)
+// 5e5 points, p = 8, all levels and both families 8.46 ms with TF32 halves, 5.50 with these
+// and 4.60 since the single threads' work a stage was cut. (Three BF16 planes, six products
+// and 6 bytes a value, took 9.04: as many MMAs as TF32.)
 constexpr int PLANES = 2;
 constexpr int BK = 64;                      // K values per k-chunk: 128-byte rows, SWIZZLE_128B
 constexpr int KSTEP = 16;                   // K values per MMA

@@ -9,8 +9,9 @@
 // Complex charges travel as one complex sequence (the kernel is real), real charges as the
 // half spectrum. Against the dense tables (2 n_s^2 a pair and column) that is 8 n^3 a pair
 // and column pair: 27 against 350 kFLOP at p = 8, 97 against 2,120 at p = 12. One
-// evaluate, complex charges, field (B200): 1e6 points, p = 8, depth 5: 210.2 -> 42.8 ms;
-// 20,000 points, depth 3: p = 8 6.69 -> 1.55 ms, p = 12 32.7 -> 3.68 ms.
+// evaluate, complex charges, field (B200): 1e6 points, p = 8, depth 5: 210.2 ms with the
+// tables, 31.8 now (products 13.4, transforms 3.3 and 4.0 of it); 20,000 points, depth 3:
+// p = 8 6.69 and 0.85 ms, p = 12 32.7 and 2.28 ms.
 //
 // Work is laid out by PARENT: the children of one parent ("slot") sit side by side, absent
 // ones as zeros, X as [frequency][slot][child]. The products of one frequency and one of

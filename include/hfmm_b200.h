@@ -41,8 +41,9 @@ extern "C" {
                                      kappa = 0 is Laplace, kernels/laplace/kernel.py:104  */
 
 #define HFMM_PREC_FP64 0      /* plain path: every phase in float64                  */
-#define HFMM_PREC_MIXED 1     /* M2L as split 3xTF32 on tcgen05 (FP32 accumulation in
-                                 short chains, folded into FP64), P2P in FP32 with an
+#define HFMM_PREC_MIXED 1     /* M2L on tcgen05 with FP16 hi/lo operand planes and
+                                 power-of-two scales (FP32 accumulation in short
+                                 chains, folded into FP64), P2P in FP32 with an
                                  FP64 phase reduction; decodes, M2M, L2L, P2M, L2P FP64.
                                  M2L needs p >= 5 (ld = n_s rounded up to 32 >= 128);
                                  smaller p runs its FP64 GEMM.                         */
@@ -134,7 +135,9 @@ int hfmm_plan_set_level_decode(hfmm_plan* plan, int32_t family, int32_t level,
  * of every level (11 GB per family at p = 12, depth 5), the plan regenerates a
  * level's matrices on the device right before that level's M2L, into a
  * workspace of hfmm_plan_workspace_bytes bytes, bit-identical to the resident
- * tables. Choose the mode after hfmm_plan_set_kernel and before the level tables
+ * tables. Where the FP64 M2L runs as a convolution, its spectra (343 (2p - 1)^2 p
+ * complex numbers a level and family) stay resident and the workspace holds the
+ * transforms, as many frequencies at a time as fit. Choose the mode after hfmm_plan_set_kernel and before the level tables
  * (which must then come without M2L_K: hfmm_plan_set_level_decode). Without a
  * bound workspace, the first hfmm_evaluate allocates the plan's own (so make
  * that call outside stream capture). hfmm_plan_bind_workspace
@@ -249,10 +252,10 @@ int hfmm_direct_noalloc(const double* pos_dev, const double* q_re_dev, const dou
  * stream. hfmm_plan_phase_times synchronises and writes the milliseconds spent
  * per phase, summed over every evaluate since profiling was enabled or the
  * previous read (up to 8192 phase instances): 0 charge gather, 1 P2M, 2 M2M GEMM, 3 upward decode,
- * 4 M2L (with L2L fused on the FP64 path), 5 X-list P2L, 6 downward decode,
- * 7 P2P, 8 L2P, 9 W-list M2P, 10 combine, 11 TF32 splits of the mixed path,
- * 12 M2L table generation of a streaming plan, 13 the FP64 L2L GEMM of the mixed
- * path, 14 compress / expand GEMMs of a compressed M2L. (Replaces the reference's
+ * 4 M2L (with L2L fused where the FP64 path reads dense M2L tables), 5 X-list P2L, 6 downward decode,
+ * 7 P2P, 8 L2P, 9 W-list M2P, 10 combine, 11 operand splits of the mixed path,
+ * 12 M2L table generation of a streaming plan, 13 the FP64 L2L GEMM (mixed
+ * path, FP64 path by convolution), 14 compress / expand GEMMs of a compressed M2L. (Replaces the reference's
  * wall-clock phase prints; it has no per-phase timers, util.py:692-724.) */
 #define HFMM_N_PHASES 15
 int hfmm_plan_set_profiling(hfmm_plan* plan, int32_t enable);
