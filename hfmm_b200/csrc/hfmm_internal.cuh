@@ -152,6 +152,7 @@ struct ConvPlan {
     bool on = false;       // the FP64 evaluate's M2L (else the dense tables)
     bool tables = false;   // K holds the current kernel's and levels' spectra
     int n = 0, n_slots = 0, n_groups = 0;
+    bool half = false;         // enough half-filled warps for k_conv_mul's form that skips them
     double spacing = 0.0;
     DevBuf<int32_t> pos, line_off, line_k;   // surface points in lattice line order
     DevBuf<double> tw, K;

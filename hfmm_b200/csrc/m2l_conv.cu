@@ -10,8 +10,8 @@
 // half spectrum. Against the dense tables (2 n_s^2 a pair and column) that is 8 n^3 a pair
 // and column pair: 27 against 350 kFLOP at p = 8, 97 against 2,120 at p = 12. One
 // evaluate, complex charges, field (B200): 1e6 points, p = 8, depth 5: 210.2 ms with the
-// tables, 31.8 now (products 13.4, transforms 3.3 and 4.0 of it); 20,000 points, depth 3:
-// p = 8 6.69 and 0.85 ms, p = 12 32.7 and 2.28 ms.
+// tables, 31.7 now (products 13.2, transforms 3.3 and 4.0 of it); 20,000 points, depth 3:
+// p = 8 6.69 and 0.84 ms, p = 12 32.7 and 2.23 ms.
 //
 // Work is laid out by PARENT: the children of one parent ("slot") sit side by side, absent
 // ones as zeros, X as [frequency][slot][child]. The products of one frequency and one of
@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 namespace hfmm {
 
@@ -345,7 +346,13 @@ __global__ void __launch_bounds__(256) k_conv_fwd(ConvCall c) {
 // offsets); K and the neighbour lists come from shared memory.
 constexpr int NT = 2, CONV_WARPS = 4, CONV_GROUP = 8 * NT * CONV_WARPS;
 
-__global__ void __launch_bounds__(32 * CONV_WARPS) k_conv_mul(ConvCall c, int nkx) {
+// HALF: warps left with one tile's slots (the eight at the coarsest level, a level's remainder)
+// skip the other tile. Where every warp is full that form takes 3 % more time, so it runs where
+// such warps are one in 16 or more: 20,000 points, p = 8 260 to 247 us, p = 12 906 to 845; 1e6
+// points 13.2 ms without, 13.7 with it. (One tile a warp everywhere: 247, 868 us and 14.8 ms.)
+// Eight CTAs an SM: with six (75 registers, the second tile under a branch in the loop) 14.2 ms.
+template <bool HALF>
+__global__ void __launch_bounds__(32 * CONV_WARPS, 8) k_conv_mul(ConvCall c, int nkx) {
     __shared__ double2 Kt[KTAB];
     __shared__ int nb[CONV_GROUP][27];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -385,49 +392,54 @@ __global__ void __launch_bounds__(32 * CONV_WARPS) k_conv_mul(ConvCall c, int nk
     const int off_t = (g & 1) * KSX + ((g >> 1) & 1) * KSY + (g >> 2);
     const int off_s = (t4 & 1) * KSX + (t4 >> 1) * KSY;
     const double2* Kl = Kt + 3 * (KSX + KSY + 1) + off_t - off_s;   // source children 4.. are one z further
-    double acc[NT][4];
+    auto tiles = [&](auto n_tiles) {
+        constexpr int N = n_tiles;
+        double acc[N][4];
 #pragma unroll
-    for (int a = 0; a < NT; ++a)
+        for (int a = 0; a < N; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-    double2 x[2][NT][2];
-    auto load = [&](int D, double2 (&v)[NT][2]) {
+            for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
+        double2 x[2][N][2];
+        auto load = [&](int D, double2 (&v)[N][2]) {
 #pragma unroll
-        for (int a = 0; a < NT; ++a) {
-            const double2* q = X + (int64_t)nb[t0 + a * 8 + g][D] * 8;
-            v[a][0] = __ldg(q);
-            v[a][1] = __ldg(q + 4);
+            for (int a = 0; a < N; ++a) {
+                const double2* q = X + (int64_t)nb[t0 + a * 8 + g][D] * 8;
+                v[a][0] = __ldg(q);
+                v[a][1] = __ldg(q + 4);
+            }
+        };
+        auto mul = [&](int D, const double2 (&v)[N][2]) {
+            int ox, oy, oz;
+            neigh_offset(D, ox, oy, oz);
+            const double2* Kd = Kl - 2 * (ox * KSX + oy * KSY + oz);
+            const double2 k0 = Kd[0], k1 = Kd[-1];
+#pragma unroll
+            for (int a = 0; a < N; ++a) dmma(acc[a], k0.x, k0.y, v[a][0].x);
+#pragma unroll
+            for (int a = 0; a < N; ++a) dmma(acc[a], -k0.y, k0.x, v[a][0].y);
+#pragma unroll
+            for (int a = 0; a < N; ++a) dmma(acc[a], k1.x, k1.y, v[a][1].x);
+#pragma unroll
+            for (int a = 0; a < N; ++a) dmma(acc[a], -k1.y, k1.x, v[a][1].y);
+        };
+        load(0, x[0]);
+#pragma unroll 1
+        for (int D = 0; D < 26; D += 2) {
+            load(D + 1, x[1]);
+            mul(D, x[0]);
+            if (D + 2 < 26) load(D + 2, x[0]);
+            mul(D + 1, x[1]);
+        }
+        double2* Y = c.Y + fo + g;
+#pragma unroll
+        for (int a = 0; a < N; ++a) {
+            const int s = t0 + a * 8 + 2 * t4;
+            if (s < G.z) Y[(int64_t)(G.y + s) * 8] = make_double2(acc[a][0], acc[a][2]);
+            if (s + 1 < G.z) Y[(int64_t)(G.y + s + 1) * 8] = make_double2(acc[a][1], acc[a][3]);
         }
     };
-    auto mul = [&](int D, const double2 (&v)[NT][2]) {
-        int ox, oy, oz;
-        neigh_offset(D, ox, oy, oz);
-        const double2* Kd = Kl - 2 * (ox * KSX + oy * KSY + oz);
-        const double2 k0 = Kd[0], k1 = Kd[-1];
-#pragma unroll
-        for (int a = 0; a < NT; ++a) dmma(acc[a], k0.x, k0.y, v[a][0].x);
-#pragma unroll
-        for (int a = 0; a < NT; ++a) dmma(acc[a], -k0.y, k0.x, v[a][0].y);
-#pragma unroll
-        for (int a = 0; a < NT; ++a) dmma(acc[a], k1.x, k1.y, v[a][1].x);
-#pragma unroll
-        for (int a = 0; a < NT; ++a) dmma(acc[a], -k1.y, k1.x, v[a][1].y);
-    };
-    load(0, x[0]);
-#pragma unroll 1
-    for (int D = 0; D < 26; D += 2) {
-        load(D + 1, x[1]);
-        mul(D, x[0]);
-        if (D + 2 < 26) load(D + 2, x[0]);
-        mul(D + 1, x[1]);
-    }
-    double2* Y = c.Y + fo + g;
-#pragma unroll
-    for (int a = 0; a < NT; ++a) {
-        const int s = t0 + a * 8 + 2 * t4;
-        if (s < G.z) Y[(int64_t)(G.y + s) * 8] = make_double2(acc[a][0], acc[a][2]);
-        if (s + 1 < G.z) Y[(int64_t)(G.y + s + 1) * 8] = make_double2(acc[a][1], acc[a][3]);
-    }
+    if (HALF && G.z - t0 <= 8) tiles(std::integral_constant<int, 1>());
+    else tiles(std::integral_constant<int, NT>());
 }
 
 // Inverse transform of a slot's children onto the surface points: per kz the x axis straight
@@ -665,6 +677,12 @@ void conv_schedule(hfmm_plan* P) {
     }
     C.n_slots = n_slots;
     C.n_groups = (int)groups.size();
+    int64_t warps = 0, halves = 0;
+    for (const int4& g : groups) {
+        warps += ceil_div(g.z, 8 * NT);
+        halves += (g.z - 1) % (8 * NT) < 8;
+    }
+    C.half = halves * 16 >= warps;
     if (!n_slots) return;
     auto up = [](auto& buf, const auto& h) {
         buf.alloc(h.size());
@@ -753,6 +771,7 @@ void conv_m2l(hfmm_plan* P, int R, int64_t fam_stride, cudaStream_t s) {
     const Kernel inv = R == 2 ? k_conv_inv<2> : k_conv_inv<1>;
     HFMM_CUDA(cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     HFMM_CUDA(cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_i));
+    auto mul = C.half ? k_conv_mul<true> : k_conv_mul<false>;
     for (int f = 0; f < P->n_fam; f += nf) {
         c.dens = P->equiv.p + f * fam_stride;
         c.check = P->check.p + f * fam_stride;
@@ -771,7 +790,7 @@ void conv_m2l(hfmm_plan* P, int R, int64_t fam_stride, cudaStream_t s) {
                 c.n_seg = std::min(segs, c.kz1 - c.kz0);
                 HFMM_LAUNCH(fwd, dim3((unsigned)(c.n_slots + 1), (unsigned)(8 / CH), (unsigned)(nf * c.n_seg)), PT,
                             smem, s, c);
-                HFMM_LAUNCH(k_conv_mul, dim3((unsigned)((int64_t)c.rows * nkx * c.n_groups), (unsigned)nf),
+                HFMM_LAUNCH(mul, dim3((unsigned)((int64_t)c.rows * nkx * c.n_groups), (unsigned)nf),
                             32 * CONV_WARPS, 0, s, c, nkx);
                 c.CH = CHi;
                 HFMM_LAUNCH(inv, dim3((unsigned)c.n_slots, (unsigned)(8 / CHi), (unsigned)nf), PT, smem_i, s, c);
