@@ -435,7 +435,10 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
     const int64_t fs = P->nb * (int64_t)R * P->ld;   // family stride of expansion arrays
     if (up) {
         PhaseTimer pt(X, s, 0);
-        gather_charges(P->n, P->sort_idx.p, q_re, q_im, P->q_s.p, s);
+        // complex charges of two families: the convolution balances the columns' magnitudes
+        const bool balance = R == 2 && NF == 2 && P->conv.on && P->rot_P == 0 && !(mixed && P->mixed_ready);
+        if (balance) HFMM_CUDA(cudaMemsetAsync(P->q_max.p, 0, 2 * sizeof(unsigned long long), s));
+        gather_charges(P->n, P->sort_idx.p, q_re, q_im, P->q_s.p, balance ? P->q_max.p : nullptr, s);
     }
     EvalView v = view(P);
 
@@ -1184,6 +1187,7 @@ int hfmm_plan_finalize(hfmm_plan* P) {
     }
     plan_queue_build(P);
     P->q_s.alloc(2 * P->n);
+    P->q_max.alloc(2);
     P->pot.alloc((size_t)2 * P->n);       // real and imaginary part per particle
     P->fld.alloc((size_t)2 * 3 * P->n);
     HFMM_CUDA(cudaDeviceSynchronize());

@@ -264,6 +264,7 @@ struct hfmm_plan {
 
     // evaluate scratch (allocated at finalize for R = 2)
     hfmm::DevBuf<double> q_s;        // R x n sorted charges
+    hfmm::DevBuf<unsigned long long> q_max;   // bits of the largest real and imaginary charge
     hfmm::DevBuf<double> check, equiv, loc, tmp;   // [fam][box][R][ld]
     hfmm::DevBuf<double> gemm_part;  // partial tiles of the main stream's split GEMMs
     int rot_P = 0, rot_n_dist = 0, rot_n_theta = 0;   // rotation-based M2L of the FP64 evaluate (0: dense)

@@ -6,8 +6,9 @@
 // multiplication by a number per frequency, summed over the V list before one inverse
 // transform per target:
 //     X = F(x) of every box;   Y_t = sum_d K_d .* X_{s(t, d)};   check_t = F^-1(Y_t).
-// Complex charges travel as one complex sequence (the kernel is real), real charges as the
-// half spectrum. Against the dense tables (2 n_s^2 a pair and column) that is 8 n^3 a pair
+// With two families complex charges travel as one complex sequence (the kernel is real), real
+// charges as the half spectrum; with one family the result's real and imaginary parts are
+// those of the charges, and each column is a real sequence of its own. Against the dense tables (2 n_s^2 a pair and column) that is 8 n^3 a pair
 // and column pair: 27 against 350 kFLOP at p = 8, 97 against 2,120 at p = 12. One
 // evaluate, complex charges, field (B200): 1e6 points, p = 8, depth 5: 210.2 ms with the
 // tables, 31.7 now (products 13.2, transforms 3.3 and 4.0 of it); 20,000 points, depth 3:
@@ -133,6 +134,27 @@ __global__ void k_conv_nbr(const int32_t* __restrict__ child, const int32_t* __r
 }
 
 // ---------------------------------------------------------------- transforms
+// A transform leaves a rounding of the larger column in the smaller one of a complex sequence.
+// The imaginary charges are therefore brought to the scale of the real ones, by a power of two
+// (exact), on the way in and back on the way out: each column's error is then that of its own
+// magnitude, as where the columns travel apart (k = 1e-6, imaginary charges 1e-8 of the real
+// ones: imaginary part off by 4e-10 without, 4e-15 with it). A column of zeros stays zeros.
+struct Balance {
+    double up = 1.0, down = 1.0;
+    bool re = true, im = true;   // the column holds a charge
+};
+__device__ __forceinline__ Balance balance(const unsigned long long* q_max) {
+    Balance b;
+    b.re = q_max[0] != 0;
+    b.im = q_max[1] != 0;
+    const int er = (int)(q_max[0] >> 52), ei = (int)(q_max[1] >> 52), d = er - ei;
+    if (er > 0 && ei > 0 && er < 2047 && ei < 2047 && abs(d) < 1000) {
+        b.up = __longlong_as_double((long long)(1023 + d) << 52);
+        b.down = __longlong_as_double((long long)(1023 - d) << 52);
+    }
+    return b;
+}
+
 // One axis is a small real matrix times many columns, and runs on the FP64 tensor
 // instruction too. The pairs (k, n - k) share their sums: with v_j complex,
 //   forward, j < p values in:   C_k = sum_j v_j cos(2 pi j k / n), S_k = sum_j v_j sin(..),
@@ -248,7 +270,7 @@ __global__ void __launch_bounds__(256) k_conv_fwd(ConvCall c) {
     extern __shared__ double2 sh[];
     const AxisShape a = axis_shape(c);
     const int p = c.p, n = c.n, nh = p, CH = c.CH, nky = c.ky1 - c.ky0;
-    const int slot = blockIdx.x, c0 = blockIdx.y * CH, fam = blockIdx.z / c.n_seg, seg = blockIdx.z % c.n_seg;
+    const int slot = blockIdx.x, c0 = blockIdx.y * CH, seq = blockIdx.z / c.n_seg, seg = blockIdx.z % c.n_seg;
     const int nz = c.kz1 - c.kz0, kz0 = c.kz0 + seg * nz / c.n_seg, kz1 = c.kz0 + (seg + 1) * nz / c.n_seg;
     double2* tw = sh;                          // n
     double2* tz = tw + n;                      // p: e^{2 pi i k kz / n}
@@ -258,7 +280,7 @@ __global__ void __launch_bounds__(256) k_conv_fwd(ConvCall c) {
     double* xs = reinterpret_cast<double*>(A2 + p * nky * a.SR);   // [point][CH][R]
     const int nkx = R == 2 ? n : nh;
     const int64_t fstride = (int64_t)(c.n_slots + 1) * 8;   // values of one frequency
-    double2* X = c.X + (int64_t)fam * c.rows * nkx * fstride + (int64_t)slot * 8 + c0;
+    double2* X = c.X + (int64_t)seq * c.rows * nkx * fstride + (int64_t)slot * 8 + c0;
     const int tid = threadIdx.x, nt = blockDim.x;
     if (slot == c.n_slots) {   // the zero slot
         for (int64_t i = tid; seg == 0 && i < (int64_t)c.rows * nkx * CH; i += nt)
@@ -266,11 +288,13 @@ __global__ void __launch_bounds__(256) k_conv_fwd(ConvCall c) {
         return;
     }
     for (int i = tid; i < n; i += nt) tw[i] = c.tw[i];
+    const Balance bal = R == 2 ? balance(c.q_max) : Balance();
     for (int ch = 0; ch < CH; ++ch) {
         const int b = c.child[slot * 8 + c0 + ch];
-        const double* src = c.dens + (int64_t)fam * c.fam_stride + (int64_t)b * R * c.ld;
+        const double* src = c.dens + seq * c.seq_stride + b * c.box_stride;
         for (int r = 0; r < R; ++r)
-            for (int s = tid; s < c.n_s; s += nt) xs[(c.pos[s] * CH + ch) * R + r] = b >= 0 ? src[r * c.ld + s] : 0.0;
+            for (int s = tid; s < c.n_s; s += nt)
+                xs[(c.pos[s] * CH + ch) * R + r] = b >= 0 ? src[r * c.ld + s] * (r ? bal.up : 1.0) : 0.0;
     }
     __syncthreads();
     axis_table(a, tw, T);
@@ -358,7 +382,7 @@ __global__ void __launch_bounds__(32 * CONV_WARPS, 8) k_conv_mul(ConvCall c, int
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int grp = blockIdx.x % c.n_groups;
     const int64_t f = blockIdx.x / c.n_groups;      // frequency within the chunk
-    const int fam = blockIdx.y;
+    const int seq = blockIdx.y;
     const int4 G = c.groups[grp];                   // level, first slot, slots
     const int nky = c.ky1 - c.ky0;
     {
@@ -370,7 +394,7 @@ __global__ void __launch_bounds__(32 * CONV_WARPS, 8) k_conv_mul(ConvCall c, int
             ky = ky ? n - ky : 0;
             kz = kz ? n - kz : 0;
         }
-        const double2* K = c.K + (((int64_t)(G.x - 2) * c.n_fam + fam) * n * n * nh +
+        const double2* K = c.K + (((int64_t)(G.x - 2) * c.n_fam + seq * c.seq_fam) * n * n * nh +
                                   ((int64_t)kz * n + ky) * nh + kx) * N_DISP;
         for (int d = tid; d < N_DISP; d += 32 * CONV_WARPS) {
             double2 v = K[d];
@@ -387,7 +411,7 @@ __global__ void __launch_bounds__(32 * CONV_WARPS, 8) k_conv_mul(ConvCall c, int
     if (t0 >= G.z) return;
     const int g = lane >> 2, t4 = lane & 3;
     const int64_t fstride = (int64_t)(c.n_slots + 1) * 8;
-    const int64_t fo = ((int64_t)fam * c.rows * nkx + f) * fstride;
+    const int64_t fo = ((int64_t)seq * c.rows * nkx + f) * fstride;
     const double2* X = c.X + fo + t4;
     const int off_t = (g & 1) * KSX + ((g >> 1) & 1) * KSY + (g >> 2);
     const int off_s = (t4 & 1) * KSX + (t4 >> 1) * KSY;
@@ -452,7 +476,7 @@ __global__ void __launch_bounds__(256) k_conv_inv(ConvCall c) {
     extern __shared__ double2 sh[];
     const AxisShape a = axis_shape(c);
     const int p = c.p, n = c.n, nh = p, CH = c.CH, nky = c.ky1 - c.ky0;
-    const int slot = blockIdx.x, c0 = blockIdx.y * CH, fam = blockIdx.z;
+    const int slot = blockIdx.x, c0 = blockIdx.y * CH, seq = blockIdx.z;
     double2* tw = sh;                          // n
     double2* tz = tw + n;                      // p
     double2* T = tz + p;
@@ -462,16 +486,17 @@ __global__ void __launch_bounds__(256) k_conv_inv(ConvCall c) {
     int* pts = reinterpret_cast<int*>(acc + c.n_s * CH * R);        // [point] U1 row and k
     const int nkx = R == 2 ? n : nh;
     const int64_t fstride = (int64_t)(c.n_slots + 1) * 8;
-    const double2* Y = c.Y + (int64_t)fam * c.rows * nkx * fstride + (int64_t)slot * 8 + c0;
+    const double2* Y = c.Y + (int64_t)seq * c.rows * nkx * fstride + (int64_t)slot * 8 + c0;
     const int tid = threadIdx.x, nt = blockDim.x;
     for (int i = tid; i < n; i += nt) tw[i] = c.tw[i];
     for (int i = tid; i < c.n_s; i += nt) pts[i] = c.line_k[i];
+    const Balance bal = R == 2 ? balance(c.q_max) : Balance();
     for (int ch = 0; ch < CH; ++ch) {
         const int b = c.child[slot * 8 + c0 + ch];
-        const double* src = c.check + (int64_t)fam * c.fam_stride + (int64_t)b * R * c.ld;
+        const double* src = c.check + seq * c.seq_stride + b * c.box_stride;
         for (int r = 0; r < R; ++r)
             for (int s = tid; s < c.n_s; s += nt)
-                acc[(c.pos[s] * CH + ch) * R + r] = c.first || b < 0 ? 0.0 : src[r * c.ld + s];
+                acc[(c.pos[s] * CH + ch) * R + r] = c.first || b < 0 ? 0.0 : src[r * c.ld + s] * (r ? bal.up : 1.0);
     }
     __syncthreads();
     axis_table(a, tw, T);
@@ -536,9 +561,10 @@ __global__ void __launch_bounds__(256) k_conv_inv(ConvCall c) {
     for (int ch = 0; ch < CH; ++ch) {
         const int b = c.child[slot * 8 + c0 + ch];
         if (b < 0) continue;
-        double* dst = c.check + (int64_t)fam * c.fam_stride + (int64_t)b * R * c.ld;
+        double* dst = c.check + seq * c.seq_stride + b * c.box_stride;
         for (int r = 0; r < R; ++r)
-            for (int s = tid; s < c.n_s; s += nt) dst[r * c.ld + s] = acc[(c.pos[s] * CH + ch) * R + r];
+            for (int s = tid; s < c.n_s; s += nt)
+                dst[r * c.ld + s] = (r ? bal.im : bal.re) ? acc[(c.pos[s] * CH + ch) * R + r] * (r ? bal.down : 1.0) : 0.0;
     }
 }
 
@@ -732,13 +758,19 @@ void conv_m2l(hfmm_plan* P, int R, int64_t fam_stride, cudaStream_t s) {
     c.groups = C.groups.p;
     c.tw = reinterpret_cast<const double2*>(C.tw.p);
     c.n_fam = P->n_fam;
-    c.fam_stride = fam_stride;
+    c.box_stride = (int64_t)R * P->ld;
+    c.q_max = P->q_max.p;
+    // sequences: the families, or the charge columns of a single family (as real ones)
+    const int n_seq = P->n_fam == 1 ? R : P->n_fam;
+    if (P->n_fam == 1) R = 1;
+    c.seq_fam = P->n_fam > 1;
+    c.seq_stride = c.seq_fam ? fam_stride : P->ld;
     const int n = C.n, nkx = R == 2 ? n : (n + 1) / 2;
     double* ws = P->streamed ? static_cast<double*>(P->ws) : C.ws.p;
     const size_t ws_values = (P->streamed ? P->ws_bytes : C.ws.n * sizeof(double)) / sizeof(double2);
-    // families together when a plane of both fits, else one after the other; whole planes
+    // sequences together when a plane of both fits, else one after the other; whole planes
     // of frequencies, or rows of one plane where not even one fits
-    int nf = P->n_fam;
+    int nf = n_seq;
     if (2 * (size_t)chunk_values(P, nkx, nf) * n > ws_values) nf = 1;
     const size_t row = 2 * (size_t)chunk_values(P, nkx, nf);
     const int planes = (int)std::min<size_t>(n, ws_values / (row * n));
@@ -772,10 +804,10 @@ void conv_m2l(hfmm_plan* P, int R, int64_t fam_stride, cudaStream_t s) {
     HFMM_CUDA(cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     HFMM_CUDA(cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_i));
     auto mul = C.half ? k_conv_mul<true> : k_conv_mul<false>;
-    for (int f = 0; f < P->n_fam; f += nf) {
-        c.dens = P->equiv.p + f * fam_stride;
-        c.check = P->check.p + f * fam_stride;
-        c.K = reinterpret_cast<const double2*>(C.K.p) + (int64_t)f * n * n * ((n + 1) / 2) * N_DISP;
+    for (int f = 0; f < n_seq; f += nf) {
+        c.dens = P->equiv.p + f * c.seq_stride;
+        c.check = P->check.p + f * c.seq_stride;
+        c.K = reinterpret_cast<const double2*>(C.K.p) + (int64_t)f * c.seq_fam * n * n * ((n + 1) / 2) * N_DISP;
         c.first = 1;
         for (int kz = 0; kz < n; kz += dz)
             for (int ky = 0; ky < n; ky += rows) {

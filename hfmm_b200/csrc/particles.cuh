@@ -197,6 +197,6 @@ __device__ __forceinline__ void pair64(int yukawa, double k, double dx, double d
 void particles_f64(const ParticlePass& p, cudaStream_t s);
 void particles_mixed(const ParticlePass& p, cudaStream_t s);
 void gather_charges(int64_t n, const int32_t* sidx, const double* q_re, const double* q_im,
-                    double* q_s, cudaStream_t s);
+                    double* q_s, unsigned long long* q_max, cudaStream_t s);
 
 }  // namespace hfmm

@@ -265,13 +265,35 @@ __global__ void __launch_bounds__(32 * P2P_WARPS) k_p2p(EvalView v, const int32_
     }
 }
 
+// Charges in leaf-major order; q_max (nullable) is raised to the bits of the largest real and
+// imaginary magnitude (infinities and NaN the largest bits there are)
 __global__ void k_gather_q(int64_t n, const int32_t* __restrict__ sidx, const double* __restrict__ q_re,
-                           const double* __restrict__ q_im, double* q_s) {
+                           const double* __restrict__ q_im, double* q_s, unsigned long long* q_max) {
+    __shared__ unsigned long long most[2];
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int64_t o = sidx[i];
-    q_s[i] = q_re[o];
-    if (q_im) q_s[n + i] = q_im[o];
+    unsigned long long m[2] = {0, 0};
+    if (i < n) {
+        const int64_t o = sidx[i];
+        const double re = q_re[o], im = q_im ? q_im[o] : 0.0;
+        q_s[i] = re;
+        if (q_im) q_s[n + i] = im;
+        m[0] = (unsigned long long)__double_as_longlong(re) & ~(1ull << 63);
+        m[1] = (unsigned long long)__double_as_longlong(im) & ~(1ull << 63);
+    }
+    if (!q_max) return;
+    if (threadIdx.x < 2) most[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long v = __shfl_xor_sync(0xffffffffu, m[c], o);
+            m[c] = v > m[c] ? v : m[c];
+        }
+        if ((threadIdx.x & 31) == 0 && m[c]) atomicMax(&most[c], m[c]);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 && most[threadIdx.x]) atomicMax(q_max + threadIdx.x, most[threadIdx.x]);
 }
 
 // The particles' sums, back to input order
@@ -346,8 +368,8 @@ void particles_mode(const ParticlePass& p, cudaStream_t s) {
 }  // namespace
 
 void gather_charges(int64_t n, const int32_t* sidx, const double* q_re, const double* q_im,
-                    double* q_s, cudaStream_t s) {
-    HFMM_LAUNCH(k_gather_q, nblk(n, 256), 256, 0, s, n, sidx, q_re, q_im, q_s);
+                    double* q_s, unsigned long long* q_max, cudaStream_t s) {
+    HFMM_LAUNCH(k_gather_q, nblk(n, 256), 256, 0, s, n, sidx, q_re, q_im, q_s, q_max);
 }
 
 void particles_f64(const ParticlePass& p, cudaStream_t s) {
