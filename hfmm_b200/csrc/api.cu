@@ -272,6 +272,9 @@ void stream_maps(hfmm_plan* P) {
             make_table_maps(maps[l].a[f], ws + f * fam, P->n_fam * fam, P->n_s, P->ld, 316);
 }
 
+// The largest magnitudes of a family's densities at a level, one per charge column
+unsigned long long* x_max(hfmm_plan* P, int f, int l) { return P->x_max.p + (f * MAX_LEVELS + l) * 2; }
+
 // The low-rank mixed M2L of one level and family (R charge columns): the call of
 // m2l_split / one entry of the batch's M2L queue.
 MixedCall cx_call(hfmm_plan* P, int l, int f, int R) {
@@ -284,7 +287,7 @@ MixedCall cx_call(hfmm_plan* P, int l, int f, int R) {
     mc.disp_compact = P->disp_compact.p;
     mc.B = lb(T.xc_s.p, T.ckld);
     mc.b_plane = T.xc_s.n / 2;
-    mc.b_max[0] = P->x_max.p + f * MAX_LEVELS + l;
+    mc.b_max[0] = x_max(P, f, l);
     mc.a_scale[0] = T.c_scale;
     mc.out = lb(T.yc.p, T.cmld);
     mc.src_lo = P->level_lo[l];   // the level's buffers hold its own boxes only
@@ -606,23 +609,22 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
             for (int f = 0; f < NF; ++f) {
                 LevelTables& T = P->tables[f][l];
                 gemm_1(K_CMP, l, f, P->equiv.p + f * fs, P->ld, level_base(T.xc.p, l, T.ckld), T.ckld,
-                       s, nullptr, P->x_max.p + f * MAX_LEVELS + l);
+                       s, nullptr, x_max(P, f, l));
                 const int64_t nbl = P->level_hi[l] - P->level_lo[l];
                 if (R == 2 && T.grid && g_m2l_grid.load())   // complete level: into the dense grid
-                    split_planes_grid(T.xc.p, P->x_max.p + f * MAX_LEVELS + l, P->m_id.p + P->level_lo[l], nbl, T.grid, T.ckld,
+                    split_planes_grid(T.xc.p, x_max(P, f, l), P->m_id.p + P->level_lo[l], nbl, T.grid, T.ckld,
                                       T.xg_s.p, s);
                 else
-                    split_planes(T.xc.p, P->x_max.p + f * MAX_LEVELS + l, T.xc_s.p, T.xc_s.n / 2, nbl * R * T.ckld,
-                                 s);
+                    split_planes(T.xc.p, x_max(P, f, l), T.xc_s.p, T.xc_s.n / 2, nbl * R, T.ckld, R, s);
             }
     } else if (up && use_mx) {   // the planes of every equivalent density (B operand)
         PhaseTimer pt(X, s, 11);
         for (int f = 0; f < NF; ++f)
             for (int l = 2; l <= P->md; ++l) {
                 const int64_t o = f * fs + (int64_t)P->level_lo[l] * R * P->ld;
-                const int64_t m = (int64_t)(P->level_hi[l] - P->level_lo[l]) * R * P->ld;
-                absmax(P->equiv.p + o, m, P->x_max.p + f * MAX_LEVELS + l, s);
-                split_planes(P->equiv.p + o, P->x_max.p + f * MAX_LEVELS + l, P->e_s.p + o, P->e_s.n / 2, m, s);
+                const int64_t rows = (int64_t)(P->level_hi[l] - P->level_lo[l]) * R;
+                absmax(P->equiv.p + o, rows, P->ld, R, x_max(P, f, l), s);
+                split_planes(P->equiv.p + o, x_max(P, f, l), P->e_s.p + o, P->e_s.n / 2, rows, P->ld, R, s);
             }
     }
     // split evaluate (a batch's queued M2L): the upward half ends here; the downward half
@@ -744,7 +746,7 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
             mc.B = P->e_s.p;
             mc.b_plane = P->e_s.n / 2;
             for (int f = 0; f < NF; ++f) {
-                mc.b_max[f] = P->x_max.p + f * MAX_LEVELS + l;
+                mc.b_max[f] = x_max(P, f, l);
                 mc.a_scale[f] = m2l_scale(P, f, l);
             }
             mc.fold2 = 0;   // dense tables: 24 MMAs a unit gave 1.1 of the TF32 halves' error, 12 give 0.6
@@ -1182,7 +1184,7 @@ int hfmm_plan_finalize(hfmm_plan* P) {
         }
         P->e_s.alloc(2 * exp);
         P->e_s.zero();
-        P->x_max.alloc(2 * MAX_LEVELS);
+        P->x_max.alloc(2 * MAX_LEVELS * 2);
         P->mixed_ready = true;
     }
     plan_queue_build(P);

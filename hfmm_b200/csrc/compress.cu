@@ -213,7 +213,7 @@ int hfmm_plan_set_m2l_compressed(hfmm_plan* P, int32_t family, int32_t level, in
         DevBuf<unsigned long long> most;
         most.alloc(1);
         most.zero();
-        absmax(C_dev, (int64_t)N_M2L * rank * rank, most.p, 0);
+        absmax(C_dev, (int64_t)N_M2L * rank, rank, 1, most.p, 0);
         unsigned long long h_most = 0;
         HFMM_CUDA(cudaMemcpy(&h_most, most.p, sizeof(h_most), cudaMemcpyDeviceToHost));
         T.c_scale = plane_scale(h_most);

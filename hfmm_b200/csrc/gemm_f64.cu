@@ -257,21 +257,24 @@ __global__ void __launch_bounds__(128, 3) k_gemm_f64(GemmCall c, int* err) {
                          : nullptr;
     const double* sc = (fam == 1 && c.scale_f1) ? c.scale_f1 : c.scale;
     if (c.most) {   // (one-entry calls without scale or split: what is stored is acc)
-        double top = 0.0;
-        bool odd = false;   // infinities and NaN: the largest bits there are
 #pragma unroll
-        for (int i = 0; i < MI * NI * 4; ++i) {
-            const double v = fabs((&acc[0][0][0])[i]);
-            odd = odd || !(v <= 1.7976931348623157e308);
-            top = fmax(top, v);
-        }
-        unsigned long long bits = odd ? 0x7ff0000000000000ull : (unsigned long long)__double_as_longlong(top);
+        for (int r = 0; r < R; ++r) {   // acc's odd values are odd columns'
+            double top = 0.0;
+            bool odd = false;   // infinities and NaN: the largest bits there are
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long v = __shfl_xor_sync(0xffffffffu, bits, o);
-            bits = v > bits ? v : bits;
+            for (int i = r; i < MI * NI * 4; i += R) {
+                const double v = fabs((&acc[0][0][0])[i]);
+                odd = odd || !(v <= 1.7976931348623157e308);
+                top = fmax(top, v);
+            }
+            unsigned long long bits = odd ? 0x7ff0000000000000ull : (unsigned long long)__double_as_longlong(top);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const unsigned long long v = __shfl_xor_sync(0xffffffffu, bits, o);
+                bits = v > bits ? v : bits;
+            }
+            if (lane == 0 && bits) atomicMax(c.most + r, bits);
         }
-        if (lane == 0 && bits) atomicMax(c.most, bits);
     }
 #pragma unroll
     for (int mi = 0; mi < MI; ++mi)

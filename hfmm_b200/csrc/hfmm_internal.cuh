@@ -234,7 +234,7 @@ struct hfmm_plan {
     hfmm::DevBuf<int32_t> gx_org[hfmm::MAX_LEVELS];
     hfmm::DevBuf<int32_t> disp_compact;     // 343 -> M2L table index or -1
     hfmm::DevBuf<uint16_t> e_s;             // split densities [plane][fam][box][R][ld]
-    hfmm::DevBuf<unsigned long long> x_max; // [fam][level] largest magnitude of the densities split
+    hfmm::DevBuf<unsigned long long> x_max; // [fam][level][column] largest magnitude of the densities split
     void* mx_maps = nullptr;                // MixedMaps per level (host array)
     bool compressed = false;                // every level has a compressed M2L (mixed path)
     bool folded = false;                    // its folded tables are those of the current tables
@@ -341,7 +341,7 @@ struct GemmCall {
     int64_t a_fam_stride;      // entries between the families' A pointer sets
     int n_fam;
     int64_t nb;                // box count (bounds checks)
-    unsigned long long* most;  // nullable: raised to the bits of the largest magnitude stored
+    unsigned long long* most;  // nullable: per column, raised to the bits of the largest magnitude stored
     double* part;              // nullable: scratch for entry splits of small grids
     int64_t part_cap;          // its size in doubles
     int n_split;               // set by gemm_f64: CTAs per output tile (entry ranges)

@@ -288,12 +288,14 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (aborted) {
                 if (lane == 0) atomicOr(c.err, ERRF_TIMEOUT);
             } else if (row_ok) {
-                const double unscale = 1.0 / (c.a_scale[0] * plane_scale(*c.b_max[0]));
+                double unscale[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) unscale[r] = 1.0 / (c.a_scale[0] * plane_scale(c.b_max[0][r]));
 #pragma unroll
                 for (int j = 0; j < COLS_PER_FOLD_WARP; ++j) {
                     const int n = c_lo + j;
                     const int t = ctl.tgt[n / R];
-                    if (t >= 0) c.out[((int64_t)t * R + (n % R)) * c.ldm + m] = sum[j] * unscale;
+                    if (t >= 0) c.out[((int64_t)t * R + (n % R)) * c.ldm + m] = sum[j] * unscale[j % R];
                 }
             }
             u_total += n_units;

@@ -279,12 +279,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_split(const __grid_constant_
         if (aborted) {
             if (lane == 0) atomicOr(c.err, ERRF_TIMEOUT);
         } else if (row_ok) {
-            const double unscale = 1.0 / (c.a_scale[fam] * plane_scale(*c.b_max[fam]));
+            double unscale[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) unscale[r] = 1.0 / (c.a_scale[fam] * plane_scale(c.b_max[fam][r]));
 #pragma unroll
             for (int j = 0; j < COLS_PER_FOLD_WARP; ++j) {
                 const int n = c_lo + j;
                 const int t = ctl.tgt[n / R];
-                if (t >= 0) out[((int64_t)t * R + (n % R)) * c.ldm + m] = sum[j] * unscale;
+                if (t >= 0) out[((int64_t)t * R + (n % R)) * c.ldm + m] = sum[j] * unscale[j % R];
             }
         }
     } else if (warp == 4) {
@@ -378,28 +380,41 @@ __global__ void __launch_bounds__(THREADS, 1) k_m2l_split(const __grid_constant_
     }
 }
 
-__global__ void k_absmax(const double* __restrict__ src, int64_t n, unsigned long long* most) {
-    unsigned long long m = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const unsigned long long v = (unsigned long long)__double_as_longlong(src[i]) & ~(1ull << 63);
-        m = v > m ? v : m;
+// A warp takes whole rows: a row is of one charge column.
+__global__ void k_absmax(const double* __restrict__ src, int64_t rows, int ld, int R, unsigned long long* most) {
+    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    unsigned long long m[2] = {0, 0};
+    for (int64_t row = blockIdx.x * (int64_t)warps + (threadIdx.x >> 5); row < rows; row += (int64_t)gridDim.x * warps) {
+        unsigned long long t = 0;
+        for (int j = lane; j < ld; j += 32) {
+            const unsigned long long v = (unsigned long long)__double_as_longlong(src[row * ld + j]) & ~(1ull << 63);
+            t = v > t ? v : t;
+        }
+        if (row % R) m[1] = t > m[1] ? t : m[1];
+        else m[0] = t > m[0] ? t : m[0];
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
-        m = v > m ? v : m;
+    for (int c = 0; c < 2; ++c) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long v = __shfl_xor_sync(0xffffffffu, m[c], o);
+            m[c] = v > m[c] ? v : m[c];
+        }
+        if (lane == 0 && m[c]) atomicMax(most + c, m[c]);
     }
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(most, m);
 }
 
 __global__ void k_split_planes(const double* __restrict__ src, const unsigned long long* __restrict__ most,
-                               uint16_t* out, int64_t plane, int64_t n) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint16_t p[2];
-    split2(src[i] * plane_scale(*most), p);
-    out[i] = p[0];
-    out[plane + i] = p[1];
+                               uint16_t* out, int64_t plane, int64_t rows, int ld, int R) {
+    const int64_t row = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    const double s = plane_scale(most[row % R]);
+    for (int64_t i = row * ld + (threadIdx.x & 31); i < (row + 1) * ld; i += 32) {
+        uint16_t p[2];
+        split2(src[i] * s, p);
+        out[i] = p[0];
+        out[plane + i] = p[1];
+    }
 }
 
 // densities [box][2][ckld] of a complete level -> planes at the box's grid position; two
@@ -414,7 +429,7 @@ __global__ void k_split_planes_grid(const double2* __restrict__ src, const unsig
     if (x >= G || y >= G || z >= G) return;
     const int64_t o = ((x * G + y) * G + z) * ckld + within, plane = (int64_t)G * G * G * ckld;
     const double2 v = src[i];
-    const double s = plane_scale(*most);
+    const double s = plane_scale(most[2 * within >= ckld]);   // ckld values of each column
     uint16_t p[2], q[2];
     split2(v.x * s, p);
     split2(v.y * s, q);
@@ -504,9 +519,10 @@ void make_grid_maps(CUtensorMap (&map)[2], const uint16_t* base, int valid, int 
     }
 }
 
-void absmax(const double* src, int64_t n, unsigned long long* most, cudaStream_t s) {
-    if (n <= 0) return;
-    HFMM_LAUNCH(k_absmax, (unsigned)std::min<int64_t>(ceil_div(n, 1024), 8 * sm_count()), 256, 0, s, src, n, most);
+void absmax(const double* src, int64_t rows, int ld, int R, unsigned long long* most, cudaStream_t s) {
+    if (rows <= 0) return;
+    HFMM_LAUNCH(k_absmax, (unsigned)std::min<int64_t>(ceil_div(rows, 8), 8 * sm_count()), 256, 0, s, src, rows, ld, R,
+                most);
 }
 
 void split_planes_grid(const double* src, const unsigned long long* most, const uint64_t* m_id, int64_t n_boxes,
@@ -517,10 +533,10 @@ void split_planes_grid(const double* src, const unsigned long long* most, const 
                 most, m_id, n, G, ckld, reinterpret_cast<uint32_t*>(out));
 }
 
-void split_planes(const double* src, const unsigned long long* most, uint16_t* out, int64_t plane, int64_t n,
-                  cudaStream_t s) {
-    if (n <= 0) return;
-    HFMM_LAUNCH(k_split_planes, (unsigned)ceil_div(n, 256), 256, 0, s, src, most, out, plane, n);
+void split_planes(const double* src, const unsigned long long* most, uint16_t* out, int64_t plane, int64_t rows,
+                  int ld, int R, cudaStream_t s) {
+    if (rows <= 0) return;
+    HFMM_LAUNCH(k_split_planes, (unsigned)ceil_div(rows, 8), 256, 0, s, src, most, out, plane, rows, ld, R);
 }
 
 void split_transpose_tables(const double* at, double scale, uint16_t* out, int ld, int count) {

@@ -26,7 +26,7 @@ struct MixedCall {
     const int32_t* disp_compact;   // 343: displacement -> M2L table index (-1 = adjacent)
     const uint16_t* B;             // equivalent densities' planes, [plane][fam][box][R][ld] FP16
     int64_t b_plane;               // elements between planes
-    const unsigned long long* b_max[2];   // per family: bits of the densities' largest magnitude
+    const unsigned long long* b_max[2];   // per family: bits of each column's largest density
     double a_scale[2];             // per family: the scale of A's planes
     double* out;                   // check potentials [fam][box][R][ld], FP64
     int R, ld, n_fam;
@@ -54,7 +54,8 @@ extern std::atomic<uint64_t> g_m2l_wait_ns;
 extern std::atomic<int> g_m2l_starve;
 
 // The two FP16 planes of a scaled value: hi its rounding, lo the rounding of the rest (exact in
-// FP64). The scale, a power of two, puts the largest magnitude of an operand in [2^13, 2^14):
+// FP64). The scale, a power of two, puts the largest magnitude of an operand (of one charge
+// column of the densities: a small column keeps its bits beside a large one) in [2^13, 2^14):
 // a value down to 2^-16 of that keeps the full 22 bits, a smaller one is off by at most 2^-25
 // in scaled units, 2^-38 of the largest.
 __device__ __forceinline__ void split2(double x, uint16_t (&p)[2]) {
@@ -84,11 +85,11 @@ __host__ __device__ __forceinline__ double plane_scale(unsigned long long most) 
 void make_table_maps(CUtensorMap (&map)[2], const uint16_t* base, size_t plane, int valid, int ld, int count,
                      int ldm = 0);
 void make_grid_maps(CUtensorMap (&map)[2], const uint16_t* base, int valid, int ckld, int G);
-// n FP64 values, the largest magnitude's bits at `most` -> their FP16 planes, `plane` elements
-// apart; absmax raises *most to the largest magnitude of src
-void split_planes(const double* src, const unsigned long long* most, uint16_t* out, int64_t plane, int64_t n,
-                  cudaStream_t s);
-void absmax(const double* src, int64_t n, unsigned long long* most, cudaStream_t s);
+// rows of ld FP64 values, row i of charge column i % R, each column's largest magnitude's bits at
+// most[column] -> their FP16 planes, `plane` elements apart; absmax raises most[column] to it
+void split_planes(const double* src, const unsigned long long* most, uint16_t* out, int64_t plane, int64_t rows,
+                  int ld, int R, cudaStream_t s);
+void absmax(const double* src, int64_t rows, int ld, int R, unsigned long long* most, cudaStream_t s);
 // a complete level's densities [box][2][ckld] (boxes in level order from m_id) -> planes of
 // the dense grid [x][y][z][2][ckld] of side G
 void split_planes_grid(const double* src, const unsigned long long* most, const uint64_t* m_id, int64_t n_boxes,

@@ -21,7 +21,7 @@ def _columns(n):
 
 
 @pytest.mark.parametrize("kappa", [0.0, 5.0])
-@pytest.mark.parametrize("precision,tol", [(0, 3e-12)])
+@pytest.mark.parametrize("precision,tol", [(0, 3e-12), (1, 2e-6)])
 def test_one_family(kappa, precision, tol):
     import hfmm_b200
     from hfmm_b200.kernels import LAPLACE, yukawa
@@ -36,7 +36,7 @@ def test_one_family(kappa, precision, tol):
     st.close()
 
 
-@pytest.mark.parametrize("precision,tol", [(0, 3e-12)])
+@pytest.mark.parametrize("precision,tol", [(0, 3e-12), (1, 2e-6)])
 def test_two_families_small_wavenumber(precision, tol):
     import hfmm_b200
     pos, a, b = _columns(9000)
