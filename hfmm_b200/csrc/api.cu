@@ -1154,7 +1154,7 @@ int hfmm_plan_finalize(hfmm_plan* P) {
     P->tmp.zero();
     // mixed path: the tables' FP16 planes, tensor maps, split density buffers (needs ld >= 128);
     // with a compressed M2L on every level the dense planes are not needed
-    if (P->ld >= 128) {
+    if (P->ld >= 128 && planes_hold(P)) {
         std::vector<int32_t> dc(N_DISP, -1);
         auto madj = nonadjacent_map();
         for (size_t i = 0; i < madj.size(); ++i) dc[madj[i]] = (int32_t)i;

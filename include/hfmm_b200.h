@@ -46,7 +46,9 @@ extern "C" {
                                  chains, folded into FP64), P2P in FP32 with an
                                  FP64 phase reduction; decodes, M2M, L2L, P2M, L2P FP64.
                                  M2L needs p >= 5 (ld = n_s rounded up to 32 >= 128);
-                                 smaller p runs its FP64 GEMM.                         */
+                                 smaller p, and a screened kernel with kappa x domain
+                                 extent > 2 (its clusters' results stay apart, beyond the
+                                 planes' range), run the M2L in FP64.                  */
 
 typedef struct hfmm_plan hfmm_plan;
 

@@ -1,0 +1,31 @@
+"""The mixed path where the charges span many orders of magnitude: two clusters in opposite
+corners, one with charges 2^e of the other's. With a screened kernel the weak cluster's
+results are its own, so its error against FP64 is measured by itself, at the mixed path's 2e-6;
+kappa on both sides of the line (kappa x extent = 2) where the M2L's operand planes hold.
+With Helmholtz the strong cluster's field reaches everywhere and sets the scale."""
+import numpy as np
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("eps", [None, 1e-7])
+@pytest.mark.parametrize("kappa", [0.0, 1.9, 2.2, 8.0, 40.0, "helmholtz"])
+def test_weak_cluster(kappa, eps):
+    import hfmm_b200
+    from hfmm_b200.kernels import LAPLACE, helmholtz, yukawa
+    rng = np.random.default_rng(11)
+    n = 8000
+    pos = np.concatenate([np.clip(c + 0.04 * rng.normal(size=(n // 2, 3)), 0, 1) for c in (0.1, 0.9)])
+    pos[0], pos[-1] = 0.0, 1.0   # the domain is the unit cube
+    q = rng.normal(size=n)
+    spec = helmholtz(9.0) if kappa == "helmholtz" else yukawa(kappa) if kappa else LAPLACE
+    st = hfmm_b200.kernel_setup(pos, spec, p=8, N_max=48, m2l_compress=eps)
+    for e in (0, 18, 26, 40):
+        v = q.copy()
+        v[: n // 2] *= 2.0 ** e
+        for x, y in zip(hfmm_b200.evaluate_field(st, v, hfmm_b200.PREC_MIXED), hfmm_b200.evaluate_field(st, v)):
+            assert O.relative_error(x[n // 2:], y[n // 2:]) < 2e-6
+    st.close()
