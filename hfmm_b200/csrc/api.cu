@@ -256,6 +256,7 @@ void upload_level(hfmm_plan* P, int fam, int l, const double* const* h) {
     if (h[7] && l >= 3) relayout(h[7], 8, none, n_s, ld, true, T.l2l);
     else T.l2l.release();
     relayout(h[8], N_DISP, nonadjacent_map(), n_s, ld, true, T.m2l);
+    T.m2l_scale = table_scale(T.m2l.p, (int64_t)T.m2l.n / ld, ld);
     T.set = true;
 }
 
@@ -1001,6 +1002,8 @@ int hfmm_plan_set_kernel(hfmm_plan* P, double k, int32_t p, int32_t n_families,
     P->n_fam = n_families;
     for (int f = 0; f < 2; ++f)
         for (int l = 0; l < MAX_LEVELS; ++l) P->tables[f][l].reset();
+    P->surf_r = 0.0;
+    for (int j = 0; j < 3 * P->n_s; ++j) P->surf_r = std::max(P->surf_r, std::fabs(equiv_pts[j]));
     std::vector<double> soa(3 * P->n_s);
     for (int which = 0; which < 2; ++which) {
         const double* src = which == 0 ? equiv_pts : check_pts;

@@ -210,13 +210,7 @@ int hfmm_plan_set_m2l_compressed(hfmm_plan* P, int32_t family, int32_t level, in
         T.c_cmp.alloc((size_t)P->ld * ckld);
         T.c_exp.alloc((size_t)cmld * P->ld);
         T.c_s.alloc(2 * (size_t)N_M2L * cmld * ckld);
-        DevBuf<unsigned long long> most;
-        most.alloc(1);
-        most.zero();
-        absmax(C_dev, (int64_t)N_M2L * rank, rank, 1, most.p, 0);
-        unsigned long long h_most = 0;
-        HFMM_CUDA(cudaMemcpy(&h_most, most.p, sizeof(h_most), cudaMemcpyDeviceToHost));
-        T.c_scale = plane_scale(h_most);
+        T.c_scale = table_scale(C_dev, (int64_t)N_M2L * rank, rank);
         HFMM_LAUNCH(k_pack_cmp, dim3((unsigned)ceil_div(ckld, 128), (unsigned)P->ld), 128, 0, 0,
                     U_dev, P->n_s, rank, P->ld, ckld, T.c_cmp.p);
         HFMM_LAUNCH(k_pack_exp, dim3((unsigned)ceil_div(P->ld, 128), (unsigned)cmld), 128, 0, 0,

@@ -101,6 +101,7 @@ struct LevelTables {
     DevBuf<double> m2l;                 // 316 x (A^T), non-adjacent displacements (host-given,
                                         // or where the convolution does not apply)
     bool host_m2l = false;
+    double m2l_scale = 1.0;             // of the planes of host-given matrices
     // rotation-based M2L (m2l_rotation.cu): multipole-from-equivalent Q, check-from-local
     // E (complex, interleaved) and the coaxial shift matrices of every distance
     DevBuf<double> rot_Q, rot_E, rot_C;
@@ -203,6 +204,7 @@ struct hfmm_plan {
     // kernel + tables
     double k = 0;
     int p = 0, n_s = 0, ld = 0, n_fam = 0;
+    double surf_r = 0.0;   // the equivalent surface's largest coordinate, in half-sides
     hfmm::DevBuf<double> equiv_pts, check_pts;   // unit surfaces, 3 x n_s SoA
     hfmm::LevelTables tables[2][hfmm::MAX_LEVELS];   // [family][level]
 

@@ -525,6 +525,16 @@ void absmax(const double* src, int64_t rows, int ld, int R, unsigned long long* 
                 most);
 }
 
+double table_scale(const double* table, int64_t rows, int ld) {
+    DevBuf<unsigned long long> most;
+    most.alloc(2);
+    most.zero();
+    absmax(table, rows, ld, 1, most.p, 0);
+    unsigned long long h = 0;
+    HFMM_CUDA(cudaMemcpy(&h, most.p, sizeof(h), cudaMemcpyDeviceToHost));
+    return plane_scale(h);
+}
+
 void split_planes_grid(const double* src, const unsigned long long* most, const uint64_t* m_id, int64_t n_boxes,
                        int G, int ckld, uint16_t* out, cudaStream_t s) {
     const int64_t n = n_boxes * ckld;   // pairs

@@ -102,6 +102,7 @@ void make_grid_maps(CUtensorMap (&map)[2], const uint16_t* base, int valid, int 
 void split_planes(const double* src, const unsigned long long* most, uint16_t* out, int64_t plane, int64_t rows,
                   int ld, int R, cudaStream_t s);
 void absmax(const double* src, int64_t rows, int ld, int R, unsigned long long* most, cudaStream_t s);
+double table_scale(const double* table, int64_t rows, int ld);   // plane_scale of the largest entry
 // a complete level's densities [box][2][ckld] (boxes in level order from m_id) -> planes of
 // the dense grid [x][y][z][2][ckld] of side G
 void split_planes_grid(const double* src, const unsigned long long* most, const uint64_t* m_id, int64_t n_boxes,

@@ -153,10 +153,13 @@ size_t stream_ws_bytes(const hfmm_plan* P) {
     return (size_t)P->n_fam * 316 * (size_t)P->ld * P->ld * sizeof(double);
 }
 
-// Scale of a level's M2L planes, from the largest entry there can be: the kernel at the least
-// distance of the surfaces of two boxes of the V list, 1.9 half-sides (|sin(kr)| / r: k at most).
+// Scale of a level's M2L planes. Tables given by the host: measured when they were uploaded.
+// Generated ones: from the largest entry there can be, the kernel at the least distance of the
+// surfaces of two boxes of the V list (1.9 half-sides at radius 1.05; |sin(kr)| / r: k at most).
 double m2l_scale(const hfmm_plan* P, int fam, int level) {
-    const double r = 1.9 * P->extent * std::ldexp(1.0, -(level + 1));
+    const LevelTables& T = P->tables[fam][level];
+    if (T.host_m2l) return T.m2l_scale;
+    const double r = std::max(4.0 - 2.0 * P->surf_r, 1e-3) * P->extent * std::ldexp(1.0, -(level + 1));
     double most = 1.0 / r;
     if (P->yukawa) most *= std::exp(-P->k * r) / (4.0 * M_PI);
     else if (fam == 1) most = std::min(most, std::fabs(P->k));

@@ -29,3 +29,20 @@ def test_weak_cluster(kappa, eps):
         for x, y in zip(hfmm_b200.evaluate_field(st, v, hfmm_b200.PREC_MIXED), hfmm_b200.evaluate_field(st, v)):
             assert O.relative_error(x[n // 2:], y[n // 2:]) < 2e-6
     st.close()
+
+
+@pytest.mark.parametrize("p", [5, 6])
+@pytest.mark.parametrize("shift", [-40, 0, 3, 20])
+def test_scaled_host_tables(monkeypatch, p, shift):
+    """M2L tables given by the host are used as given, whatever their size: with every entry
+    times 2^shift (and the other tables as they are) mixed still follows FP64 on the same plan."""
+    import hfmm_b200
+    from cases import complex_uniform
+    tables = hfmm_b200.level_tables
+    monkeypatch.setattr(hfmm_b200, "level_tables",
+                        lambda *a, **k: dict(tables(*a, **k), M2L_K=tables(*a, **k)["M2L_K"] * 2.0 ** shift))
+    pos, q = complex_uniform(6000)
+    st = hfmm_b200.setup(pos, 5.0, p=p, N_max=24, tables="host")
+    for x, y in zip(hfmm_b200.evaluate_field(st, q, hfmm_b200.PREC_MIXED), hfmm_b200.evaluate_field(st, q)):
+        assert np.isfinite(x).all() and O.relative_error(x, y) < 2e-6
+    st.close()
