@@ -69,8 +69,9 @@ __global__ void __launch_bounds__(DT, 5) k_direct_partial(const double* __restri
         if (!act) continue;
         const int np = (int)((hi - p0 < DSTAGE) ? hi - p0 : DSTAGE);
         // The staged sources into sums of their own, so that a stage with a separation outside
-        // [1e-290, 1e290] or a phase over 1e5 (judged by r2's high word) is done over in the
-        // general form; a coincident source counts as one at zero charge.
+        // [1e-290, 1e290] (a NaN among them) or a phase over 1e5 (judged by r2's high word) is
+        // done over in the general form; a coincident source counts as one at zero charge there,
+        // and a separation that is no number is left out.
         double part[NA];
         bool odd = false;
         auto sources = [&](auto fast) {
@@ -80,7 +81,8 @@ __global__ void __launch_bounds__(DT, 5) k_direct_partial(const double* __restri
             for (int i = 0; i < np; ++i) {
                 const double dx = x - sx[i], dy = y - sy[i], dz = z - sz[i];
                 const double r2 = dx * dx + dy * dy + dz * dz;
-                const bool far = r2 > 0.0;
+                if (!decltype(fast)::value && !(r2 >= 0.0)) continue;
+                const bool far = r2 != 0.0;
                 double q[NF][R];
 #pragma unroll
                 for (int f = 0; f < NF; ++f)

@@ -35,3 +35,27 @@ def test_single_source(k):
     err = np.abs(E - f[:, None] * x).max(1) * r ** 2 / (1 + np.abs(kr))
     assert (err < 2 * tol).all()
     st.close()
+
+
+@pytest.mark.parametrize("kappa", [None, 2.0])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_referee_leaves_out_nan_points(cplx, kappa):
+    """A source whose position is no number has no distance to the target and adds nothing:
+    the sums are those without it, to the rounding of another summation order (2 eps a source)."""
+    import torch
+    import hfmm_b200
+    from hfmm_b200.kernels import yukawa
+    rng = np.random.default_rng(9)
+    n = 700
+    pos, q = rng.uniform(size=(n, 3)), rng.normal(size=n) + (1j * rng.normal(size=n) if cplx else 0.0)
+    st = hfmm_b200.setup(pos, 2.0, p=3, N_max=64) if kappa is None else hfmm_b200.kernel_setup(pos, yukawa(kappa), p=3)
+    out = []
+    for bad in (0.0, np.nan):
+        x, c = pos.copy(), q.copy()
+        x[[100, 650], 1] += bad
+        c[[100, 650]] = 0.0
+        st.positions = torch.as_tensor(x).cuda()   # the referee reads them from the state
+        out.append(hfmm_b200.direct(st, c, np.arange(20), field=True))
+    for a, b in zip(*out):
+        assert np.isfinite(b).all() and np.abs(a - b).max() <= 2 * n * EPS * np.abs(a).max()
+    st.close()
