@@ -11,6 +11,7 @@ struct EvalView {
     int yukawa;                // 0: Helmholtz (two families); 1: exp(-kappa r) / (4 pi r)
     int fast;                  // Helmholtz with two families, every phase k r under 1e5 and the
                                // domain's size in [1e-100, 1e100]: pair64's FAST form
+    int root;                  // phases so large that the near field takes pair64's ROOT form
     const double* pos_s;       // 3 x n, leaf-major sorted
     const float* pos_f;        // 6 x n: FP32 hi parts x|y|z, then lo parts (pos = hi + lo)
     const double* q_s;         // R x n, leaf-major sorted
@@ -162,12 +163,22 @@ __device__ __forceinline__ int p2p_lanes(int cnt) {
 
 // One FP64 pair at separation (dx, dy, dz), r2 > 0, into the sums. FAST: a Helmholtz phase
 // under 1e5 and r2 in [1e-290, 1e290], without a branch; else any kernel and any values.
-template <int NF, int R, bool FIELD, bool FAST>
+// ROOT: r to the last bit, one Newton step on from r2 / sqrt(r2), for large phases k r.
+template <int NF, int R, bool FIELD, bool FAST, bool ROOT = false>
 __device__ __forceinline__ void pair64(int yukawa, double k, double dx, double dy, double dz, double r2,
                                        const double (&d)[NF][R],
                                        double (&acc)[PairSums<NF, R, FIELD>::N]) {
     constexpr int NC = PairSums<NF, R, FIELD>::NC;
-    const double ir = FAST ? rsqrt_normal(r2) : rsqrt(r2), kr = k * (r2 * ir);
+    double ir, r;
+    if (ROOT && !FAST && !(r2 > 1e-290 && r2 < 1e290)) {
+        r = sqrt(r2);
+        ir = 1.0 / r;
+    } else {
+        ir = FAST ? rsqrt_normal(r2) : rsqrt(r2);
+        r = r2 * ir;
+        if (ROOT) r = fma(fma(-r, r, r2), 0.5 * ir, r);
+    }
+    const double kr = k * r;
     double sn, cs;
     if (FAST) sincos_reduced64(kr, &sn, &cs);
     else kernel_pair64(yukawa, kr, &sn, &cs);

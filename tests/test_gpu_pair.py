@@ -59,3 +59,36 @@ def test_referee_leaves_out_nan_points(cplx, kappa):
     for a, b in zip(*out):
         assert np.isfinite(b).all() and np.abs(a - b).max() <= 2 * n * EPS * np.abs(a).max()
     st.close()
+
+
+@pytest.mark.parametrize("k", [0.5, 24.0, 26.0, 400.0, 6000.0])
+def test_near_field_accuracy(k):
+    """The FP64 near field of one box against extended precision, on points of a lattice of
+    spacing 2^-10, whose squared distances are exact. The phase then carries one rounding of r
+    and one of k r: the bar is the error that these two alone make (10 % for the spread of four
+    clouds' mean) and four eps for the weights and sums. A third rounding in r is over it where
+    k is large."""
+    import hfmm_b200
+    errs, bars = [], []
+    for seed in range(4):
+        rng = np.random.default_rng([seed, 3])
+        n = 1000
+        pos, q = rng.integers(0, 1024, (n, 3)) / 1024.0, rng.normal(size=n) + 1j * rng.normal(size=n)
+        pos[0], pos[-1] = 0.0, 1.0   # extent 1: the kernel's form changes at k = 25
+        st = hfmm_b200.setup(pos, k, p=3, N_max=n, max_depth=1)
+        phi = hfmm_b200.evaluate_field(st, q)[0]
+        st.close()
+
+        def total(r, kr):
+            w = np.exp(1j * kr.astype(np.longdouble)) / r.astype(np.longdouble)
+            np.fill_diagonal(w, 0)
+            return w @ q.astype(np.clongdouble)
+        d = pos[:, None] - pos[None]
+        d2 = (d.astype(np.longdouble) ** 2).sum(-1)
+        np.fill_diagonal(d2, 1)
+        exact = total(np.sqrt(d2), np.longdouble(k) * np.sqrt(d2))
+        r = np.sqrt(d2).astype(np.float64)
+        rounded = total(np.sqrt(d2), k * r)
+        errs.append(float(np.linalg.norm(phi - exact) / np.linalg.norm(exact)))
+        bars.append(float(np.linalg.norm(rounded - exact) / np.linalg.norm(exact)))
+    assert np.mean(errs) < 1.1 * np.mean(bars) + 4 * EPS
