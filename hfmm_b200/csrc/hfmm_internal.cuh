@@ -41,6 +41,15 @@ extern std::atomic<int64_t> g_launches;
                                                  cudaGetErrorString(_e)};                \
     } while (0)
 
+// Dynamic shared memory a CTA may have, and a kernel's permission to use all of it. The limit is
+// the kernel's, one for the whole process: set to a call's own size, another thread's call could
+// lower it between this one's setting and its launch, which is then refused.
+constexpr size_t SMEM_MAX = 227 * 1024;
+template <typename Kernel>
+void allow_smem(Kernel kern, size_t static_bytes = 0) {
+    HFMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_MAX - static_bytes)));
+}
+
 // Device error flag bits (kernels OR these into plan->d_err).
 enum : int {
     ERRF_BOUNDS = 1,      // an index left its buffer (access skipped)

@@ -575,7 +575,6 @@ size_t transform_smem(int p, int n_s, int R, int CH, int nky) {
            (size_t)n_s * CH * R * sizeof(double) + (size_t)n_s * sizeof(int);
 }
 
-constexpr size_t SMEM_MAX = 227 * 1024;
 // The transforms' working set when the plan owns it: chunks of whole planes up to this
 // size (1e6 points, p = 8: 8 GiB of spectra in all, four chunks; larger chunks measured
 // the same, smaller ones add launches)
@@ -801,8 +800,8 @@ void conv_m2l(hfmm_plan* P, int R, int64_t fam_stride, cudaStream_t s) {
         default: fwd = R == 2 ? k_conv_fwd<2, 0> : k_conv_fwd<1, 0>; break;
     }
     const Kernel inv = R == 2 ? k_conv_inv<2> : k_conv_inv<1>;
-    HFMM_CUDA(cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    HFMM_CUDA(cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_i));
+    allow_smem(fwd);
+    allow_smem(inv);
     auto mul = C.half ? k_conv_mul<true> : k_conv_mul<false>;
     for (int f = 0; f < n_seq; f += nf) {
         c.dens = P->equiv.p + f * c.seq_stride;

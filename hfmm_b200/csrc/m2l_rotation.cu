@@ -339,15 +339,14 @@ void rot_m2l(hfmm_plan* P, int l, int R, int64_t fam_stride, cudaStream_t s) {
         if (nbl == 0) continue;
         c.TT = ROT_MAXCOL / R;
         const size_t smem_mp = (size_t)c.TT * R * P->n_s * sizeof(double);
-        HFMM_CUDA(cudaFuncSetAttribute(k_rot_multipole, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem_mp));
+        allow_smem(k_rot_multipole);
         HFMM_LAUNCH(k_rot_multipole, (unsigned)ceil_div(nbl, (int64_t)c.TT), ROT_MP_THREADS, smem_mp, s, c);
         c.TT = TT;
         // X and Y, then the m-major row table (int16) rounded up to 16 bytes
         const size_t smem = (size_t)2 * NC * TT * R * sizeof(double2) + (size_t)ceil_div(NC * 2, 16) * 16;
         const unsigned grid = (unsigned)ceil_div(nbl, (int64_t)TT);
         auto launch = [&](auto kern) {
-            HFMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            allow_smem(kern, ROT_MAXCOL * sizeof(int32_t));
             HFMM_LAUNCH(kern, grid, ROT_THREADS, smem, s, c);
         };
         switch (rows) {

@@ -185,7 +185,7 @@ void sample_pass(const float* P, const float* X, const float* T, int n, int in, 
                  float* Y, Work* w, cudaStream_t s) {
     const Offs o = offsets(in, out);
     const int smem = o.total * (int)sizeof(float);
-    HFMM_CUDA(cudaFuncSetAttribute(k_mlp_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    allow_smem(k_mlp_sample);
     HFMM_LAUNCH(k_mlp_sample, (unsigned)ceil_div(n, 64), 64, (size_t)smem, s, P, X, T, n, in, out, Y,
                 w ? w->act.p : nullptr, w ? w->dlt.p : nullptr, w ? w->gout.p : nullptr,
                 w ? w->sq.p : nullptr);

@@ -344,7 +344,7 @@ void particles_impl(const ParticlePass& p, cudaStream_t s) {
         case ParticleOp::M2P: {
             size_t smem = (size_t)(NF * R + 3) * v.n_s * sizeof(double);
             auto kern = k_particles_from_surface<NF, R, FIELD, FAST>;
-            HFMM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            allow_smem(kern);
             // M2P, and L2P of few leaves (under two waves of CTAs): the chunks of a leaf in CTAs
             // of their own, up to eight. L2P of many leaves: one CTA a leaf, which then loads its
             // densities once (1e6 points, p = 8: 1.56 against 1.80 ms; 512 leaves: 63 against 51 us)
