@@ -866,6 +866,7 @@ int hfmm_tree_build(const double* pos_dev, int64_t n, int32_t n_max, int32_t max
     hfmm_plan* P = new hfmm_plan();
     dev_plan_count(1);
     API_BEGIN
+    KeepBlocks keep;
     HFMM_CUDA(cudaGetDevice(&P->device));
     require_device_ptr(pos_dev, "positions");
     P->n = n;
@@ -904,6 +905,7 @@ int hfmm_tree_build_in_domain(const double* pos_dev, int64_t n, int32_t n_max, i
     hfmm_plan* P = new hfmm_plan();
     dev_plan_count(1);
     API_BEGIN
+    KeepBlocks keep;
     HFMM_CUDA(cudaGetDevice(&P->device));
     require_device_ptr(pos_dev, "positions");
     P->n = n;
@@ -938,6 +940,7 @@ int hfmm_plan_rebuild(hfmm_plan* P, const double* pos_dev) {
     if (P->batch_owner) return fail(HFMM_ERR_STATE, "the plan belongs to a batch (its graph holds the old tree)");
     if (!pos_dev) return fail(HFMM_ERR_ARG, "positions are NULL");
     API_BEGIN
+    KeepBlocks keep;
     require_device_ptr(pos_dev, "positions");
     HFMM_CUDA(cudaDeviceSynchronize());   // no evaluate of the old tree in flight
     tree_build(P, pos_dev);               // checks the domain before it changes anything
@@ -1074,6 +1077,7 @@ int hfmm_plan_set_level(hfmm_plan* P, int32_t family, int32_t level, const doubl
     if (level < P->md && !M2M_K) return fail(HFMM_ERR_ARG, "M2M_K required below max_depth");
     if (level >= 3 && !L2L_K) return fail(HFMM_ERR_ARG, "L2L_K required from level 3");
     API_BEGIN
+    KeepBlocks keep;
     const double* h[9] = {F_up_U, F_up_d, F_up_Vt, F_dn_U, F_dn_d, F_dn_Vt, M2M_K, L2L_K, M2L_K};
     upload_level(P, family, level, h);
     P->finalized = false;
@@ -1091,6 +1095,7 @@ int hfmm_plan_set_level_decode(hfmm_plan* P, int32_t family, int32_t level, cons
     if (!F_up_U || !F_up_d || !F_up_Vt || !F_dn_U || !F_dn_d || !F_dn_Vt)
         return fail(HFMM_ERR_ARG, "decode factors are required");
     API_BEGIN
+    KeepBlocks keep;
     const double* h[9] = {F_up_U, F_up_d, F_up_Vt, F_dn_U, F_dn_d, F_dn_Vt, nullptr, nullptr, nullptr};
     upload_level(P, family, level, h);
     P->finalized = false;
@@ -1107,6 +1112,7 @@ int hfmm_plan_finalize(hfmm_plan* P) {
                 return fail(HFMM_ERR_STATE, "tables missing for family " + std::to_string(f) +
                                                 " level " + std::to_string(l));
     API_BEGIN
+    KeepBlocks keep;
     if (!P->V.p) {
         lists_build(P);
         schedules_build(P);
@@ -1453,6 +1459,8 @@ int hfmm_direct_kernel(int32_t kind, const double* pos, const double* q_re, cons
     int h = 0;
     HFMM_CUDA(cudaMemcpyAsync(&h, err.p, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     HFMM_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+    scratch.release(true);
+    err.release(true);
     if (h) return fail(HFMM_ERR_ARG, "target index out of range");
     return HFMM_OK;
     API_END

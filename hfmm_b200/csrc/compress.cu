@@ -198,6 +198,7 @@ int hfmm_plan_set_m2l_compressed(hfmm_plan* P, int32_t family, int32_t level, in
     if (rank < 1 || rank > P->n_s) return fail(HFMM_ERR_ARG, "rank must be in [1, n_s]");
     if (!U_dev || !C_dev) return fail(HFMM_ERR_ARG, "U and C are required");
     try {
+        KeepBlocks keep;
         require_device_ptr(U_dev, "U");
         require_device_ptr(C_dev, "C");
         LevelTables& T = P->tables[family][level];

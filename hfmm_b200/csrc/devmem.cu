@@ -1,10 +1,11 @@
 // Device memory blocks of the library (hfmm::DevBuf). A plan rebuilt for moved points makes
 // and drops about 160 buffers; a cudaMalloc and cudaFree pair of each took 26 of the 32 ms of
 // such a call at 1e5 points (90 us a call here, and milliseconds at times on a shared host).
-// A dropped block of at most MOST_BLOCK bytes is kept, up to MOST_KEPT bytes in all, and
-// serves the next allocation of its size class on its device. Keeping one first waits for the
-// device, as cudaFree does, so whoever gets it finds no kernel of any stream on it. Nothing
-// is kept while no plan is alive, and the last plan's end frees all of it.
+// A block of at most MOST_BLOCK bytes that is dropped idle, or inside a KeepBlocks scope, is
+// kept, up to MOST_KEPT bytes in all, and serves the next allocation of its size class on its
+// device. A scope's block is kept after a wait for the device, so whoever gets one finds no
+// kernel of any stream on it. Nothing is kept while no plan is alive, and the last plan's end
+// frees all of it.
 #include "hfmm_internal.cuh"
 
 #include <map>
@@ -41,7 +42,13 @@ void free_all() {   // with the lock held
     k.bytes = 0;
 }
 
+thread_local int t_keep = 0;
+
 }  // namespace
+
+KeepBlocks::KeepBlocks() { ++t_keep; }
+KeepBlocks::~KeepBlocks() { --t_keep; }
+bool keeping_blocks() { return t_keep > 0; }
 
 void* dev_alloc(size_t bytes, size_t* cap, int* device) {
     HFMM_CUDA(cudaGetDevice(device));
@@ -74,10 +81,10 @@ void* dev_alloc(size_t bytes, size_t* cap, int* device) {
     return p;
 }
 
-void dev_free(void* p, size_t cap, int device) noexcept {
+void dev_free(void* p, size_t cap, int device, bool idle) noexcept {
     Kept& k = kept();
     int now = -1;
-    if (cap <= MOST_BLOCK && cudaGetDevice(&now) == cudaSuccess && now == device) {
+    if (cap <= MOST_BLOCK && (idle || t_keep > 0) && cudaGetDevice(&now) == cudaSuccess && now == device) {
         bool keep;
         {
             std::lock_guard<std::mutex> g(k.mu);
@@ -85,7 +92,7 @@ void dev_free(void* p, size_t cap, int device) noexcept {
             if (keep) k.bytes += cap;   // reserved
         }
         if (keep) {
-            const bool idle = cudaDeviceSynchronize() == cudaSuccess;
+            if (!idle) idle = cudaDeviceSynchronize() == cudaSuccess;
             std::lock_guard<std::mutex> g(k.mu);
             if (idle && k.plans > 0) {
                 try {

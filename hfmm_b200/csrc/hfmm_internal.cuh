@@ -58,12 +58,23 @@ enum : int {
 };
 
 // ---------------------------------------------------------------- device memory
-// Blocks of device memory for DevBuf (devmem.cu). Like cudaFree, giving a block back waits
-// for the device, so no kernel on any stream still uses it; while plans are alive, blocks
-// are then kept for the next allocation of their size (a bounded amount per process).
+// Blocks of device memory for DevBuf (devmem.cu). While plans are alive, blocks given back are
+// kept for the next allocation of their size (a bounded amount per process), where it is known
+// that no kernel of any stream uses them any more: the caller says so (idle), or it works inside
+// a KeepBlocks scope, which allows waiting for the device first. Everywhere else a block goes to
+// cudaFree at once: a wait for the device would break a stream capture of any other thread.
 void* dev_alloc(size_t bytes, size_t* cap, int* device);
-void dev_free(void* p, size_t cap, int device) noexcept;
+void dev_free(void* p, size_t cap, int device, bool idle) noexcept;
 void dev_plan_count(int change);   // plans alive; the last one gives every kept block back
+bool keeping_blocks();             // this thread is inside a KeepBlocks scope
+
+// For calls that build or rebuild a plan, which wait for the device anyway
+struct KeepBlocks {
+    KeepBlocks();
+    ~KeepBlocks();
+    KeepBlocks(const KeepBlocks&) = delete;
+    KeepBlocks& operator=(const KeepBlocks&) = delete;
+};
 
 template <typename T>
 struct DevBuf {
@@ -79,7 +90,7 @@ struct DevBuf {
     void alloc(size_t count) {
         if (count == 0) count = 1;
         const size_t bytes = count * sizeof(T);
-        if (p && cap >= bytes && cap / 4 <= bytes) {
+        if (p && keeping_blocks() && cap >= bytes && cap / 4 <= bytes) {
             HFMM_CUDA(cudaDeviceSynchronize());   // earlier users of the block
         } else {
             release();
@@ -88,8 +99,8 @@ struct DevBuf {
         n = count;
     }
     void zero(cudaStream_t s = 0) { HFMM_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s)); }
-    void release() {
-        if (p) dev_free(p, cap, device);
+    void release(bool idle = false) {   // idle: whatever used the block has been waited for
+        if (p) dev_free(p, cap, device, idle);
         p = nullptr;
         n = cap = 0;
     }

@@ -195,6 +195,7 @@ double read_loss(Work& w, int n, int out, cudaStream_t s) {
     std::vector<float> sq(n);
     HFMM_CUDA(cudaMemcpyAsync(sq.data(), w.sq.p, n * sizeof(float), cudaMemcpyDeviceToHost, s));
     HFMM_CUDA(cudaStreamSynchronize(s));
+    for (auto* b : {&w.Y, &w.act, &w.dlt, &w.gout, &w.sq, &w.G}) b->release(true);
     double loss = 0.0;
     for (float v : sq) loss += v;
     return loss / ((double)n * out);

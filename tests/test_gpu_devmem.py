@@ -43,3 +43,44 @@ def test_threads_share_blocks():
             assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
     torch.cuda.synchronize()
     assert torch.cuda.mem_get_info()[0] > before - (64 << 20)
+
+
+@pytest.mark.parametrize("mode", ["thread_local", "relaxed"])
+@pytest.mark.parametrize("what", ["close", "direct"])
+def test_other_threads_capture(mode, what):
+    """A plan closed, or a direct sum run, on one thread leaves a stream capture of another
+    thread whole (in the modes that let other threads allocate and free): the captured evaluate
+    gives the same bits."""
+    import torch
+    import hfmm_b200
+    pos, q = complex_uniform(3000)
+    a = hfmm_b200.setup(pos, 3.0, p=4, N_max=48)
+    b = hfmm_b200.setup(pos, 2.0, p=4, N_max=48)
+    tg = np.arange(50)
+    hfmm_b200.direct(b, q, tg)
+    qd = torch.as_tensor(q.real.copy()).cuda()
+    phi = torch.empty(len(q), dtype=torch.complex128, device="cuda")
+    hfmm_b200.evaluate_into(a, qd, None, phi)
+    want = phi.cpu().numpy()
+    # the direct sum's own stream and inputs, so that torch allocates nothing in the capture
+    side = torch.cuda.Stream()
+    tgd = torch.as_tensor(tg.astype(np.int32)).cuda()
+    with torch.cuda.stream(side):
+        hfmm_b200.direct_at(b, qd, None, tgd, stream=side)
+    torch.cuda.synchronize()
+
+    def other():
+        with torch.cuda.stream(side):
+            b.close() if what == "close" else hfmm_b200.direct_at(b, qd, None, tgd, stream=side)
+
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode=mode):
+        hfmm_b200.evaluate_into(a, qd, None, phi)
+        t = threading.Thread(target=other)
+        t.start()
+        t.join()
+    phi.zero_()
+    graph.replay()
+    assert np.array_equal(phi.cpu().numpy(), want)
+    a.close()
+    b.close()
