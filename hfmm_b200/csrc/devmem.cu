@@ -85,23 +85,22 @@ void dev_free(void* p, size_t cap, int device, bool idle) noexcept {
     Kept& k = kept();
     int now = -1;
     if (cap <= MOST_BLOCK && (idle || t_keep > 0) && cudaGetDevice(&now) == cudaSuccess && now == device) {
-        bool keep;
-        {
-            std::lock_guard<std::mutex> g(k.mu);
-            keep = k.plans > 0 && k.bytes + cap <= MOST_KEPT;
-            if (keep) k.bytes += cap;   // reserved
+        // what is counted is what is in the store: the lock is open during the wait, and another
+        // thread may empty the store meanwhile
+        auto room = [&] { return k.plans > 0 && k.bytes + cap <= MOST_KEPT; };
+        std::unique_lock<std::mutex> g(k.mu);
+        if (room() && !idle) {
+            g.unlock();
+            idle = cudaDeviceSynchronize() == cudaSuccess;
+            g.lock();
         }
-        if (keep) {
-            if (!idle) idle = cudaDeviceSynchronize() == cudaSuccess;
-            std::lock_guard<std::mutex> g(k.mu);
-            if (idle && k.plans > 0) {
-                try {
-                    k.blocks.emplace(std::make_pair(device, cap), p);
-                    return;
-                } catch (...) {
-                }
+        if (idle && room()) {
+            try {
+                k.blocks.emplace(std::make_pair(device, cap), p);
+                k.bytes += cap;
+                return;
+            } catch (...) {
             }
-            k.bytes -= cap;
         }
     }
     cudaFree(p);
