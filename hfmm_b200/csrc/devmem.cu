@@ -28,8 +28,10 @@ Kept& kept() {
     return *k;
 }
 
-// eight classes an octave, 512 bytes at least
+// eight classes an octave, 512 bytes at least; a block too large to be kept has its own size
+// (rounded up it could be what no longer fits the device)
 size_t size_class(size_t bytes) {
+    if (bytes > MOST_BLOCK) return bytes;
     size_t step = 512;
     while (step * 16 < bytes) step *= 2;
     return (bytes + step - 1) / step * step;

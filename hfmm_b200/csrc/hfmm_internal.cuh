@@ -86,11 +86,12 @@ struct DevBuf {
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
-    // contents are undefined, also where the block at hand is large enough and stays
+    // contents are undefined, also where the block at hand is large enough (and no more than a
+    // quarter larger) and stays
     void alloc(size_t count) {
         if (count == 0) count = 1;
         const size_t bytes = count * sizeof(T);
-        if (p && keeping_blocks() && cap >= bytes && cap / 4 <= bytes) {
+        if (p && keeping_blocks() && cap >= bytes && cap - bytes <= bytes / 4 + 512) {
             HFMM_CUDA(cudaDeviceSynchronize());   // earlier users of the block
         } else {
             release();

@@ -60,6 +60,14 @@ extern "C" void* take(size_t n, size_t* cap) {
     int dev;
     return hfmm::dev_alloc(n, cap, &dev);
 }
+// cap of a DevBuf of `first` bytes after a second alloc of `second` bytes
+extern "C" size_t resized(size_t first, size_t second) {
+    hfmm::KeepBlocks keep;
+    hfmm::DevBuf<char> b;
+    b.alloc(first);
+    b.alloc(second);
+    return b.cap;
+}
 extern "C" void give(void* p, size_t cap, int scope) {   // scope: inside a KeepBlocks
     if (scope) {
         hfmm::KeepBlocks keep;
@@ -85,7 +93,8 @@ def lib(tmp_path_factory):
     so.take.restype = ctypes.c_void_p
     so.take.argtypes = [ctypes.c_size_t, ctypes.POINTER(ctypes.c_size_t)]
     so.give.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int]
-    so.live.restype = ctypes.c_size_t
+    so.live.restype = so.resized.restype = ctypes.c_size_t
+    so.resized.argtypes = [ctypes.c_size_t, ctypes.c_size_t]
     return so
 
 
@@ -125,3 +134,26 @@ def test_outside_a_scope_nothing_is_kept(lib):
     assert lib.live() == 0
     lib.in_wait(0)
     lib.plans(-1)
+
+
+@pytest.mark.parametrize("n", [1, 513, MIB - 1, 31 * MIB + 5, 32 * MIB + 1, 33 * MIB + 7, 3 << 30, (5 << 30) + 12345])
+def test_block_sizes(lib, n):
+    """A block that may be kept is rounded up by an eighth (512 bytes) at most, a larger one not
+    at all, so that a plan near the device's memory takes what its buffers hold."""
+    lib.plans(1)
+    p, cap = _take(lib, n)
+    before = lib.live()
+    assert n <= cap <= (n + max(n // 8, 512) if n <= 32 * MIB else n) and before >= cap
+    lib.give(p, cap, 0)
+    lib.plans(-1)
+    assert lib.live() == 0
+
+
+@pytest.mark.parametrize("second", [100 * MIB, 99 * MIB, 81 * MIB, 79 * MIB, 26 * MIB, MIB, 101 * MIB])
+def test_resized_buffer(lib, second):
+    """A buffer asked for less keeps its block only while that is at most a quarter larger."""
+    lib.plans(1)
+    cap = lib.resized(100 * MIB, second)
+    assert second <= cap <= second + second // 4 + 512
+    lib.plans(-1)
+    assert lib.live() == 0
