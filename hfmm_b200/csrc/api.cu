@@ -1202,6 +1202,7 @@ int hfmm_plan_finalize(hfmm_plan* P) {
     P->q_max.alloc(2);
     P->pot.alloc((size_t)2 * P->n);       // real and imaginary part per particle
     P->fld.alloc((size_t)2 * 3 * P->n);
+    conv_workspace(P);
     HFMM_CUDA(cudaDeviceSynchronize());
     P->finalized = true;
     return HFMM_OK;

@@ -99,6 +99,18 @@ struct DevBuf {
         }
         n = count;
     }
+    // `most` values, or as many of their halves, down to `least`, as the device has room for
+    void alloc_between(size_t least, size_t most) {
+        for (size_t count = most;; count = count / 2 > least ? count / 2 : least) {
+            try {
+                alloc(count);
+                return;
+            } catch (const Error&) {
+                if (count <= least) throw;
+                cudaGetLastError();
+            }
+        }
+    }
     void zero(cudaStream_t s = 0) { HFMM_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s)); }
     void release(bool idle = false) {   // idle: whatever used the block has been waited for
         if (p) dev_free(p, cap, device, idle);
@@ -317,6 +329,7 @@ double m2l_scale(const hfmm_plan* P, int fam, int level);
 bool conv_surface(hfmm_plan* P, const double* equiv);
 void conv_tables(hfmm_plan* P);
 void conv_schedule(hfmm_plan* P);
+void conv_workspace(hfmm_plan* P);
 bool conv_fits(const hfmm_plan* P);
 void conv_m2l(hfmm_plan* P, int R, int64_t fam_stride, cudaStream_t s);
 size_t stream_ws_bytes(const hfmm_plan* P);

@@ -681,7 +681,7 @@ void conv_tables(hfmm_plan* P) {
     C.tables = true;
 }
 
-// Slots, neighbour lists and groups of the current tree, and the plan's own workspace.
+// Slots, neighbour lists and groups of the current tree.
 void conv_schedule(hfmm_plan* P) {
     ConvPlan& C = P->conv;
     std::vector<int32_t> slot_of(P->nb, -1), child;
@@ -721,17 +721,24 @@ void conv_schedule(hfmm_plan* P) {
     HFMM_LAUNCH(k_conv_nbr, (unsigned)ceil_div((int64_t)n_slots * 26, 256), 256, 0, 0, C.child.p,
                 P->m2l_src.p, P->p_id.p, so.p, n_slots, C.nbr.p);
     HFMM_CUDA(cudaDeviceSynchronize());
-    if (!P->streamed) {
-        // X and Y of as many whole planes as the limit holds; where not one fits, the limit
-        // (one family or some rows of a plane at a time), one row of one family at least
-        const size_t row = 2 * (size_t)chunk_values(P, C.n, 1) * sizeof(double2);
-        const size_t plane = row * C.n * P->n_fam;
-        const size_t planes = std::min<size_t>(C.n, CONV_WS / plane);
-        const size_t want = (planes ? plane * planes : std::max(row, CONV_WS)) / sizeof(double);
-        if (C.ws.n < want) C.ws.alloc(want);
-    } else {
+}
+
+// The plan's own workspace (a streamed plan's is P->ws): X and Y of as many whole planes as the
+// limit holds; where not one fits, the limit (one family or some rows of a plane at a time).
+// Taken after every other buffer of the plan, and smaller where the device is nearly full, one
+// row of one family at least: chunks cost time (1e6 points, p = 4: 7.5 ms with 2 GiB, 9.4 with
+// 64 MiB), but a plan that otherwise fits is not refused for them.
+void conv_workspace(hfmm_plan* P) {
+    ConvPlan& C = P->conv;
+    if (!C.on || !C.n_slots || P->streamed) {
         C.ws.release();
+        return;
     }
+    const size_t row = 2 * (size_t)chunk_values(P, C.n, 1) * sizeof(double2);
+    const size_t plane = row * C.n * P->n_fam;
+    const size_t planes = std::min<size_t>(C.n, CONV_WS / plane);
+    const size_t want = (planes ? plane * planes : std::max(row, CONV_WS)) / sizeof(double);
+    if (C.ws.n < want) C.ws.alloc_between(row / sizeof(double), want);
 }
 
 bool conv_fits(const hfmm_plan* P) {   // a streamed plan's workspace must hold one row

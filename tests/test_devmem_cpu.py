@@ -68,6 +68,18 @@ extern "C" size_t resized(size_t first, size_t second) {
     b.alloc(second);
     return b.cap;
 }
+// bytes of a buffer of between `least` and `most`, the device full `times` times (0: refused)
+extern "C" size_t between(size_t least, size_t most, int times) {
+    hfmm::DevBuf<char> b;
+    g_fail = 2 * times;   // dev_alloc tries again once the store is empty
+    try {
+        b.alloc_between(least, most);
+    } catch (const hfmm::Error&) {
+        g_fail = 0;
+        return 0;
+    }
+    return b.n;
+}
 extern "C" void give(void* p, size_t cap, int scope) {   // scope: inside a KeepBlocks
     if (scope) {
         hfmm::KeepBlocks keep;
@@ -93,7 +105,8 @@ def lib(tmp_path_factory):
     so.take.restype = ctypes.c_void_p
     so.take.argtypes = [ctypes.c_size_t, ctypes.POINTER(ctypes.c_size_t)]
     so.give.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int]
-    so.live.restype = so.resized.restype = ctypes.c_size_t
+    so.live.restype = so.resized.restype = so.between.restype = ctypes.c_size_t
+    so.between.argtypes = [ctypes.c_size_t, ctypes.c_size_t, ctypes.c_int]
     so.resized.argtypes = [ctypes.c_size_t, ctypes.c_size_t]
     return so
 
@@ -155,5 +168,13 @@ def test_resized_buffer(lib, second):
     lib.plans(1)
     cap = lib.resized(100 * MIB, second)
     assert second <= cap <= second + second // 4 + 512
+    lib.plans(-1)
+    assert lib.live() == 0
+
+
+@pytest.mark.parametrize("times,n", [(0, 2048 * MIB), (1, 1024 * MIB), (3, 256 * MIB), (4, 200 * MIB), (5, 0)])
+def test_as_much_as_fits(lib, times, n):
+    lib.plans(1)
+    assert lib.between(200 * MIB, 2048 * MIB, times) == n and lib.between(7, 7, 0) == 7
     lib.plans(-1)
     assert lib.live() == 0
