@@ -184,8 +184,8 @@ __global__ void __launch_bounds__(L2P_THREADS) k_particles_from_surface(
 // ROOT (EvalView::root): the last bit of r matters where k r is large. One leaf of 1,200 points
 // in a unit cube, error of the potential without / with it / with sqrt and a division: k = 10
 // 7.4 / 7.0 / 9.6e-16, 30 1.30 / 1.11 / 1.31e-15, 100 3.92 / 3.26 / 3.33e-15, 1000 3.82 / 3.15 /
-// 3.15e-14; it costs 5 % of the smallest call and 0.8 % of 1e6 points, p = 8, so it runs from
-// k x extent = 25 on, and in the general form.
+// 3.15e-14; it costs 5 % of the smallest call and 0.8 % of 1e6 points, p = 8 (13 % of a call that
+// the general form's near field bounds), so it runs from k x extent = 25 on.
 constexpr int P2P_WARPS = 4;
 template <int NF, int R, bool FIELD, bool FAST, bool ROOT>
 __global__ void __launch_bounds__(32 * P2P_WARPS) k_p2p(EvalView v, const int32_t* __restrict__ leaves,
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(32 * P2P_WARPS) k_p2p(EvalView v, const int32_
                         for (int f = 0; f < NF; ++f)
 #pragma unroll
                             for (int r = 0; r < R; ++r) q[f][r] = far ? st[3 + r][k] : 0.0;
-                        pair64<NF, R, FIELD, F, !F || ROOT>(v.yukawa, v.k, dx, dy, dz, far ? d2 : 1.0, q, acc);
+                        pair64<NF, R, FIELD, F, ROOT>(v.yukawa, v.k, dx, dy, dz, far ? d2 : 1.0, q, acc);
                     }
                 };
                 if (FAST && thr >= 1e-290) sources(std::true_type());
@@ -355,8 +355,8 @@ void particles_impl(const ParticlePass& p, cudaStream_t s) {
             break;
         }
         case ParticleOp::P2P:
-            if (FAST && v.root)
-                HFMM_LAUNCH((k_p2p<NF, R, FIELD, FAST, FAST>), p.nrows, 32 * P2P_WARPS, 0, s, v, p.rows, p.off, p.srcs,
+            if (v.root)
+                HFMM_LAUNCH((k_p2p<NF, R, FIELD, FAST, true>), p.nrows, 32 * P2P_WARPS, 0, s, v, p.rows, p.off, p.srcs,
                             p.pot, p.fld);
             else
                 HFMM_LAUNCH((k_p2p<NF, R, FIELD, FAST, false>), p.nrows, 32 * P2P_WARPS, 0, s, v, p.rows, p.off, p.srcs,
