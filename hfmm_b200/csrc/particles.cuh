@@ -11,6 +11,8 @@ struct EvalView {
     int yukawa;                // 0: Helmholtz (two families); 1: exp(-kappa r) / (4 pi r)
     int fast;                  // Helmholtz with two families, every phase k r under 1e5 and the
                                // domain's size in [1e-100, 1e100]: pair64's FAST form
+    double own2;               // a squared distance that stands in for a coincident point's: the
+                               // domain's, whose phase is among those the forms are made for
     int root;                  // phases so large that the near field takes pair64's ROOT form
     const double* pos_s;       // 3 x n, leaf-major sorted
     const float* pos_f;        // 6 x n: FP32 hi parts x|y|z, then lo parts (pos = hi + lo)

@@ -92,3 +92,23 @@ def test_near_field_accuracy(k):
         errs.append(float(np.linalg.norm(phi - exact) / np.linalg.norm(exact)))
         bars.append(float(np.linalg.norm(rounded - exact) / np.linalg.norm(exact)))
     assert np.mean(errs) < 1.1 * np.mean(bars) + 4 * EPS
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("scale", [1e-90, 1e-60, 1e-12, 1.0, 1e12, 1e90])
+def test_any_unit_of_length(scale, cplx):
+    """The same problem in another unit of length, k times extent unchanged: phi and E scale by
+    1 / scale and 1 / scale^2. To 1e-9: the damped decodes' rounding, which the scaled tables
+    draw anew, amplified as in the parity tests at their loosest."""
+    import hfmm_b200
+    rng = np.random.default_rng(21)
+    n = 2000
+    pos, q = rng.uniform(size=(n, 3)), rng.normal(size=n) + (1j * rng.normal(size=n) if cplx else 0.0)
+    out = []
+    for s in (1.0, scale):
+        st = hfmm_b200.setup(pos * s, 3.0 / s, p=5, N_max=32)
+        phi, E = hfmm_b200.evaluate_field(st, q)
+        st.close()
+        out.append((phi * s, (E * s) * s))
+    for a, b in zip(*out):
+        assert np.isfinite(b).all() and np.linalg.norm(a - b) <= 1e-9 * np.linalg.norm(a)
