@@ -21,6 +21,7 @@
 #include <exception>
 #include <memory>
 #include <mutex>
+#include <optional>
 
 namespace hfmm {
 
@@ -1305,6 +1306,9 @@ int hfmm_plan_phase_times(hfmm_plan* P, double* ms) {
 void hfmm_plan_destroy(hfmm_plan* P) {
     if (!P) return;
     if (P->batch_owner) batch_forget_plan(P->batch_owner, P);
+    // the first buffer's cudaFree waits for the plan's work; the others can then be kept
+    std::optional<KeepBlocks> keep;
+    if (P->check.release_and_wait()) keep.emplace(true);
     drop_extra(P);
     delete[] static_cast<MixedMaps*>(P->mx_maps);
     P->mx_maps = nullptr;
@@ -1319,6 +1323,7 @@ void hfmm_plan_destroy(hfmm_plan* P) {
     if (P->nf_fork) cudaEventDestroy(P->nf_fork);
     if (P->nf_join) cudaEventDestroy(P->nf_join);
     delete P;
+    keep.reset();
     dev_plan_count(-1);
 }
 

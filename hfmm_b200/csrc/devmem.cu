@@ -44,12 +44,18 @@ void free_all() {   // with the lock held
     k.bytes = 0;
 }
 
-thread_local int t_keep = 0;
+thread_local int t_keep = 0, t_idle = 0;   // scopes, and those whose blocks are idle
 
 }  // namespace
 
-KeepBlocks::KeepBlocks() { ++t_keep; }
-KeepBlocks::~KeepBlocks() { --t_keep; }
+KeepBlocks::KeepBlocks(bool idle_) : idle(idle_) {
+    ++t_keep;
+    t_idle += idle;
+}
+KeepBlocks::~KeepBlocks() {
+    --t_keep;
+    t_idle -= idle;
+}
 bool keeping_blocks() { return t_keep > 0; }
 
 void* dev_alloc(size_t bytes, size_t* cap, int* device) {
@@ -86,6 +92,7 @@ void* dev_alloc(size_t bytes, size_t* cap, int* device) {
 void dev_free(void* p, size_t cap, int device, bool idle) noexcept {
     Kept& k = kept();
     int now = -1;
+    idle = idle || t_idle > 0;
     if (cap <= MOST_BLOCK && (idle || t_keep > 0) && cudaGetDevice(&now) == cudaSuccess && now == device) {
         // what is counted is what is in the store: the lock is open during the wait, and another
         // thread may empty the store meanwhile

@@ -61,17 +61,20 @@ enum : int {
 // Blocks of device memory for DevBuf (devmem.cu). While plans are alive, blocks given back are
 // kept for the next allocation of their size (a bounded amount per process), where it is known
 // that no kernel of any stream uses them any more: the caller says so (idle), or it works inside
-// a KeepBlocks scope, which allows waiting for the device first. Everywhere else a block goes to
-// cudaFree at once: a wait for the device would break a stream capture of any other thread.
+// a KeepBlocks scope, which allows waiting for the device first or knows that it is idle.
+// Everywhere else a block goes to cudaFree at once: cudaDeviceSynchronize would break a stream
+// capture of any other thread.
 void* dev_alloc(size_t bytes, size_t* cap, int* device);
 void dev_free(void* p, size_t cap, int device, bool idle) noexcept;
 void dev_plan_count(int change);   // plans alive; the last one gives every kept block back
 bool keeping_blocks();             // this thread is inside a KeepBlocks scope
 
-// For calls that build or rebuild a plan, which wait for the device anyway
+// For calls that build or rebuild a plan, which wait for the device anyway; idle: for the end of
+// a plan, whose work a first cudaFree has waited for
 struct KeepBlocks {
-    KeepBlocks();
+    explicit KeepBlocks(bool idle = false);
     ~KeepBlocks();
+    const bool idle;
     KeepBlocks(const KeepBlocks&) = delete;
     KeepBlocks& operator=(const KeepBlocks&) = delete;
 };
@@ -112,6 +115,14 @@ struct DevBuf {
         }
     }
     void zero(cudaStream_t s = 0) { HFMM_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s)); }
+    // Back to cudaFree, which waits for the work of every stream (also where a capture of another
+    // thread lets it pass, and cudaDeviceSynchronize would break that): true when it has
+    bool release_and_wait() {
+        const bool waited = p && cudaFree(p) == cudaSuccess;
+        p = nullptr;
+        n = cap = 0;
+        return waited;
+    }
     void release(bool idle = false) {   // idle: whatever used the block has been waited for
         if (p) dev_free(p, cap, device, idle);
         p = nullptr;

@@ -80,9 +80,9 @@ extern "C" size_t between(size_t least, size_t most, int times) {
     }
     return b.n;
 }
-extern "C" void give(void* p, size_t cap, int scope) {   // scope: inside a KeepBlocks
+extern "C" void give(void* p, size_t cap, int scope) {   // scope: 1 inside a KeepBlocks, 2 an idle one
     if (scope) {
-        hfmm::KeepBlocks keep;
+        hfmm::KeepBlocks keep(scope == 2);
         hfmm::dev_free(p, cap, 0, false);
     } else {
         hfmm::dev_free(p, cap, 0, false);
@@ -135,6 +135,17 @@ def test_bound_holds_across_threads(lib, what):
     assert lib.allocs() == n
     for p, cap in again:
         lib.give(p, cap, 1)
+    lib.plans(-1)
+    assert lib.live() == 0
+
+
+def test_idle_scope_keeps_without_a_wait(lib):
+    lib.plans(1)
+    p, cap = _take(lib, MIB)
+    lib.in_wait(1)   # would end the plan, and with it the block, if the device were waited for
+    lib.give(p, cap, 2)
+    assert lib.live() == cap
+    lib.in_wait(0)
     lib.plans(-1)
     assert lib.live() == 0
 

@@ -84,3 +84,31 @@ def test_other_threads_capture(mode, what):
     assert np.array_equal(phi.cpu().numpy(), want)
     a.close()
     b.close()
+
+
+def test_plan_closed_while_it_runs():
+    """A plan closed with evaluates still in flight: they finish on its own memory, which only
+    then serves the plans built after it."""
+    import torch
+    import hfmm_b200
+    pos, q = complex_uniform(60000)
+    small = hfmm_b200.setup(pos[:4000], 2.0, p=4, N_max=24)   # keeps the store of blocks open
+    want_small = hfmm_b200.evaluate_field(small, q[:4000])
+    qd = torch.as_tensor(q.real.copy()).cuda()
+    want = None
+    for _ in range(3):
+        st = hfmm_b200.setup(pos, 3.0, p=6, N_max=32)
+        phi = [torch.zeros(len(q), dtype=torch.complex128, device="cuda") for _ in range(8)]
+        side = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        for x in phi:
+            hfmm_b200.evaluate_into(st, qd, None, x, stream=side)
+        st.close()
+        other = hfmm_b200.setup(pos[:4000], 2.0, p=4, N_max=24)
+        got = hfmm_b200.evaluate_field(other, q[:4000])
+        other.close()
+        assert all(np.array_equal(x, y) for x, y in zip(got, want_small))
+        torch.cuda.synchronize()
+        want = phi[0].cpu().numpy() if want is None else want
+        assert all(np.array_equal(x.cpu().numpy(), want) for x in phi)
+    small.close()
