@@ -167,10 +167,8 @@ EvalView view(hfmm_plan* P) {
     v.ld = P->ld;
     v.k = P->k;
     v.yukawa = P->yukawa ? 1 : 0;
-    v.fast = !P->yukawa && P->n_fam == 2 && std::fabs(P->k) * P->extent < 2.5e4 && P->extent > 1e-100 &&
-             P->extent < 1e100;   // every distance met is under 4 extents
-    v.own2 = P->extent * P->extent;
-    if (!(v.own2 > 0.0) || !std::isfinite(v.own2)) v.own2 = 1.0;
+    v.fast = !P->yukawa && P->n_fam == 2 && std::fabs(P->k) * P->extent < 2.5e4 && std::fabs(P->k) < 1e15 &&
+             P->extent > 1e-100 && P->extent < 1e100;   // every distance met is under 4 extents
     v.root = std::fabs(P->k) * P->extent > 25.0;
     v.pos_s = P->pos_s.p;
     v.pos_f = P->pos_f.p;

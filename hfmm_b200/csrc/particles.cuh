@@ -9,10 +9,10 @@ struct EvalView {
     int n_s, ld;
     double k;                  // Helmholtz wavenumber, or the screening constant kappa
     int yukawa;                // 0: Helmholtz (two families); 1: exp(-kappa r) / (4 pi r)
-    int fast;                  // Helmholtz with two families, every phase k r under 1e5 and the
-                               // domain's size in [1e-100, 1e100]: pair64's FAST form
-    double own2;               // a squared distance that stands in for a coincident point's: the
-                               // domain's, whose phase is among those the forms are made for
+    int fast;                  // Helmholtz with two families, every phase k r under 1e5, |k| under
+                               // 1e15 (a coincident point stands in at r = 1 with no charge: its
+                               // phase need not be right, but finite) and the domain's size in
+                               // [1e-100, 1e100]: pair64's FAST form
     int root;                  // phases so large that the near field takes pair64's ROOT form
     const double* pos_s;       // 3 x n, leaf-major sorted
     const float* pos_f;        // 6 x n: FP32 hi parts x|y|z, then lo parts (pos = hi + lo)

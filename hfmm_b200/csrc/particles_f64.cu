@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(32 * P2P_WARPS) k_p2p(EvalView v, const int32_
                         for (int f = 0; f < NF; ++f)
 #pragma unroll
                             for (int r = 0; r < R; ++r) q[f][r] = far ? st[3 + r][k] : 0.0;
-                        pair64<NF, R, FIELD, F, ROOT>(v.yukawa, v.k, dx, dy, dz, far ? d2 : v.own2, q, acc);
+                        pair64<NF, R, FIELD, F, ROOT>(v.yukawa, v.k, dx, dy, dz, far ? d2 : 1.0, q, acc);
                     }
                 };
                 if (FAST && thr >= 1e-290) sources(std::true_type());
