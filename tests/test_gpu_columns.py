@@ -47,3 +47,16 @@ def test_two_families_small_wavenumber(precision, tol):
         y = one + 1j * s * two
         assert O.relative_error(x.imag, y.imag) < tol and O.relative_error(x.real, y.real) < tol
     st.close()
+
+
+@pytest.mark.parametrize("s", [1.0, 1e-8])
+def test_streamed_rows_of_a_plane(s):
+    """A streamed plan whose workspace holds no plane of complex frequencies (p = 2, five levels)
+    transforms the columns apart."""
+    import hfmm_b200
+    pos, a, b = _columns(20000)
+    st = hfmm_b200.setup(pos, 1e-6, p=2, N_max=32, max_depth=5, stream_tables=True)
+    one, two = (hfmm_b200.evaluate(st, v) for v in (a, b))
+    x, y = hfmm_b200.evaluate_field(st, a + 1j * s * b)[0], one + 1j * s * two
+    assert O.relative_error(x.imag, y.imag) < 3e-12 and O.relative_error(x.real, y.real) < 3e-12
+    st.close()
