@@ -14,6 +14,7 @@ HFMM_OK = 0
 HFMM_PREC_FP64 = 0
 HFMM_PREC_MIXED = 1
 N_PHASES = 15
+# "tf32_split" keeps its name: the split of the mixed M2L's operands, into FP16 planes
 PHASES = ("gather", "p2m", "m2m_gemm", "up_decode", "m2l_l2l_gemm", "p2l", "down_decode",
           "p2p", "l2p", "m2p", "combine", "tf32_split", "m2l_tables", "l2l_gemm",
           "m2l_compress")

@@ -185,7 +185,7 @@ struct __align__(8) Ctl {
     int n_act;
     int tgt[BN];
     short act[M2L_ENTRIES + 1];
-    short zidx[M2L_ENTRIES + 1];   // A-table index of each active entry (M2L or L2L table)
+    short zidx[M2L_ENTRIES + 1];   // A-table index of each active entry
     unsigned char used[M2L_ENTRIES + 1];   // entry has a source for some target of the tile
     short ztab[M2L_ENTRIES + 1];           // A-table index of every entry (-1: none)
 };

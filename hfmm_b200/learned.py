@@ -68,10 +68,10 @@ def precision_for(tol, p):
 
 def compress_for(tol, precision):
     """Low-rank M2L tolerance of the mixed path: a tenth of the requested tolerance,
-    at most 1e-7; None for the FP64 path. Measured on 1M points at p = 8: the dense
-    mixed M2L gives 4.5e-7 / 6.9e-7 (potential / field), eps 1e-8 gives 5.5e-7 /
-    6.9e-7 and eps 1e-7 5.3e-7 / 7.1e-7 (its truncation stays under the
-    operands' rounding), with the evaluate at 76, 47 and 43.5 ms."""
+    at most 1e-7; None for the FP64 path. Measured on 1M points at p = 8: the FP64
+    evaluate gives 2.1e-7 / 6.1e-7 (potential / field), the dense mixed M2L 3.4e-7 /
+    6.2e-7, eps 1e-8 4.5e-7 / 6.2e-7 and eps 1e-7 4.4e-7 / 6.4e-7, at 31.6, 39.3, 15.5
+    and 13.8 ms."""
     from . import PREC_MIXED
     return min(1e-7, 1e-1 * tol) if precision == PREC_MIXED else None
 

@@ -43,8 +43,8 @@ extern "C" {
 #define HFMM_PREC_FP64 0      /* plain path: every phase in float64                  */
 #define HFMM_PREC_MIXED 1     /* M2L on tcgen05 with FP16 hi/lo operand planes and
                                  power-of-two scales (FP32 accumulation in short
-                                 chains, folded into FP64), P2P in FP32 with an
-                                 FP64 phase reduction; decodes, M2M, L2L, P2M, L2P FP64.
+                                 chains, folded into FP64), P2P in FP32, phases
+                                 included; decodes, M2M, L2L, P2M, L2P FP64.
                                  M2L needs p >= 5 (ld = n_s rounded up to 32 >= 128);
                                  smaller p, and a screened kernel with kappa x domain
                                  extent > 2 (its clusters' results stay apart, beyond the

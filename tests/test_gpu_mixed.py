@@ -1,7 +1,7 @@
-"""The mixed-precision path (M2L + L2L as split 3xTF32 on tcgen05, FP32
+"""The mixed-precision path (M2L on tcgen05 with two FP16 planes an operand, FP32
 accumulation) against the plain FP64 path on the same plan and against the
-FP64 direct sum. Tolerances: mixed vs FP64 relative L2 below 2e-6 (TF32x3
-products carry ~2^-22 relative error); mixed vs direct sum no worse than the
+FP64 direct sum. Tolerances: mixed vs FP64 relative L2 below 2e-6 (the planes'
+products carry ~2^-22 relative error, the FP32 near field 2^-24); mixed vs direct sum no worse than the
 FP64 error plus 2e-6."""
 import numpy as np
 import pytest

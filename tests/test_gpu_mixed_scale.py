@@ -5,7 +5,8 @@ stays inside its range at 2^+-60), and zero charges give zeros. Ranks from the l
 compression to none (k-chunks of one to four steps, row blocks of 64 and 128), real and
 complex charges, sources gathered (clusters) and from the grid (uniform).
 One charge 2^30 times the others sets every plane's scale: the error against FP64 on the same
-plan stays at the mixed path's bar, 2e-6 in the norm, which that charge carries."""
+plan stays at the mixed path's bar, 2e-6 in the norm, which that charge carries (what is left
+of the weaker charges' own results: test_gpu_mixed_range.py)."""
 import numpy as np
 import pytest
 
