@@ -442,7 +442,8 @@ void evaluate_fp64(hfmm_plan* P, const double* q_re, const double* q_im, double*
     if (up) {
         PhaseTimer pt(X, s, 0);
         // complex charges of two families: the convolution balances the columns' magnitudes
-        const bool balance = R == 2 && NF == 2 && P->conv.on && P->rot_P == 0 && !(mixed && P->mixed_ready);
+        const bool balance = R == 2 && NF == 2 && P->conv.on && P->conv.n_slots > 0 && P->rot_P == 0 &&
+                             !(mixed && P->mixed_ready);
         if (balance) HFMM_CUDA(cudaMemsetAsync(P->q_max.p, 0, 2 * sizeof(unsigned long long), s));
         gather_charges(P->n, P->sort_idx.p, q_re, q_im, P->q_s.p, balance ? P->q_max.p : nullptr, s);
     }

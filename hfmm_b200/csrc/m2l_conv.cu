@@ -735,7 +735,8 @@ void conv_workspace(hfmm_plan* P) {
         return;
     }
     const size_t row = 2 * (size_t)chunk_values(P, C.n, 1) * sizeof(double2);
-    const size_t plane = row * C.n * P->n_fam;
+    // two complex sequences, or one family's two real ones of (n + 1) / 2 values a row
+    const size_t plane = (P->n_fam > 1 ? 2 * row : row / C.n * (C.n + 1)) * C.n;
     const size_t planes = std::min<size_t>(C.n, CONV_WS / plane);
     const size_t want = (planes ? plane * planes : std::max(row, CONV_WS)) / sizeof(double);
     if (C.ws.n < want) C.ws.alloc_between(row / sizeof(double), want);
