@@ -135,22 +135,26 @@ __global__ void k_conv_nbr(const int32_t* __restrict__ child, const int32_t* __r
 
 // ---------------------------------------------------------------- transforms
 // A transform leaves a rounding of the larger column in the smaller one of a complex sequence.
-// The imaginary charges are therefore brought to the scale of the real ones, by a power of two
-// (exact), on the way in and back on the way out: each column's error is then that of its own
+// The column of smaller charges is therefore brought to the scale of the other, by a power of two
+// (exact; up, so that nothing underflows), on the way in and back on the way out: each column's error is then that of its own
 // magnitude, as where the columns travel apart (k = 1e-6, imaginary charges 1e-8 of the real
 // ones: imaginary part off by 4e-10 without, 4e-15 with it). A column of zeros stays zeros.
 struct Balance {
-    double up = 1.0, down = 1.0;
-    bool re = true, im = true;   // the column holds a charge
+    double up[2] = {1.0, 1.0}, down[2] = {1.0, 1.0};
+    bool any[2] = {true, true};   // the column holds a charge
 };
 __device__ __forceinline__ Balance balance(const unsigned long long* q_max) {
     Balance b;
-    b.re = q_max[0] != 0;
-    b.im = q_max[1] != 0;
-    const int er = (int)(q_max[0] >> 52), ei = (int)(q_max[1] >> 52), d = er - ei;
-    if (er > 0 && ei > 0 && er < 2047 && ei < 2047 && abs(d) < 1000) {
-        b.up = __longlong_as_double((long long)(1023 + d) << 52);
-        b.down = __longlong_as_double((long long)(1023 - d) << 52);
+    b.any[0] = q_max[0] != 0;
+    b.any[1] = q_max[1] != 0;
+    const int er = (int)(q_max[0] >> 52), ei = (int)(q_max[1] >> 52), d = abs(er - ei);
+    if (er > 0 && ei > 0 && er < 2047 && ei < 2047 && d < 1000) {
+        const double up = __longlong_as_double((long long)(1023 + d) << 52);
+        const double down = __longlong_as_double((long long)(1023 - d) << 52);
+        b.up[0] = er < ei ? up : 1.0;
+        b.down[0] = er < ei ? down : 1.0;
+        b.up[1] = er < ei ? 1.0 : up;
+        b.down[1] = er < ei ? 1.0 : down;
     }
     return b;
 }
@@ -294,7 +298,7 @@ __global__ void __launch_bounds__(256) k_conv_fwd(ConvCall c) {
         const double* src = c.dens + seq * c.seq_stride + b * c.box_stride;
         for (int r = 0; r < R; ++r)
             for (int s = tid; s < c.n_s; s += nt)
-                xs[(c.pos[s] * CH + ch) * R + r] = b >= 0 ? src[r * c.ld + s] * (r ? bal.up : 1.0) : 0.0;
+                xs[(c.pos[s] * CH + ch) * R + r] = b >= 0 ? src[r * c.ld + s] * (R == 2 ? bal.up[r] : 1.0) : 0.0;
     }
     __syncthreads();
     axis_table(a, tw, T);
@@ -496,7 +500,7 @@ __global__ void __launch_bounds__(256) k_conv_inv(ConvCall c) {
         const double* src = c.check + seq * c.seq_stride + b * c.box_stride;
         for (int r = 0; r < R; ++r)
             for (int s = tid; s < c.n_s; s += nt)
-                acc[(c.pos[s] * CH + ch) * R + r] = c.first || b < 0 ? 0.0 : src[r * c.ld + s] * (r ? bal.up : 1.0);
+                acc[(c.pos[s] * CH + ch) * R + r] = c.first || b < 0 ? 0.0 : src[r * c.ld + s] * (R == 2 ? bal.up[r] : 1.0);
     }
     __syncthreads();
     axis_table(a, tw, T);
@@ -564,7 +568,8 @@ __global__ void __launch_bounds__(256) k_conv_inv(ConvCall c) {
         double* dst = c.check + seq * c.seq_stride + b * c.box_stride;
         for (int r = 0; r < R; ++r)
             for (int s = tid; s < c.n_s; s += nt)
-                dst[r * c.ld + s] = (r ? bal.im : bal.re) ? acc[(c.pos[s] * CH + ch) * R + r] * (r ? bal.down : 1.0) : 0.0;
+                dst[r * c.ld + s] = R == 1 || bal.any[r] ? acc[(c.pos[s] * CH + ch) * R + r] * (R == 2 ? bal.down[r] : 1.0)
+                                                         : 0.0;
     }
 }
 

@@ -49,6 +49,21 @@ def test_two_families_small_wavenumber(precision, tol):
     st.close()
 
 
+@pytest.mark.parametrize("small,large", [(1e-290, 1.0), (1.0, 1e280), (1e-290, 1e-5)])
+def test_columns_far_apart(small, large):
+    """Columns hundreds of orders of magnitude apart, at a wavenumber that keeps the results
+    apart: each by itself as accurate as alone, whichever is the larger."""
+    import hfmm_b200
+    pos, a, b = _columns(6000)
+    st = hfmm_b200.setup(pos, 0.0, p=5, N_max=32)   # two families, the sin family's sums all zero
+    one, two = (hfmm_b200.evaluate_field(st, v) for v in (a, b))
+    for x, u, v in zip(hfmm_b200.evaluate_field(st, a * large + 1j * b * small), one, two):
+        assert O.relative_error(x.real / large, u.real) < 3e-12 and O.relative_error(x.imag / small, v.real) < 3e-12
+    for x, u, v in zip(hfmm_b200.evaluate_field(st, a * small + 1j * b * large), one, two):
+        assert O.relative_error(x.real / small, u.real) < 3e-12 and O.relative_error(x.imag / large, v.real) < 3e-12
+    st.close()
+
+
 @pytest.mark.parametrize("s", [1.0, 1e-8])
 def test_streamed_rows_of_a_plane(s):
     """A streamed plan whose workspace holds no plane of complex frequencies (p = 2, five levels)
