@@ -81,15 +81,25 @@ __host__ __device__ __forceinline__ double plane_scale(unsigned long long most) 
 
 // Do planes with one scale a level serve this plan's densities? Their absolute error is 2^-38 of
 // the level's largest, everywhere. Under a kernel that falls like 1 / r the field of the largest
-// hides it; a screened one leaves clusters some screening lengths apart their own results, and
-// the weaker cluster's are lost. Mixed against FP64 on the weaker of two clusters across the
-// domain, charges 2^14 to 2^36 apart, p = 8, depth 6 and 10 (TF32 halves had 1.3e-6 at most):
-// kappa x extent 2: 7.9e-7, 3: 1.4e-6, 4: 6.5e-6, 6: 1.6e-4, 12: 0.6. Past 2 the M2L runs in
-// FP64, by convolution one family of which is as fast or faster: 5e5 points, p = 8, kappa = 20,
-// whole evaluate, real / complex charges: low-rank planes 6.7 / 10.1 ms, dense planes 13.8 /
-// 22.1, FP64 M2L 8.3 / 15.3 (TF32 halves 11.9 / 16.2 and 18.6 / 30.5); 20,000 points 2.6 / 2.6
-// with dense planes, 0.41 / 0.56 without.
-inline bool planes_hold(const hfmm_plan* P) { return !P->yukawa || P->k * P->extent <= 2.0; }
+// hides it, in two cases not:
+//  * A screened kernel leaves clusters some screening lengths apart their own results, and the
+//    weaker cluster's are lost. Mixed against FP64 on the weaker of two clusters across the
+//    domain, charges 2^14 to 2^36 apart, p = 8, depth 6 and 10 (TF32 halves had 1.3e-6 at most):
+//    kappa x extent 2: 7.9e-7, 3: 1.4e-6, 4: 6.5e-6, 6: 1.6e-4, 12: 0.6.
+//  * The field -grad phi of a faraway strong cluster falls like 1 / r^2, the error's like 1 / (box
+//    side)^2: on small boxes the error shows. Clusters of sigma 0.0005, depth 10, low rank, field
+//    on the weaker: Laplace 3e-5 (TF32 halves 5e-7), Helmholtz k x extent = 1 1e-5 (8e-7), 3 and
+//    more the same (1e-5: the tables' own error, sin family); sigma 0.004 (boxes of level 8)
+//    3e-6 (7e-7), depth 6 the same.
+// There the M2L runs in FP64. By convolution one family of it is as fast or faster: 5e5 points,
+// p = 8, kappa = 20, whole evaluate, real / complex charges: low-rank planes 6.7 / 10.1 ms, dense
+// planes 13.8 / 22.1, FP64 M2L 8.3 / 15.3 (TF32 halves 11.9 / 16.2 and 18.6 / 30.5); 20,000
+// points 2.6 / 2.6 with dense planes, 0.41 / 0.56 without.
+inline bool planes_hold(const hfmm_plan* P) {
+    const double kd = (P->k < 0.0 ? -P->k : P->k) * P->extent;
+    if (P->yukawa && kd > 2.0) return false;
+    return P->md < 8 || (!P->yukawa && kd >= 3.0);
+}
 
 // Maps of the two planes of tables [count][ldm][ld] (ldm 0: ld), `plane` apart, and of a grid
 // [plane][x][y][z][2][ckld]: rows and K values from `valid` on are zeros, which the loads

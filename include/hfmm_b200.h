@@ -46,9 +46,10 @@ extern "C" {
                                  chains, folded into FP64), P2P in FP32, phases
                                  included; decodes, M2M, L2L, P2M, L2P FP64.
                                  M2L needs p >= 5 (ld = n_s rounded up to 32 >= 128);
-                                 smaller p, and a screened kernel with kappa x domain
-                                 extent > 2 (its clusters' results stay apart, beyond the
-                                 planes' range), run the M2L in FP64.                  */
+                                 smaller p, a screened kernel with kappa x domain
+                                 extent > 2, and trees of depth 8 or more with k x extent
+                                 under 3 (results beyond the planes' range) run the M2L
+                                 in FP64.                                              */
 
 typedef struct hfmm_plan hfmm_plan;
 

@@ -31,6 +31,29 @@ def test_weak_cluster(kappa, eps):
     st.close()
 
 
+@pytest.mark.parametrize("eps", [None, 1e-7])
+@pytest.mark.parametrize("kind,k", [("laplace", 0.0), ("yukawa", 1.9), ("helmholtz", 0.01), ("helmholtz", 1.0)])
+def test_field_on_a_weak_deep_cluster(kind, k, eps):
+    """Two clusters a thousandth of the domain wide (depth 10): the strong one's field at the weak
+    one is 1 / r^2 of its charges, what its densities' rounding leaves there 1 / (box side)^2."""
+    import hfmm_b200
+    from hfmm_b200.kernels import LAPLACE, helmholtz, yukawa
+    rng = np.random.default_rng(12)
+    n = 20000
+    pos = np.concatenate([np.clip(c + 0.0005 * rng.normal(size=(n // 2, 3)), 0, 1) for c in (0.05, 0.95)])
+    pos[0], pos[-1] = 0.0, 1.0
+    q = rng.normal(size=n)
+    spec = LAPLACE if kind == "laplace" else yukawa(k) if kind == "yukawa" else helmholtz(k)
+    st = hfmm_b200.kernel_setup(pos, spec, p=8, N_max=24, m2l_compress=eps)
+    assert st.max_depth >= 8
+    for e in (0, 26, 34):
+        v = q.copy()
+        v[: n // 2] *= 2.0 ** e
+        for x, y in zip(hfmm_b200.evaluate_field(st, v, hfmm_b200.PREC_MIXED), hfmm_b200.evaluate_field(st, v)):
+            assert O.relative_error(x[n // 2:], y[n // 2:]) < 2e-6
+    st.close()
+
+
 @pytest.mark.parametrize("p", [5, 6])
 @pytest.mark.parametrize("shift", [-40, 0, 3, 20])
 def test_scaled_host_tables(monkeypatch, p, shift):
