@@ -1305,9 +1305,9 @@ int hfmm_plan_phase_times(hfmm_plan* P, double* ms) {
 void hfmm_plan_destroy(hfmm_plan* P) {
     if (!P) return;
     if (P->batch_owner) batch_forget_plan(P->batch_owner, P);
-    // the first buffer's cudaFree waits for the plan's work; the others can then be kept
+    // one buffer's cudaFree waits for the plan's work; the others can then be kept
     std::optional<KeepBlocks> keep;
-    if (P->check.release_and_wait()) keep.emplace(true);
+    if (P->d_err.release_and_wait()) keep.emplace(true);
     drop_extra(P);
     delete[] static_cast<MixedMaps*>(P->mx_maps);
     P->mx_maps = nullptr;
